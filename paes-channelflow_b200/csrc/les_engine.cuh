@@ -274,8 +274,13 @@ struct Engine : EngineBase {
       for (auto& b : flux) b.alloc(pb * NZ);
     }
     divacc.alloc(NZ); sgsacc.alloc((size_t)NZ * 8); wacc.alloc((size_t)2 * kWallBlocks * 8); acc.alloc((size_t)NZ * 16);
-    // one partial per padded row (k_row_fused) or per 256-point block (k_flux)
-    nstat_parts = fused ? MY : (int)cdiv(pb, 256);
+    // one partial per warp of k_row_fused or per 256-point block of k_flux
+    nstat_parts = (int)cdiv(pb, 256);
+    if (fused)
+      with_small(NX, [&](auto cn) {
+        using C = FusedCfg<T, decltype(cn)::value>;
+        nstat_parts = MY / C::ROWS * C::WARPS;
+      });
     divpart.alloc((size_t)NZ * nstat_parts); sgspart.alloc((size_t)NZ * nstat_parts * 6);
     wp.alloc(1); err.alloc(1); amax.alloc(4);
     for (auto& b : phys) b.alloc(ps * (NZ + 2));
@@ -817,29 +822,32 @@ struct Engine : EngineBase {
     fa.lflag = learned_on() ? lflag.p : nullptr;
     with_small(NX, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
-      const int threads = FusedCfg<N>::template threads<T>();
-      const size_t smem = FusedCfg<N>::template smem<T>();
-      if (fused_chunks == 0) fused_chunks = fused_chunk_count((const void*)k_row_fused<T, N>, threads, smem);
+      using C = FusedCfg<T, N>;
+      if (fused_chunks == 0)
+        fused_chunks = fused_chunk_count((const void*)k_row_fused<T, N>, C::THREADS, C::smem(), MY / C::ROWS);
       fa.zchunk = (int)cdiv(NZ, fused_chunks);
-      launch(k_row_fused<T, N>, dim3(MY, (unsigned)cdiv(NZ, fa.zchunk)), dim3(threads), smem, st, fa, a, tw);
+      launch(k_row_fused<T, N>, dim3(MY / C::ROWS, (unsigned)cdiv(NZ, fa.zchunk)), dim3(C::THREADS), C::smem(), st, fa,
+             a, tw);
     });
   }
-  // z chunks per padded row of the fused kernel: a CTA walks its chunk with
-  // a sliding window, so chunks only add prologues (about half a level of
-  // work each), while the last wave of CTAs leaves SMs idle.  Minimise
-  // waves x (levels per chunk + 1/2) over 1..NZ/8 chunks, the waves counted
-  // with the kernel's resident CTAs per SM.
+  // z chunks of the fused kernel: a CTA walks its rows' chunk with a sliding
+  // window, so chunks only add prologues (about half a level of work each),
+  // while the last wave of CTAs leaves SMs idle.  Minimise waves x (levels
+  // per chunk + 1/2) over 1..NZ chunks, the waves counted with the kernel's
+  // resident CTAs per SM.  A grid that fits one wave is bound by the latency
+  // of a CTA's chain of levels, so its chunks shrink to a level or two
+  // (32x32x16: 16 chunks instead of the 2 of an 8-level minimum).
   int fused_chunks = 0;
-  int fused_chunk_count(const void* kernel, int threads, size_t smem) {
+  int fused_chunk_count(const void* kernel, int threads, size_t smem, int rows) {
     if (smem > 48 * 1024) set_smem_limit(kernel, smem);
     int per_sm = 0;
     LES_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     const double resident = (double)std::max(1, per_sm) * nsm;
     int best = 1;
     double best_cost = 0.0;
-    for (int c = 1; c <= std::max(1, NZ / 8); c++) {
+    for (int c = 1; c <= NZ; c++) {
       const int zc = (int)cdiv(NZ, c), n = (int)cdiv(NZ, zc);
-      const double cost = std::ceil((double)MY * n / resident) * (zc + 0.5);
+      const double cost = std::ceil((double)rows * n / resident) * (zc + 0.5);
       if (c == 1 || cost < best_cost) { best = c; best_cost = cost; }
     }
     return best;

@@ -1,191 +1,280 @@
 // les_fused.cuh -- the padded-grid part of comp1 as one kernel per (padded
-// y row, z chunk): inverse x transforms of the mixed arrays, the pointwise
+// y rows, z chunk): inverse x transforms of the mixed arrays, the pointwise
 // advection / SGS fluxes, and the forward x transforms with -d/dx folded in,
 // without ever writing the padded physical fields to HBM.
 //
-// The CTA walks up its z chunk keeping a window of physical rows in shared
-// memory (levels z-1, z, z+1 of U, V, W, E, packed as complex rows U+iV and
-// W+iE), exactly the sliding window of comp1.f90:91-121 / 179-184 but along
-// one row of the padded plane.  Six teams (one warp each) each own one
-// transform per phase:
+// The CTA walks up its z chunk with the sliding window of comp1.f90:91-121 /
+// 179-184 along ROWS rows of the padded plane.  Each row has six teams of TP
+// threads and six shared-memory buffers; team w owns transform w of both
+// phases and buffer w:
 //   phase I   (inverse)  w0: U+iV (z+1)   w1: W+iE (z+1)   w2: UX+iVX (z)
 //                        w3: UY+iVY (z)   w4: WX+iWY (z)   w5: EX+iEY (le)
 //             (when the learned closure supplies the interior momentum
 //             stresses only ux and vy are needed, for the divergence
 //             diagnostic: w2 transforms UX+iVY, w3 and w4 idle)
-//   phase II  (pointwise, all threads) the eleven flux rows of k_flux
+//   phase II  (pointwise, all threads) the eleven flux rows of k_flux,
+//             written over the six rows it read
 //   phase III (forward)  w0: A+iPu  w1: B+iPv  w2: C+iG  w3: D+iPw
 //                        w4: F+iPe  w5: H
-// Transforms are warp-synchronous four-step FFTs (lanes = N2 in pass A,
-// N1 in pass B, __syncwarp between passes) or, for rows whose second
-// factor exceeds 24 (768), three Stockham passes synchronised by the team's
-// named barrier; block barriers only separate the three phases.
+// Each thread keeps its own points of the window (levels z-1 and z) in
+// registers, so a row needs six buffers instead of eleven.
 #pragma once
 #include "les_kernels.cuh"
 
 namespace les {
 
-// XOR swizzle of natural-layout indices in the fused kernel's buffers:
-// within each 128-byte block the low bits are XORed with the block index, so
-// strided butterfly writes (stride R elements) land in distinct banks.  A
-// bijection on [0, N) when N is a multiple of the block length.
-template <class T, int N> struct Swz {
-  static constexpr int SHIFT = (sizeof(cx<T>) == 16) ? 3 : 4;
-  static constexpr int MASK = (N % (1 << SHIFT) == 0) ? ((1 << SHIFT) - 1) : 0;
-  static __device__ __forceinline__ int f(int a) { return a ^ ((a >> SHIFT) & MASK); }
+// Row transforms of the fused kernel, N = 12 M1.  The inverse runs decimation
+// in frequency, natural order in, permuted order out; the forward transform
+// runs the same passes backwards, permuted in, natural out.  The pointwise
+// phase does not care about the order of the points, so nothing is ever
+// reordered: every pass reads and writes the same elements in place, and a
+// pass needs one team barrier instead of the two of an autosorting pass.
+//   element n = b M1 + r R3 + i   (M1 = R2 R3, b < 12, r < R2, i < R3)
+//   pass 1 (radix 12, over b): thread j = r R3 + i
+//   pass 2 (radix R2, over r): thread (b, i), twiddle W_M1^(r i)
+//   pass 3 (radix R3, over i): thread (b, r); none when R3 = 1
+// The first factor is 12 because a padded row has modes |k| < N/3 only: of
+// pass 1's 12 inputs (outputs, forward) the middle 4 are zero (unwanted) at
+// compile time, and thread j's positive modes j + M1 b and its partner
+// M1 - j's negative ones are mirror images, exchanged by shuffles, so each
+// spectral value is loaded (stored) once.
+// Pass 1's twiddles: for N = 3 * 2^m (PFA) the factor 3 is split off by the
+// prime-factor map (no twiddles; thread j's 3-point transforms are rotated by
+// W_3^s, s = s(j), which costs two real factors per term) and the factor 4
+// needs W_(N/3)^(j k), k = 1..3: three table values a thread instead of
+// eleven.  Else (N = 9 * 2^m) W_N^(b j).  With R2 = 4 pass 2 is exactly three
+// rounds of M1 threads with one i each, again three table values.
+// Elements are padded by one per PB (one 128-byte group per element offset),
+// with which all passes' accesses at N = 768 are conflict-free, and every
+// address is a per-thread base plus a constant.
+template <int MX> struct RowPlan;
+template <> struct RowPlan<24> { static constexpr int R2 = 2, R3 = 1; };
+template <> struct RowPlan<48> { static constexpr int R2 = 4, R3 = 1; };
+template <> struct RowPlan<96> { static constexpr int R2 = 8, R3 = 1; };
+template <> struct RowPlan<144> { static constexpr int R2 = 12, R3 = 1; };
+template <> struct RowPlan<192> { static constexpr int R2 = 16, R3 = 1; };
+template <> struct RowPlan<288> { static constexpr int R2 = 4, R3 = 6; };
+template <> struct RowPlan<384> { static constexpr int R2 = 4, R3 = 8; };
+template <> struct RowPlan<576> { static constexpr int R2 = 4, R3 = 12; };
+template <> struct RowPlan<768> { static constexpr int R2 = 4, R3 = 16; };
+
+template <class T, int NSX> struct FusedCfg {
+  static constexpr int MX = 3 * NSX / 2, KX = NSX / 2;
+  static constexpr int R2 = RowPlan<MX>::R2, R3 = RowPlan<MX>::R3, M1 = MX / 12;
+  static_assert(R2 * R3 == M1 && 4 * M1 == KX, "row plan");
+  // threads of a team: M1 rounded up to a power of two
+  static constexpr int TP = M1 <= 2 ? 2 : M1 <= 4 ? 4 : M1 <= 8 ? 8 : M1 <= 16 ? 16 : M1 <= 32 ? 32 : 64;
+  static constexpr int TR = 6 * TP;                      // threads of a row
+  static constexpr int ROWS = TR >= 96 ? 1 : 96 / TR;    // rows of a CTA (divides every padded ny)
+  static constexpr int THREADS = TR * ROWS;
+  static constexpr int WARPS = THREADS / 32;
+  static constexpr int PPT = (MX + TR - 1) / TR;         // points of a thread in phase II
+  static constexpr bool PFA = M1 % 3 != 0;
+  static constexpr int PB = sizeof(T) == 4 ? 16 : 8;
+  static constexpr int SB = R3 == 1 ? (M1 | 1) : M1 + M1 / PB + (sizeof(T) == 8 ? 1 : 0);  // stride of b
+  static constexpr int BUF = 12 * SB + (TP == 8 ? 12 : TP == 2 ? 14 : 0);
+  static constexpr int NT1 = PFA ? 3 : 11;               // pass 1 twiddles of a thread
+  static constexpr int NTW = NT1 * M1 + (R3 > 1 ? (R2 - 1) * R3 : 0);
+  // x of the point at element n: b = 4 x3 + k4 and kappa = k4 + 4 (r + R2 i)
+  // stand for x mod 3 = x3, x mod N/3 = 3 kappa (PFA); else b + 12 (r + R2 i)
+  static __device__ __forceinline__ int x_of(int n) {
+    const int b = n / M1, m = n - b * M1, o = m / R3 + R2 * (m % R3);
+    if (!PFA) return b + 12 * o;
+    constexpr int Q = 4 * M1, U = Q % 3 == 1 ? Q : 2 * Q;  // U = 1 mod 3, 0 mod Q
+    return ((b >> 2) * U + 3 * ((b & 3) + 4 * o)) % MX;
+  }
+  static constexpr size_t smem() { return ((size_t)6 * ROWS * BUF + NTW) * sizeof(cx<T>); }
+  // Resident CTAs per SM the register budget aims at: 24 warps of <= 80
+  // registers in FP32, 12 of <= 168 in FP64.  Tighter budgets spill (FP64 at
+  // 18 warps: 64-point grids 47 -> 60 us per launch), looser ones leave the
+  // passes' shared-memory latency uncovered (FP32 at 12 warps: 512x512x32
+  // 719 -> 885 us).
+  static constexpr int CTAS = (sizeof(T) == 4 ? 768 : 384) / THREADS;
+  // offset of r R3 + i within b
+  static __device__ __forceinline__ constexpr int off(int m) { return R3 == 1 ? m : m + m / PB; }
+  // address of element n
+  static __device__ __forceinline__ int at(int n) {
+    const int b = n / M1, m = n - b * M1;
+    return b * SB + off(m);
+  }
 };
 
-// Warp-level four-step transform of one length-N sequence in `buf`
-// (smem_fft_elems<N,false>(1) elements).  IN: load(n) from global memory or,
-// with IN_SMEM, buf in natural layout.  OUT: buf in natural layout.
-template <int N, int S, bool IN_SMEM, class T, class LoadF>
-__device__ __forceinline__ void warp_fft(cx<T>* buf, const cx<T>* twn, LoadF load) {
-  constexpr int N1 = Split<N>::N1;
-  constexpr int N2 = Split<N>::N2;
-  constexpr int LD = N2 + 1;
-  static_assert(N1 <= 32 && N2 <= 32, "warp transform needs N1, N2 <= 32");
-  const int lane = threadIdx.x & 31;
-  {
-    cx<T> v[N1];
-    if (lane < N2) {
+// a + s b, one packed instruction in FP32
+template <class T> __device__ __forceinline__ cx<T> axpy(cx<T> a, T s, cx<T> b) { return mk(a.x + s * b.x, a.y + s * b.y); }
+template <> __device__ __forceinline__ cx<float> axpy<float>(cx<float> a, float s, cx<float> b) {
+  cx<float> r;
+  asm("{\n\t.reg .b64 a, b, s, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 s, {%6, %6};\n\t"
+      "fma.rn.f32x2 r, b, s, a;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(s));
+  return r;
+}
+// a + s i b
+template <class T> __device__ __forceinline__ cx<T> axipy(cx<T> a, T s, cx<T> b) { return mk(a.x - s * b.y, a.y + s * b.x); }
+
+// 12-point DFTs as 3 x 4 without inner twiddles (prime-factor maps: input
+// n = 4 a + 3 c, output k = 4 k3 + 9 k4, both mod 12).
+// Inverse with inputs 4..7 zero: x[0..3] inputs 0..3, x[4..7] inputs 8..11.
+template <class T> __device__ __forceinline__ void dft12_padded(const cx<T> (&x)[8], cx<T> (&y)[12]) {
+  constexpr T h = (T)0.5, s3 = (T)0.86602540378443864676372317075293618;
+  cx<T> g[3][4];  // [k3][c]
+  // c = 0: inputs 0, 4, 8;  c = 1: 3, 7, 11 (the second is zero)
 #pragma unroll
-      for (int n1 = 0; n1 < N1; n1++) {
-        if constexpr (IN_SMEM) v[n1] = buf[Swz<T, N>::f(lane + N2 * n1)];
-        else v[n1] = load(lane + N2 * n1);
-      }
-    }
-    if (IN_SMEM) __syncwarp();
-    if (lane < N2) {
-      Dft<N1, S, T>::run(v);
-#pragma unroll
-      for (int k1 = 0; k1 < N1; k1++) {
-        cx<T> w = twn[k1 * N2 + lane];  // [k1][n2] layout: consecutive lanes, no bank conflicts
-        if (S > 0) w.y = -w.y;
-        buf[k1 * LD + lane] = (k1 == 0) ? v[k1] : cmul(v[k1], w);
-      }
-    }
+  for (int c = 0; c < 2; c++) {
+    const cx<T> p = c == 0 ? x[0] : x[3], q = c == 0 ? x[4] : x[7];
+    const cx<T> t = axpy<T>(p, -h, q);
+    g[0][c] = p + q;
+    g[1][c] = axipy<T>(t, -s3, q);
+    g[2][c] = axipy<T>(t, s3, q);
   }
-  __syncwarp();
-  {
-    cx<T> v[N2];
-    if (lane < N1) {
-#pragma unroll
-      for (int n2 = 0; n2 < N2; n2++) v[n2] = buf[lane * LD + n2];
-    }
-    __syncwarp();
-    if (lane < N1) {
-      Dft<N2, S, T>::run(v);
-#pragma unroll
-      for (int k2 = 0; k2 < N2; k2++) buf[Swz<T, N>::f(lane + N1 * k2)] = v[k2];
-    }
+  {  // c = 2: inputs 6, 10, 2 (the first is zero)
+    const cx<T> s = x[6] + x[2], d = x[6] - x[2], t = s * (-h);
+    g[0][2] = s;
+    g[1][2] = axipy<T>(t, s3, d);
+    g[2][2] = axipy<T>(t, -s3, d);
   }
-  __syncwarp();
+  {  // c = 3: inputs 9, 1, 5 (the third is zero)
+    const cx<T> t = axpy<T>(x[5], -h, x[1]);
+    g[0][3] = x[5] + x[1];
+    g[1][3] = axipy<T>(t, s3, x[1]);
+    g[2][3] = axipy<T>(t, -s3, x[1]);
+  }
+#pragma unroll
+  for (int k3 = 0; k3 < 3; k3++) {
+    Dft<4, +1, T>::run(g[k3]);
+#pragma unroll
+    for (int k4 = 0; k4 < 4; k4++) y[(4 * k3 + 9 * k4) % 12] = g[k3][k4];
+  }
+}
+// Forward with all inputs; the caller leaves outputs 4..7 unused.
+template <class T> __device__ __forceinline__ void dft12_forward(const cx<T> (&x)[12], cx<T> (&y)[12]) {
+  constexpr T h = (T)0.5, s3 = (T)0.86602540378443864676372317075293618;
+  cx<T> g[3][4];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) g[a][c] = x[(4 * a + 3 * c) % 12];
+    Dft<4, -1, T>::run(g[a]);
+  }
+#pragma unroll
+  for (int k4 = 0; k4 < 4; k4++) {
+    const cx<T> s = g[1][k4] + g[2][k4], d = g[1][k4] - g[2][k4], t = axpy<T>(g[0][k4], -h, s);
+    y[(9 * k4) % 12] = g[0][k4] + s;
+    y[(4 + 9 * k4) % 12] = axipy<T>(t, -s3, d);
+    y[(8 + 9 * k4) % 12] = axipy<T>(t, s3, d);
+  }
 }
 
-// Team Stockham transform: TEAM threads (a multiple of 32) share one
-// transform and synchronise with a named barrier `bar` (1..15), so several
-// teams run independent transforms inside one CTA.  In place in buf
-// (natural layout, N elements); each pass holds ceil(N/R/TEAM)*R values
-// per thread.
-template <int TEAM>
-__device__ __forceinline__ void team_sync(int bar) {
-  if (TEAM == 32) __syncwarp();
-  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(TEAM) : "memory");
+template <class T> __device__ __forceinline__ cx<T> shfl_cx(unsigned mask, cx<T> v, int src) {
+  return mk(__shfl_sync(mask, v.x, src), __shfl_sync(mask, v.y, src));
 }
-template <int N, int R, int NS, int S, bool FIRST, int TEAM, class T, class LoadF>
-__device__ __forceinline__ void team_stockham_pass(cx<T>* buf, const cx<T>* twn, LoadF load, int tl, int bar) {
-  constexpr int M = N / R;
-  constexpr int J = (M + TEAM - 1) / TEAM;
-  cx<T> v[J][R];
+
+// Rotated 12-point DFT of pass 1 for N = 3 * 2^m: 3-point transforms over a
+// (input n = j + M1 (c + 4 a), rotated by W_3^(s_c x3), s_c = s + c M1 u mod 3
+// with u = (N/3)^-1 mod 3), then 4-point transforms over c; output b = 4 x3 + k4.
+// w[s] = W_3^(s(j) + s) for s = 0..2.
+template <class T, int M1> struct Dft12Pfa {
+  static constexpr int U = (4 * M1) % 3, STEP = (U * M1) % 3;  // u = Q^-1 = Q mod 3
+  // inverse, inputs 4..7 zero: x[0..3] inputs 0..3, x[4..7] inputs 8..11
+  static __device__ __forceinline__ void padded(const cx<T> (&x)[8], const cx<T> (&w)[3], cx<T> (&y)[12]) {
 #pragma unroll
-  for (int jj = 0; jj < J; jj++) {
-    const int j = tl + TEAM * jj;
-    if (j < M) {
-      const int k = j % NS;
+    for (int c = 0; c < 4; c++) {
+      const cx<T> p = x[c], q = x[4 + c], al = w[(c * STEP) % 3], be = w[(c * STEP + 2) % 3];
+      const cx<T> re = axpy<T>(p * al.x, be.x, q), im = axpy<T>(p * al.y, be.y, q);
+      y[c] = p + q;
+      y[4 + c] = mk(re.x - im.y, re.y + im.x);
+      y[8 + c] = mk(re.x + im.y, re.y - im.x);
+    }
 #pragma unroll
-      for (int r = 0; r < R; r++) {
-        cx<T> x;
-        if constexpr (FIRST) x = load(j + r * M);
-        else x = buf[Swz<T, N>::f(j + r * M)];
-        if (NS > 1 && r > 0) {
-          cx<T> w = twn[r * NS + k];  // this pass's table, [r][k] layout
-          if (S > 0) w.y = -w.y;
-          x = cmul(x, w);
+    for (int k3 = 0; k3 < 3; k3++) Dft<4, +1, T>::run(y + 4 * k3);
+  }
+  // forward, outputs 0..3 and 8..11 (z[0..3], z[4..7])
+  static __device__ __forceinline__ void forward(cx<T> (&y)[12], const cx<T> (&w)[3], cx<T> (&z)[8]) {
+#pragma unroll
+    for (int k3 = 0; k3 < 3; k3++) Dft<4, -1, T>::run(y + 4 * k3);
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const cx<T> s = y[4 + c] + y[8 + c], d = y[4 + c] - y[8 + c], al = w[(c * STEP) % 3], be = w[(c * STEP + 2) % 3];
+      z[c] = axipy<T>(axpy<T>(y[c], al.x, s), -al.y, d);
+      z[4 + c] = axipy<T>(axpy<T>(y[c], be.x, s), -be.y, d);
+    }
+  }
+};
+
+// Passes 2 and 3 of a team's transform in its buffer.  t = thread of the
+// team.  INV: pass 2 then 3; else 3 then 2, with the conjugate twiddles.
+template <class T, int NSX, bool INV> struct RowPasses {
+  using C = FusedCfg<T, NSX>;
+  static constexpr int R2 = C::R2, R3 = C::R3, TP = C::TP, M1 = C::M1;
+  static __device__ __forceinline__ void pass2(cx<T>* buf, const cx<T>* tw2, int t) {
+    if constexpr (R3 > 1) {
+      static_assert(R2 == 4, "three rounds of M1 threads");
+      if (TP > M1 && t >= M1) return;
+      const int i = t % R3;
+      cx<T>* p = buf + (t / R3) * C::SB + (i + i / C::PB);
+      cx<T> w[R2];
+#pragma unroll
+      for (int r = 1; r < R2; r++) w[r] = INV ? conj(tw2[(r - 1) * R3 + i]) : tw2[(r - 1) * R3 + i];
+#pragma unroll
+      for (int jj = 0; jj < 3; jj++) {
+        cx<T> v[R2];
+#pragma unroll
+        for (int r = 0; r < R2; r++) {
+          v[r] = p[4 * jj * C::SB + row_off(r, i)];
+          if (!INV && r > 0) v[r] = cmul(v[r], w[r]);
         }
-        v[jj][r] = x;
+        Dft<R2, INV ? +1 : -1, T>::run(v);
+#pragma unroll
+        for (int r = 0; r < R2; r++) p[4 * jj * C::SB + row_off(r, i)] = (INV && r > 0) ? cmul(v[r], w[r]) : v[r];
+      }
+    } else {
+      constexpr int J = (12 + TP - 1) / TP;
+#pragma unroll
+      for (int jj = 0; jj < J; jj++) {
+        const int b = t + TP * jj;
+        if (J * TP > 12 && b >= 12) break;
+        cx<T>* p = buf + b * C::SB;
+        cx<T> v[R2];
+#pragma unroll
+        for (int r = 0; r < R2; r++) v[r] = p[r];
+        Dft<R2, INV ? +1 : -1, T>::run(v);
+#pragma unroll
+        for (int r = 0; r < R2; r++) p[r] = v[r];
       }
     }
   }
-  team_sync<TEAM>(bar);
+  // off(r R3 + i) - off(i): a constant when PB divides R3 or R3 divides PB
+  static __device__ __forceinline__ int row_off(int r, int i) {
+    if (R3 % C::PB == 0 || C::PB % R3 == 0) return r * R3 + (r * R3) / C::PB;
+    return C::off(r * R3 + i) - C::off(i);
+  }
+  static __device__ __forceinline__ void pass3(cx<T>* buf, int t) {
+    constexpr int ITEMS = 12 * R2, J = (ITEMS + TP - 1) / TP;
 #pragma unroll
-  for (int jj = 0; jj < J; jj++) {
-    const int j = tl + TEAM * jj;
-    if (j < M) {
-      const int k = j % NS;
-      Dft<R, S, T>::run(v[jj]);
-      const int base = (j / NS) * NS * R + k;
+    for (int jj = 0; jj < J; jj++) {
+      const int it = t + TP * jj;
+      if (J * TP > ITEMS && it >= ITEMS) break;
+      const int b = it / R2, r = it - b * R2;
+      cx<T>* p = buf + b * C::SB + C::off(r * R3);
+      cx<T> v[R3];
 #pragma unroll
-      for (int r = 0; r < R; r++) buf[Swz<T, N>::f(base + r * NS)] = v[jj][r];
+      for (int i = 0; i < R3; i++) v[i] = p[col_off(r, i)];
+      Dft<R3, INV ? +1 : -1, T>::run(v);
+#pragma unroll
+      for (int i = 0; i < R3; i++) p[col_off(r, i)] = v[i];
     }
   }
-  team_sync<TEAM>(bar);
-}
-template <int N> struct Radix3;
-template <> struct Radix3<24> { static constexpr int R1 = 2, R2 = 2, R3 = 6; };
-template <> struct Radix3<48> { static constexpr int R1 = 4, R2 = 2, R3 = 6; };
-template <> struct Radix3<96> { static constexpr int R1 = 4, R2 = 4, R3 = 6; };
-template <> struct Radix3<144> { static constexpr int R1 = 4, R2 = 6, R3 = 6; };
-template <> struct Radix3<192> { static constexpr int R1 = 8, R2 = 4, R3 = 6; };
-template <> struct Radix3<288> { static constexpr int R1 = 8, R2 = 6, R3 = 6; };
-template <> struct Radix3<384> { static constexpr int R1 = 8, R2 = 8, R3 = 6; };
-template <> struct Radix3<576> { static constexpr int R1 = 8, R2 = 6, R3 = 12; };
-template <> struct Radix3<768> { static constexpr int R1 = 8, R2 = 8, R3 = 12; };
-template <int N, int S, bool IN_SMEM, int TEAM, class T, class LoadF>
-__device__ __forceinline__ void team_fft(cx<T>* buf, const cx<T>* twn, LoadF load, int tl, int bar) {
-  constexpr int R1 = Radix3<N>::R1, R2 = Radix3<N>::R2, R3 = Radix3<N>::R3;
-  static_assert(R1 * R2 * R3 == N, "radices must multiply to N");
-  // twn: the per-pass tables of stockham_twiddles (pass 2 at 0, pass 3 at R1*R2)
-  team_stockham_pass<N, R1, 1, S, !IN_SMEM, TEAM, T>(buf, twn, load, tl, bar);
-  team_stockham_pass<N, R2, R1, S, false, TEAM, T>(buf, twn, load, tl, bar);
-  team_stockham_pass<N, R3, R1 * R2, S, false, TEAM, T>(buf, twn + R1 * R2, load, tl, bar);
-}
-// Entries of the per-pass twiddle tables used by team_fft: pass 2 (NS = R1,
-// radix R2) then pass 3 (NS = R1*R2, radix R3), each as [r][k] with entry
-// W_N^(k*r*N/(NS*R)).  Returns the length of the table (R1*R2 + R1*R2*R3).
-template <int N> __host__ __device__ constexpr int stockham_twiddle_len() {
-  return Radix3<N>::R1 * Radix3<N>::R2 + N;
-}
-// exponent (in units of 2 pi / N) of entry i of the table
-template <int N> __device__ __forceinline__ int stockham_twiddle_exp(int i) {
-  constexpr int R1 = Radix3<N>::R1, R2 = Radix3<N>::R2, R3 = Radix3<N>::R3;
-  if (i < R1 * R2) {
-    const int r = i / R1, k = i % R1;  // NS = R1, R = R2
-    return k * r * (N / (R1 * R2));
+  static __device__ __forceinline__ int col_off(int r, int i) {
+    if (R3 % C::PB == 0 || C::PB % R3 == 0) return i + i / C::PB;
+    return C::off(r * R3 + i) - C::off(r * R3);
   }
-  i -= R1 * R2;
-  const int r = i / (R1 * R2), k = i % (R1 * R2);  // NS = R1*R2, R = R3
-  return k * r * (N / (R1 * R2 * R3));
-}
-
-// Transform used by the fused kernel for a length: the two-pass warp form
-// unless its N2-point register DFT has 24 points or more (288, 384, 576,
-// 768), then the three-pass Stockham form (radices <= 12): the 24- and
-// 32-point register DFTs spill, and on B200 the three passes ran 6-31%
-// faster at 288-576.
-template <int N, class T> struct FusedPlan {
-  static constexpr bool three = (Split<N>::N2 >= 24);
-  static constexpr int BUF = three ? N : smem_fft_elems<N, false>(1);
 };
-// One transform by a team of TEAM threads (tl = index in the team, bar = the
-// team's named barrier; the two-pass warp form needs TEAM = 32).
-template <int N, int S, bool IN_SMEM, int TEAM, class T, class LoadF>
-__device__ __forceinline__ void fused_fft(cx<T>* buf, const cx<T>* twn, LoadF load, int tl, int bar) {
-  if constexpr (FusedPlan<N, T>::three) {
-    team_fft<N, S, IN_SMEM, TEAM, T>(buf, twn, load, tl, bar);
-  } else {
-    static_assert(TEAM == 32, "the two-pass transform is warp-synchronous");
-    warp_fft<N, S, IN_SMEM, T>(buf, twn, load);
-  }
+
+// Barrier of one team: the lanes `mask` of a warp, or the named barrier of a
+// team of two warps.
+template <int TP> __device__ __forceinline__ void team_sync(int bar, unsigned mask) {
+  if (TP <= 32) __syncwarp(mask);
+  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(TP) : "memory");
 }
 
 struct FusedArgs {
@@ -196,27 +285,12 @@ struct FusedArgs {
   const void* dEY;
   const int* clipflag;   // per level 1..nnz-1 (index z-1)
   const WallParams* wp;
-  double* divpart;  // [level][y] partial sums of divz, one writer each
-  double* sgspart;  // [level][y][6] partial SGS means (stage 1 with mnout)
+  double* divpart;  // [level][CTA][warp] partial sums of divz, one writer each
+  double* sgspart;  // [level][CTA][warp][6] partial SGS means (stage 1 with mnout)
   // learned closure: when lflag is set and *lflag != 0 the interior momentum
   // stresses are left to the network (the wall-model rows stay)
   const int* lflag;
   int zchunk;
-};
-
-template <int NSX> struct FusedCfg {
-  static constexpr int MX = 3 * NSX / 2;
-  static constexpr int NBUF = 11;  // 6 level slots (3 levels x 2), 4 work buffers, 1 carried tuw/tvw
-  // threads per transform: one warp.  (Two warps for the FP64 768-point
-  // plan double the resident warps but cap the 384-thread block at 168
-  // registers, which spills; on B200 that ran 9% slower.)
-  template <class T> static constexpr int team() { return 32; }
-  template <class T> static constexpr int threads() { return 6 * team<T>(); }
-  template <class T> static constexpr int buf() { return FusedPlan<MX, T>::BUF; }
-  // buffers + the twiddle table of length MX staged in shared memory
-  template <class T> static constexpr size_t smem() {
-    return ((size_t)NBUF * buf<T>() + MX + 64) * sizeof(cx<T>);
-  }
 };
 
 // Square root of the TKE in the FP32 form: the hardware approximation
@@ -230,297 +304,350 @@ template <> __device__ __forceinline__ float tke_sqrt<float>(float e) {
   return r;
 }
 
+// What bounds it: shared-memory wavefronts and issue slots, not HBM (15% of
+// its peak).  At 512x512x32 (768-point rows) FP32 runs the load/store data
+// path at 70% and issues 0.56 per scheduler and cycle, FP64 62% and 0.36 with
+// the FP64 pipe at 41%.  Before, autosorted rows of one warp per transform
+// and the window in shared memory left 6 (FP64) or 12 (FP32) warps per SM:
+// 1939 -> 1283 us (FP64), 887 -> 643 us (FP32), 827 -> 586 us (FP32, learned);
+// 64x64x64 FP64 168 -> 47 us.
 template <class T, int NSX>
-__global__ void __launch_bounds__(FusedCfg<NSX>::template threads<T>(), (sizeof(T) == 4) ? 2 : 1)
+__global__ void __launch_bounds__(FusedCfg<T, NSX>::THREADS, FusedCfg<T, NSX>::CTAS)
 k_row_fused(FusedArgs f, StageArgs a, const cx<T>* __restrict__ tw) {
-  constexpr int MX = 3 * NSX / 2;
-  constexpr int KX = NSX / 2;
-  constexpr int BUF = FusedCfg<NSX>::template buf<T>();
-  constexpr int TEAM = FusedCfg<NSX>::template team<T>();
+  using C = FusedCfg<T, NSX>;
+  constexpr int MX = C::MX, KX = C::KX, M1 = C::M1, R2 = C::R2, R3 = C::R3, TP = C::TP, TR = C::TR;
+  constexpr int BUF = C::BUF, SB = C::SB, PPT = C::PPT;
   extern __shared__ __align__(16) unsigned char smraw[];
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  // twiddles staged once per CTA in the layout each transform reads with
-  // consecutive lanes: [k1][n2] (two-pass) or the per-pass [r][k] tables
-  // (three-pass Stockham)
-  cx<T>* tws = sm + (size_t)11 * BUF;
+  cx<T>* tw1 = sm + (size_t)6 * C::ROWS * BUF;  // [k - 1][j]: W_(N/3)^(k j) (PFA) or W_N^(k j)
+  cx<T>* tw2 = tw1 + C::NT1 * M1;               // [r - 1][i]: W_M1^(r i)
   {
     const cx<T>* twg = tw + tw_off(MX);
-    if constexpr (FusedPlan<MX, T>::three) {
-      for (int i = threadIdx.x; i < stockham_twiddle_len<MX>(); i += blockDim.x)
-        tws[i] = twg[stockham_twiddle_exp<MX>(i) % MX];
-    } else {
-      constexpr int N1 = Split<MX>::N1, N2 = Split<MX>::N2;
-      for (int i = threadIdx.x; i < N1 * N2; i += blockDim.x) tws[i] = twg[(i / N2) * (i % N2)];
-    }
+    for (int i = threadIdx.x; i < C::NT1 * M1; i += C::THREADS)
+      tw1[i] = twg[(C::PFA ? 3 : 1) * (i / M1 + 1) * (i % M1)];
+    if (R3 > 1)
+      for (int i = threadIdx.x; i < (R2 - 1) * R3; i += C::THREADS) tw2[i] = twg[12 * (i / R3 + 1) * (i % R3)];
   }
   __syncthreads();
-  cx<T>* work[6];
-#pragma unroll
-  for (int i = 0; i < 4; i++) work[i] = sm + (size_t)(6 + i) * BUF;
-  cx<T>* carry = sm + (size_t)10 * BUF;  // (TUW, TVW) of level z-1
-  // level slots: slot s holds (U+iV) at sm + (2s)*BUF and (W+iE) at sm + (2s+1)*BUF
-  auto UVs = [&](int s) { return sm + (size_t)(2 * s) * BUF; };
-  auto WEs = [&](int s) { return sm + (size_t)(2 * s + 1) * BUF; };
 
   const int NZ = a.NZ, MY = a.MY;
-  const int y = blockIdx.x;
+  const int row = C::ROWS > 1 ? (int)threadIdx.x / TR : 0;
+  const int tr = C::ROWS > 1 ? (int)threadIdx.x % TR : (int)threadIdx.x;  // thread of the row
+  const int team = tr / TP, t = tr % TP;
+  const int y = blockIdx.x * C::ROWS + row;
   const int z0 = blockIdx.y * f.zchunk + 1;
   const int z1 = min(z0 + f.zchunk - 1, NZ);
   if (z0 > NZ) return;
-  // team w (threads [TEAM w, TEAM (w+1))) owns transform w of every phase
-  const int warp = threadIdx.x / TEAM, lane = threadIdx.x % TEAM;
-  const int bar = 1 + warp;
-  auto S = [](int q) { return Swz<T, MX>::f(q); };  // swizzled position of element q
-  const T kx0 = (T)a.kx0, dzm = (T)a.dzm, todzm = (T)a.todzm, emin = (T)a.emin;
+  const int lane = threadIdx.x & 31;
+  cx<T>* rowbuf = sm + (size_t)row * 6 * BUF;
+  cx<T>* buf = rowbuf + team * BUF;
+  const int bar = 1 + team;
+  const unsigned mask = TP >= 32 ? 0xffffffffu : ((1u << (TP & 31)) - 1u) << (lane & ~(TP - 1));
+
+  // pass 1: this thread's j and the lane of its mirror partner M1 - j.  A
+  // team of two warps splits j so that both are in the same warp.
+  int j, partner;
+  if (TP <= 32) {
+    j = t;
+    partner = (lane & ~(TP - 1)) | (t == 0 || t >= M1 ? t : M1 - t);
+  } else {
+    constexpr int H = M1 / 4;
+    const int l = t & 31;
+    if (t < 32) {
+      j = l < H ? l : (l == H ? 2 * H : l + 2 * H);
+      partner = (l == 0 || l == H || l >= 2 * H) ? l : 2 * H - l;
+    } else {
+      j = l < H ? H + l : l + H + 1;
+      partner = l >= 2 * H ? l : 2 * H - 1 - l;
+    }
+    if (l >= 2 * H) j = M1;
+  }
+  const bool act = (TP == M1) || j < M1;
+  if (!act) j = 0;
+  cx<T>* pj = buf + C::off(j);
+  const cx<T>* twj = tw1 + j;
+  cx<T> w3[3];  // W_3^(s(j) + 0, 1, 2), s(j) = j u mod 3 (PFA)
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    const int e = (j * Dft12Pfa<T, M1>::U + s) % 3;
+    w3[s] = mk(e ? (T)-0.5 : (T)1, e == 0 ? (T)0 : (e == 1 ? (T)1 : (T)-1) * (T)0.86602540378443864676372317075293618);
+  }
+
+  const T dzm = (T)a.dzm, todzm = (T)a.todzm, emin = (T)a.emin;
   const T xkmax = (T)a.xkmax, nu = (T)a.nu, c01 = (T)0.1 * (T)a.dsl;
   const WallParams& wp = *f.wp;
   // weight of the interior momentum stresses: 0 when the learned closure
   // supplies them (the wall rows stay)
   const bool learned = (f.lflag && f.lflag[0]);
   const T mom = learned ? (T)0 : (T)1;
+  auto xkk = [&](T sq) { return tmin(c01 * sq, xkmax) + nu; };  // from the square root of e
 
-  auto mixrow = [&](int j, int z) -> const cx<T>* {
-    return reinterpret_cast<const cx<T>*>(f.in.p[j]) + ((size_t)(z - 1) * MY + y) * KX;
+  const size_t zstride = (size_t)MY * KX;
+  auto mix = [&](int q, int z) -> const cx<T>* {
+    return reinterpret_cast<const cx<T>*>(f.in.p[q]) + (size_t)(z - 1) * zstride + (size_t)y * KX;
   };
-  // complex row Z = A + iB of two real c2r outputs from x-spectral rows A, B
-  // (optional i*kx on each; NULL = zero row)
-  auto c2r_load = [&](const cx<T>* A, bool ma, const cx<T>* B, bool mb, int n) -> cx<T> {
-    int k = -1;
-    bool mir = false;
-    if (n < KX) k = n;
-    else if (n > MX - KX) { k = MX - n; mir = true; }
-    if (k < 0) return zero_cx<T>();
-    cx<T> av = A ? A[k] : zero_cx<T>(), bv = B ? B[k] : zero_cx<T>();
-    T kk = kx0 * (T)k;
-    if (ma) av = mul_i(av) * kk;
-    if (mb) bv = mul_i(bv) * kk;
-    if (k == 0) { av.y = 0; bv.y = 0; }
-    if (mir) { av = conj(av); bv = conj(bv); }
-    return mk(av.x - bv.y, av.y + bv.x);
-  };
-  // inverse transform of one (A, B) pair into buf (by the calling team)
-  auto inv = [&](cx<T>* buf, const cx<T>* A, bool ma, const cx<T>* B, bool mb) {
-    fused_fft<MX, +1, false, TEAM, T>(buf, tws, [&](int n) { return c2r_load(A, ma, B, mb, n); }, lane, bar);
-  };
-  auto clipE = [&](cx<T>* we) {
-    for (int x = lane; x < MX; x += TEAM) we[S(x)].y = tmax(we[S(x)].y, emin);
-    team_sync<TEAM>(bar);
-  };
-  auto xkk = [&](T e) { return tmin(c01 * tke_sqrt(e), xkmax) + nu; };
+  // this team's inputs A + iB (array, i kx on A and on B) and outputs:
+  // -i kx a^ + b^ to array o1, a^ to o2, b^ to o3 (8: none)
+  auto pick = [&](unsigned table) { return (int)((table >> (4 * team)) & 15u); };
+  const int qa = pick(0x641040), qb = pick(learned ? 0x753362 : 0x753262);
+  const bool ma = (learned ? 0x34 : 0x34) >> team & 1, mb = !learned && team == 2;
+  const int o1 = pick(0x864820), o2 = pick(0x788318), o3 = pick(0x888588);
 
-  // ---- prologue: slots for levels z0-1 and z0, carried tuw/tvw of z0-1 ----
-  int sm1 = 0, s0 = 1, sp1 = 2;  // slots of z-1, z, z+1
-  {
-    // one transform per warp, described by (destination, A, ikx on A, B, ikx on B, clip E)
-    cx<T>* dst = nullptr;
-    const cx<T>* A = nullptr;
-    const cx<T>* B = nullptr;
-    bool ma = false, mb = false, ce = false;
-    const int zm = z0 - 1;
-    if (z0 == 1) {
-      if (warp == 0) { dst = UVs(s0); A = mixrow(0, 1); B = mixrow(2, 1); }
-      if (warp == 1) { dst = WEs(s0); A = mixrow(4, 1); B = mixrow(6, 1); ce = true; }
-    } else {
-      if (warp == 0) { dst = UVs(sm1); A = mixrow(0, zm); B = mixrow(2, zm); }
-      if (warp == 1) { dst = WEs(sm1); A = mixrow(4, zm); B = mixrow(6, min(zm, NZ - 1)); ce = true; }
-      if (warp == 2) { dst = UVs(s0); A = mixrow(0, z0); B = mixrow(2, z0); }
-      if (warp == 3) { dst = WEs(s0); A = z0 < NZ ? mixrow(4, z0) : nullptr; B = mixrow(6, min(z0, NZ - 1)); ce = true; }
-      if (warp == 4 && !learned) { dst = work[0]; A = mixrow(4, zm); ma = true; B = mixrow(5, zm); }  // WX + iWY at z0-1
-    }
-    if (dst) {
-      inv(dst, A, ma, B, mb);
-      if (ce) clipE(dst);
-    }
-  }
-  __syncthreads();
-  if (z0 == 1) {
-    for (int x = threadIdx.x; x < MX; x += blockDim.x) {
-      cx<T> uv = UVs(s0)[S(x)];
-      UVs(sm1)[S(x)] = zero_cx<T>();
-      WEs(sm1)[S(x)] = mk((T)0, WEs(s0)[S(x)].y);  // w(0) = 0, e(0) = e(1)
-      T tu, tv;
-      wall_stress<T>(wp.w[0], wp, a, 0, uv.x, uv.y, tu, tv);
-      carry[x] = mk(tu, tv);
-    }
-  } else if (learned) {
-    for (int x = threadIdx.x; x < MX; x += blockDim.x) carry[x] = zero_cx<T>();
-  } else {
-    for (int x = threadIdx.x; x < MX; x += blockDim.x) {
-      cx<T> uvm = UVs(sm1)[S(x)], uv0 = UVs(s0)[S(x)], wxy = work[0][S(x)];
-      T xk = xkk(WEs(sm1)[S(x)].y);
-      T uz = (uv0.x - uvm.x) * dzm, vz = (uv0.y - uvm.y) * dzm;
-      carry[x] = mk(-xk * (uz + wxy.x), -xk * (vz + wxy.y));
-    }
-  }
-  __syncthreads();
+  // the window at this thread's points: level z - 1 and level z
+  // (s: the square roots of e; FP32 takes them again, cheaper than the registers)
+  constexpr bool KEEP = sizeof(T) == 8;
+  T Um[PPT], Vm[PPT], Wm[PPT], Em[PPT], sm1[KEEP ? PPT : 1], tum[PPT], tvm[PPT];
+  T U0[PPT], V0[PPT], W0[PPT], E0[PPT], s0[KEEP ? PPT : 1];
 
-  double divz_part = 0.0;
-  double sgs_part[6] = {0, 0, 0, 0, 0, 0};
-  for (int z = z0; z <= z1; z++) {
+  // iteration z0 - 1 fills the window (levels z0 - 1 and z0)
+  for (int z = z0 - 1; z <= z1; z++) {
+    const bool pre = z < z0, top = z == NZ;
     const int le = z < NZ - 2 ? z : NZ - 2;
-    // ---- phase I: inverse transforms (one per warp) ----
+    // ---- phase I: inverse transforms ----
     {
-      cx<T>* dst = nullptr;
-      const cx<T>* A = nullptr;
-      const cx<T>* B = nullptr;
-      bool ma = false, mb = false, ce = false, zero = false;
-      switch (warp) {
-        case 0:  // U + iV at z+1
-          dst = UVs(sp1);
-          if (z + 1 <= NZ) { A = mixrow(0, z + 1); B = mixrow(2, z + 1); } else zero = true;
-          break;
-        case 1:  // W + iE at z+1 (w = 0 above nnz-1, e clamped to level nnz-1)
-          dst = WEs(sp1);
-          A = (z + 1 <= NZ - 1) ? mixrow(4, z + 1) : nullptr;
-          B = mixrow(6, min(z + 1, NZ - 1));
-          ce = true;
-          break;
-        case 2:
-          if (learned) { dst = work[0]; A = mixrow(0, z); ma = true; B = mixrow(3, z); }  // UX + iVY
-          else { dst = work[0]; A = mixrow(0, z); B = mixrow(2, z); ma = mb = true; }     // UX + iVX
-          break;
-        case 3: if (!learned) { dst = work[1]; A = mixrow(1, z); B = mixrow(3, z); } break;  // UY + iVY
-        case 4:                                                                              // WX + iWY
-          if (learned) break;
-          dst = work[2];
-          if (z <= NZ - 1) { A = mixrow(4, z); ma = true; B = mixrow(5, z); } else zero = true;
-          break;
-        default:  // EX + iEY at le
-          if (z <= NZ - 1) { dst = work[3]; A = mixrow(6, le); ma = true; B = mixrow(7, le); }
-          break;
-      }
-      if (zero) {
-        for (int x = lane; x < MX; x += TEAM) dst[x] = zero_cx<T>();
-        team_sync<TEAM>(bar);
-      } else if (dst) {
-        inv(dst, A, ma, B, mb);
-        if (ce) clipE(dst);
-      }
-    }
-    __syncthreads();
-    // L2 prefetch (one thread, nothing waits on it) of the rows the next
-    // level's phase I reads from DRAM: U, V, W, E at z+2 and VY, UY, WY, EY at
-    // z+1 (U, V, W, E at z+1 were this level's window rows and are in L2)
-    if (threadIdx.x == 0 && z + 1 <= z1) {
-      constexpr unsigned RB = KX * sizeof(cx<T>);
-      if (z + 2 <= NZ) { tma::prefetch_l2(mixrow(0, z + 2), RB); tma::prefetch_l2(mixrow(2, z + 2), RB); }
-      if (z + 2 <= NZ - 1) { tma::prefetch_l2(mixrow(4, z + 2), RB); tma::prefetch_l2(mixrow(6, z + 2), RB); }
-      tma::prefetch_l2(mixrow(3, z + 1), RB);
-      if (!learned) tma::prefetch_l2(mixrow(1, z + 1), RB);
-      if (z + 1 <= NZ - 1) {
-        if (!learned) tma::prefetch_l2(mixrow(5, z + 1), RB);
-        tma::prefetch_l2(mixrow(7, min(z + 1, NZ - 2)), RB);
-      }
-    }
-    // ---- phase II: fluxes (k_flux) ----
-    // the forward transforms of F+iPe and H reuse the z-1 window slots,
-    // whose rows are dead once each point has read them
-    work[4] = UVs(sm1);
-    work[5] = WEs(sm1);
-    const bool top = (z == NZ);
-    const bool clip = (!top) && f.clipflag[le - 1];
-    const T* dEX = reinterpret_cast<const T*>(f.dEX) + ((size_t)(le - 1) * MY + y) * MX;
-    const T* dEY = reinterpret_cast<const T*>(f.dEY) + ((size_t)(le - 1) * MY + y) * MX;
-    for (int x = threadIdx.x; x < MX; x += blockDim.x) {
-      const cx<T> uvm = UVs(sm1)[S(x)], uv0 = UVs(s0)[S(x)], uv1 = UVs(sp1)[S(x)];
-      const cx<T> wem = WEs(sm1)[S(x)], we0 = WEs(s0)[S(x)], we1 = WEs(sp1)[S(x)];
-      // learned: work[0] holds (ux, vy); the other gradients are not needed
-      const cx<T> w0 = work[0][S(x)];
-      const cx<T> dxv = learned ? mk(w0.x, (T)0) : w0;
-      const cx<T> dyv = learned ? mk((T)0, w0.y) : work[1][S(x)];
-      const cx<T> wxy = learned ? zero_cx<T>() : work[2][S(x)];
-      cx<T> exy = top ? zero_cx<T>() : work[3][S(x)];
-      if (clip) { exy.x += dEX[x]; exy.y += dEY[x]; }
-      const cx<T> tprev = carry[x];
-      const T U0 = uv0.x, V0 = uv0.y, Um = uvm.x, Vm = uvm.y, U1 = uv1.x, V1 = uv1.y;
-      const T W0 = we0.x, Wm = wem.x, W1 = we1.x, E0 = we0.y, Em = wem.y, E1 = we1.y;
-      const T ux = dxv.x, vx = dxv.y, uy = dyv.x, vy = dyv.y;
-      const T xkm = xkk(Em), xk0 = xkk(E0);
-      const T s = mom * (xkm + xk0);
-      const T tuu = -s * ux, tvv = -s * vy, tuv = -s * (uy + vx) * (T)0.5;
-      T tuw0, tvw0;
-      if (top) {
-        wall_stress<T>(wp.w[1], wp, a, 1, U0, V0, tuw0, tvw0);
-      } else {
-        const T uz = (U1 - U0) * dzm, vz = (V1 - V0) * dzm;
-        tuw0 = -mom * xk0 * (uz + wxy.x);
-        tvw0 = -mom * xk0 * (vz + wxy.y);
-      }
-      const T wz0 = (W0 - Wm) * dzm;
-      const T tww0 = -s * wz0;
-      const T A = U0 * U0 + tuu, B = U0 * V0 + tuv, C = V0 * V0 + tvv;
-      const T Pu = -((U1 + U0) * W0 - (Um + U0) * Wm) * todzm + (T)a.forcing - (tuw0 - tprev.x) * dzm;
-      const T Pv = -((V1 + V0) * W0 - (Vm + V0) * Wm) * todzm - (tvw0 - tprev.y) * dzm;
-      work[0][S(x)] = mk(A, Pu);
-      work[1][S(x)] = mk(B, Pv);
-      if (!top) {
-        const T xkp = xkk(E1);
-        const T wz1 = (W1 - W0) * dzm;
-        const T tww1 = -mom * (xk0 + xkp) * wz1;
-        const T D = (T)0.5 * (U0 + U1) * W0 + tuw0;
-        const T G = (T)0.5 * (V0 + V1) * W0 + tvw0;
-        const T hp = (T)0.5 * (W1 + W0), hm = (T)0.5 * (W0 + Wm);
-        const T Pw = -(hp * hp - hm * hm) * dzm - (tww1 - tww0) * dzm;
-        const T F = (T)0.5 * E0 * (U0 + U1) - (T)2 * xk0 * exy.x;
-        const T H = (T)0.5 * E0 * (V0 + V1) - (T)2 * xk0 * exy.y;
-        const T Pe = -(W1 * E1 - Wm * Em) * todzm +
-                     ((xkp + xk0) * (E1 - E0) - (xk0 + xkm) * (E0 - Em)) * (T)a.dzm2 - (T)a.ceps * E0 * tke_sqrt(E0);
-        work[2][S(x)] = mk(C, G);
-        work[3][S(x)] = mk(D, Pw);
-        work[4][S(x)] = mk(F, Pe);
-        work[5][S(x)] = mk(H, (T)0);
-      } else {
-        work[2][S(x)] = mk(C, (T)0);
-      }
-      carry[x] = mk(tuw0, tvw0);
-      const T d = ux + vy + wz0;
-      divz_part += (double)(d * d);
-      if (a.mnout_sgs) {
-        sgs_part[0] += (double)tuu; sgs_part[1] += (double)tvv; sgs_part[2] += (double)tuv;
-        sgs_part[3] += (double)tww0; sgs_part[4] += (double)tuw0; sgs_part[5] += (double)tvw0;
-      }
-    }
-    __syncthreads();
-    // per-level statistics of this row
-    {
-      const size_t slot = (size_t)(z - 1) * MY + y;
-      double v1[1] = {divz_part};
-      block_sum_store<1>(v1, f.divpart + slot);
-      divz_part = 0.0;
-      if (a.mnout_sgs) {
-        __syncthreads();
-        block_sum_store<6>(sgs_part, f.sgspart + slot * 6);
+      // team 0: U + iV at z + 1; 1: W + iE at z + 1 (w = 0 above nnz - 1, e
+      // clamped to level nnz - 1); 2: UX + iVX (learned: UX + iVY); 3: UY +
+      // iVY; 4: WX + iWY; 5: EX + iEY at le.  While filling the window teams
+      // 2 and 3 take U + iV and W + iE at z = z0 - 1.
+      const bool fill = pre && (team == 2 || team == 3);
+      const int ja = fill ? 4 * (team - 2) : qa, jb = fill ? 4 * (team - 2) + 2 : qb;
+      const bool ia = ma && !fill, ib = mb && !fill;
+      const int za = team < 2 ? z + 1 : (team == 5 ? le : z), zb = (jb == 6) ? min(za, NZ - 1) : za;
+      const bool on = team < 2 ? !top
+                               : team == 2 ? z >= 1
+                                           : team == 3 ? (pre ? z >= 1 : !learned)
+                                                       : team == 4 ? (!learned && z >= 1 && !top) : (!pre && !top);
+      const bool hasA = !(ja == 4 && za > NZ - 1);
+      if (on) {
+        const cx<T>* A = mix(ja, hasA ? za : 1) + j;
+        const cx<T>* B = mix(jb, zb) + j;
+        // modes k = j + M1 m of Z = A + iB and their mirror images
+        cx<T> x[8], mir[4];
 #pragma unroll
-        for (int q = 0; q < 6; q++) sgs_part[q] = 0.0;
-      }
-    }
-    // ---- phase III: forward transforms, -d/dx, truncation to kx < nx/2 ----
-    if (!(top && warp >= 3)) {
-      cx<T>* buf = work[warp];
-      fused_fft<MX, -1, true, TEAM, T>(buf, tws, NoLoad{}, lane, bar);
-      const size_t orow = ((size_t)(z - 1) * MY + y) * KX;
-      auto O = [&](int j) { return reinterpret_cast<cx<T>*>(f.out.p[j]) + orow; };
-      for (int k = lane; k < KX; k += TEAM) {
-        cx<T> zk = buf[S(k)], zmr = conj(buf[S((MX - k) % MX)]);
-        cx<T> ah = (zk + zmr) * (T)0.5;
-        cx<T> dd = zk - zmr;
-        cx<T> bh = mk(dd.y * (T)0.5, -dd.x * (T)0.5);
-        T kk = kx0 * (T)k;
-        cx<T> dxa = mk(kk * ah.y, -kk * ah.x);  // -i kx a^
-        switch (warp) {
-          case 0: O(0)[k] = dxa + bh; break;                          // Xu1
-          case 1: O(2)[k] = dxa + bh; O(1)[k] = ah; break;            // Xv1, Xu2
-          case 2: O(3)[k] = ah; if (!top) O(5)[k] = bh; break;        // Xv2, Xw2
-          case 3: O(4)[k] = dxa + bh; break;                          // Xw1
-          case 4: O(6)[k] = dxa + bh; break;                          // Xe1
-          default: O(7)[k] = ah; break;                               // Xe2
+        for (int m = 0; m < 4; m++) {
+          const int k = j + M1 * m;
+          cx<T> av = hasA ? A[M1 * m] : zero_cx<T>(), bv = B[M1 * m];
+          const T kk = (T)a.kx0 * (T)k;
+          if (ia) av = mul_i(av) * kk;
+          if (ib) bv = mul_i(bv) * kk;
+          if (m == 0 && j == 0) { av.y = 0; bv.y = 0; }
+          x[m] = mk(av.x - bv.y, av.y + bv.x);
+          mir[m] = mk(av.x + bv.y, bv.x - av.y);
+        }
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          const cx<T> r = shfl_cx(mask, mir[m], partner), own = m < 3 ? mir[m + 1] : zero_cx<T>();
+          x[7 - m] = j == 0 ? own : r;
+        }
+        if (act) {
+          cx<T> v[12];
+          if constexpr (C::PFA) {
+            Dft12Pfa<T, M1>::padded(x, w3, v);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              const cx<T> w = k ? conj(twj[(k - 1) * M1]) : zero_cx<T>();
+#pragma unroll
+              for (int b = k; b < 12; b += 4) pj[b * SB] = k ? cmul(v[b], w) : v[b];
+            }
+          } else {
+            dft12_padded<T>(x, v);
+            pj[0] = v[0];
+#pragma unroll
+            for (int b = 1; b < 12; b++) pj[b * SB] = cmul(v[b], conj(twj[(b - 1) * M1]));
+          }
+        }
+        team_sync<TP>(bar, mask);
+        RowPasses<T, NSX, true>::pass2(buf, tw2, t);
+        if (R3 > 1) {
+          team_sync<TP>(bar, mask);
+          RowPasses<T, NSX, true>::pass3(buf, t);
         }
       }
     }
     __syncthreads();
-    // rotate the window: z -> z-1, z+1 -> z
-    const int t = sm1;
-    sm1 = s0; s0 = sp1; sp1 = t;
+    if (pre) {
+#pragma unroll
+      for (int q = 0; q < PPT; q++) {
+        const int n = tr + TR * q;
+        if (PPT * TR > MX && n >= MX) break;
+        const cx<T>* p = rowbuf + C::at(n);
+        const cx<T> uv = p[0], we = p[BUF];
+        U0[q] = uv.x; V0[q] = uv.y; W0[q] = we.x; E0[q] = tmax(we.y, emin);
+        if (KEEP) s0[q] = tke_sqrt(E0[q]);
+        if (z == 0) {  // w(0) = 0, e(0) = e(1)
+          Um[q] = Vm[q] = Wm[q] = (T)0;
+          Em[q] = E0[q];
+          if (KEEP) sm1[q] = s0[q];
+          wall_stress<T>(wp.w[0], wp, a, 0, uv.x, uv.y, tum[q], tvm[q]);
+        } else {
+          const cx<T> uvm = p[2 * BUF], wem = p[3 * BUF];
+          const cx<T> wxy = learned ? zero_cx<T>() : p[4 * BUF];
+          Um[q] = uvm.x; Vm[q] = uvm.y; Wm[q] = wem.x; Em[q] = tmax(wem.y, emin);
+          const T sq = tke_sqrt(Em[q]), xk = xkk(sq);
+          if (KEEP) sm1[q] = sq;
+          tum[q] = -mom * xk * ((uv.x - uvm.x) * dzm + wxy.x);
+          tvm[q] = -mom * xk * ((uv.y - uvm.y) * dzm + wxy.y);
+        }
+      }
+      __syncthreads();
+      continue;
+    }
+    // L2 prefetch (one thread, nothing waits on it) of the rows the next
+    // level's phase I reads from DRAM: U, V, W, E at z+2 and VY, UY, WY, EY at
+    // z+1 (U, V, W, E at z+1 were this level's window rows and are in L2)
+    if (threadIdx.x == 0 && z + 1 <= z1) {
+      constexpr unsigned RB = C::ROWS * KX * sizeof(cx<T>);
+      if (z + 2 <= NZ) { tma::prefetch_l2(mix(0, z + 2), RB); tma::prefetch_l2(mix(2, z + 2), RB); }
+      if (z + 2 <= NZ - 1) { tma::prefetch_l2(mix(4, z + 2), RB); tma::prefetch_l2(mix(6, z + 2), RB); }
+      tma::prefetch_l2(mix(3, z + 1), RB);
+      if (!learned) tma::prefetch_l2(mix(1, z + 1), RB);
+      if (z + 1 <= NZ - 1) {
+        if (!learned) tma::prefetch_l2(mix(5, z + 1), RB);
+        tma::prefetch_l2(mix(7, min(z + 1, NZ - 2)), RB);
+      }
+    }
+    // ---- phase II: fluxes (k_flux) ----
+    double divz_part = 0.0;
+    double sgs_part[6] = {0, 0, 0, 0, 0, 0};
+    const bool clip = (!top) && f.clipflag[le - 1];
+#pragma unroll
+    for (int q = 0; q < PPT; q++) {
+      const int n = tr + TR * q;
+      if (PPT * TR > MX && n >= MX) break;
+      cx<T>* p = rowbuf + C::at(n);
+      // learned: buffer 2 holds (ux, vy); the other gradients are not needed
+      const cx<T> d2 = p[2 * BUF];
+      const cx<T> d3 = learned ? mk((T)0, d2.y) : p[3 * BUF];
+      const T ux = d2.x, vx = learned ? (T)0 : d2.y, uy = d3.x, vy = d3.y;
+      const T sq0 = KEEP ? s0[q] : tke_sqrt(E0[q]), sqm = KEEP ? sm1[q] : tke_sqrt(Em[q]);
+      const T xkm = xkk(sqm), xk0 = xkk(sq0);
+      const T s = mom * (xkm + xk0);
+      const T tuu = -s * ux, tvv = -s * vy, tuv = -s * (uy + vx) * (T)0.5;
+      const T wz0 = (W0[q] - Wm[q]) * dzm;
+      const T tww0 = -s * wz0;
+      const T A = U0[q] * U0[q] + tuu, B = U0[q] * V0[q] + tuv, Cc = V0[q] * V0[q] + tvv;
+      T tuw0, tvw0, U1 = (T)0, V1 = (T)0;
+      const T d = ux + vy + wz0;
+      divz_part += (double)(d * d);
+      if (!top) {
+        const cx<T> uv1 = p[0], we1 = p[BUF];
+        const cx<T> wxy = learned ? zero_cx<T>() : p[4 * BUF];
+        cx<T> exy = p[5 * BUF];
+        if (clip) {
+          const size_t o = ((size_t)(le - 1) * MY + y) * MX + C::x_of(n);
+          exy.x += reinterpret_cast<const T*>(f.dEX)[o];
+          exy.y += reinterpret_cast<const T*>(f.dEY)[o];
+        }
+        U1 = uv1.x; V1 = uv1.y;
+        const T W1 = we1.x, E1 = tmax(we1.y, emin), sq1 = tke_sqrt(E1), xkp = xkk(sq1);
+        tuw0 = -mom * xk0 * ((U1 - U0[q]) * dzm + wxy.x);
+        tvw0 = -mom * xk0 * ((V1 - V0[q]) * dzm + wxy.y);
+        const T wz1 = (W1 - W0[q]) * dzm;
+        const T tww1 = -mom * (xk0 + xkp) * wz1;
+        const T D = (T)0.5 * (U0[q] + U1) * W0[q] + tuw0;
+        const T G = (T)0.5 * (V0[q] + V1) * W0[q] + tvw0;
+        const T hp = (T)0.5 * (W1 + W0[q]), hm = (T)0.5 * (W0[q] + Wm[q]);
+        const T Pw = -(hp * hp - hm * hm) * dzm - (tww1 - tww0) * dzm;
+        const T F = (T)0.5 * E0[q] * (U0[q] + U1) - (T)2 * xk0 * exy.x;
+        const T H = (T)0.5 * E0[q] * (V0[q] + V1) - (T)2 * xk0 * exy.y;
+        const T Pe = -(W1 * E1 - Wm[q] * Em[q]) * todzm +
+                     ((xkp + xk0) * (E1 - E0[q]) - (xk0 + xkm) * (E0[q] - Em[q])) * (T)a.dzm2 -
+                     (T)a.ceps * E0[q] * sq0;
+        p[2 * BUF] = mk(Cc, G);
+        p[3 * BUF] = mk(D, Pw);
+        p[4 * BUF] = mk(F, Pe);
+        p[5 * BUF] = mk(H, (T)0);
+        const T Pu = -((U1 + U0[q]) * W0[q] - (Um[q] + U0[q]) * Wm[q]) * todzm + (T)a.forcing - (tuw0 - tum[q]) * dzm;
+        const T Pv = -((V1 + V0[q]) * W0[q] - (Vm[q] + V0[q]) * Wm[q]) * todzm - (tvw0 - tvm[q]) * dzm;
+        p[0] = mk(A, Pu);
+        p[BUF] = mk(B, Pv);
+        if (a.mnout_sgs) {
+          sgs_part[0] += (double)tuu; sgs_part[1] += (double)tvv; sgs_part[2] += (double)tuv;
+          sgs_part[3] += (double)tww0; sgs_part[4] += (double)tuw0; sgs_part[5] += (double)tvw0;
+        }
+        Um[q] = U0[q]; Vm[q] = V0[q]; Wm[q] = W0[q]; Em[q] = E0[q]; tum[q] = tuw0; tvm[q] = tvw0;
+        if (KEEP) { sm1[q] = sq0; s0[q] = sq1; }
+        U0[q] = U1; V0[q] = V1; W0[q] = W1; E0[q] = E1;
+      } else {
+        wall_stress<T>(wp.w[1], wp, a, 1, U0[q], V0[q], tuw0, tvw0);
+        p[2 * BUF] = mk(Cc, (T)0);
+        const T Pu = (Um[q] + U0[q]) * Wm[q] * todzm + (T)a.forcing - (tuw0 - tum[q]) * dzm;
+        const T Pv = (Vm[q] + V0[q]) * Wm[q] * todzm - (tvw0 - tvm[q]) * dzm;
+        p[0] = mk(A, Pu);
+        p[BUF] = mk(B, Pv);
+        if (a.mnout_sgs) {
+          sgs_part[0] += (double)tuu; sgs_part[1] += (double)tvv; sgs_part[2] += (double)tuv;
+          sgs_part[3] += (double)tww0; sgs_part[4] += (double)tuw0; sgs_part[5] += (double)tvw0;
+        }
+      }
+    }
+    // statistics of this level: one partial sum per warp
+    {
+      const size_t slot = ((size_t)(z - 1) * gridDim.x + blockIdx.x) * C::WARPS + (threadIdx.x >> 5);
+      for (int o = 16; o > 0; o >>= 1) divz_part += __shfl_xor_sync(0xffffffffu, divz_part, o);
+      if (lane == 0) f.divpart[slot] = divz_part;
+      if (a.mnout_sgs) {
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+          for (int o = 16; o > 0; o >>= 1) sgs_part[q] += __shfl_xor_sync(0xffffffffu, sgs_part[q], o);
+          if (lane == 0) f.sgspart[slot * 6 + q] = sgs_part[q];
+        }
+      }
+    }
+    __syncthreads();
+    // ---- phase III: forward transforms, -d/dx, truncation to kx < nx/2 ----
+    if (!(top && team >= 3)) {
+      if (R3 > 1) {
+        RowPasses<T, NSX, false>::pass3(buf, t);
+        team_sync<TP>(bar, mask);
+      }
+      RowPasses<T, NSX, false>::pass2(buf, tw2, t);
+      team_sync<TP>(bar, mask);
+      cx<T> zf[8];  // outputs 0..3 and 8..11
+      {
+        cx<T> v[12];
+        if constexpr (C::PFA) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            const cx<T> w = k ? twj[(k - 1) * M1] : zero_cx<T>();
+#pragma unroll
+            for (int b = k; b < 12; b += 4) v[b] = k ? cmul(pj[b * SB], w) : pj[b * SB];
+          }
+          Dft12Pfa<T, M1>::forward(v, w3, zf);
+        } else {
+          v[0] = pj[0];
+#pragma unroll
+          for (int b = 1; b < 12; b++) v[b] = cmul(pj[b * SB], twj[(b - 1) * M1]);
+          cx<T> o[12];
+          dft12_forward<T>(v, o);
+#pragma unroll
+          for (int m = 0; m < 4; m++) { zf[m] = o[m]; zf[4 + m] = o[8 + m]; }
+        }
+      }
+      const size_t orow = (size_t)(z - 1) * zstride + (size_t)y * KX + j;
+      auto O = [&](int q) { return reinterpret_cast<cx<T>*>(f.out.p[q & 7]) + orow; };
+      cx<T>* const p1 = O(o1);
+      cx<T>* const p2 = O(o2);
+      cx<T>* const p3 = O(o3);
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        const cx<T> zk = zf[m];
+        const cx<T> other = shfl_cx(mask, zf[7 - m], partner);
+        const cx<T> zmr = conj(j == 0 ? zf[m ? 8 - m : 0] : other);
+        if (!act) continue;
+        const int k = j + M1 * m;
+        const cx<T> ah = (zk + zmr) * (T)0.5;
+        const cx<T> dd = zk - zmr;
+        const cx<T> bh = mk(dd.y * (T)0.5, -dd.x * (T)0.5);
+        const T kk = (T)a.kx0 * (T)k;
+        const cx<T> dxa = mk(kk * ah.y, -kk * ah.x);  // -i kx a^
+        if (o1 < 8) p1[M1 * m] = dxa + bh;
+        if (o2 < 8) p2[M1 * m] = ah;
+        if (o3 < 8 && !top) p3[M1 * m] = bh;
+      }
+    }
+    // no barrier here: the next level's pass 1 writes the elements this
+    // thread's pass 1 read, in the same buffer
   }
 }
 

@@ -194,6 +194,31 @@ def test_fused_row_plans_at_production_widths(gpu_lib, product, n):
     assert relerr(fg["e"], fo["e"]) < 2e-5, n
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(16, 32, 4), (32, 16, 9), (64, 16, 5), (96, 32, 7), (128, 16, 5), (192, 16, 5),
+                                      (256, 16, 4), (384, 16, 4), (512, 16, 5)])
+def test_fused_row_plans_with_clipped_tke(gpu_lib, product, nx, ny, nz):
+    """Every row plan of the fused kernel (padded rows 24 to 768, odd level
+    counts) with a TKE whose expansion the floor clips: the correction terms
+    are read at the permuted position of each point.  Tolerances of the
+    unclipped stage tests."""
+    rng = np.random.default_rng(nx + nz)
+    e = 1e-3 * rng.random((nz, ny, nx)) ** 4
+    for precision, tol in ((8, 1e-11), (4, 2e-5)):
+        o, g, f = make_pair(product, nx, ny, nz, precision=precision, amp=0.3)
+        o.set_fields(e=e)
+        o.deal_fields()
+        f = o.get_fields()
+        g.upload(f["u"], f["v"], f["w"], f["e"], f["p"])
+        for s in (1, 2):
+            o.stage(0, 1, s)
+            g.stage(0, True, s)
+        fo, fg = o.get_fields(), g.download()
+        vscale = np.abs(fo["u"]).max()
+        for k in "uvw":
+            assert relerr(fg[k], fo[k], vscale) < tol, (precision, k)
+        assert relerr(fg["e"], fo["e"]) < tol, precision
+
+
 def test_mixed_precision_envelope(gpu_lib, product):
     o, g, f = make_pair(product, 64, 64, 32, precision=4, amp=0.1)
     for it in range(3):
