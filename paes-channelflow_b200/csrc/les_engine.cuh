@@ -256,7 +256,8 @@ struct Engine : EngineBase {
     size_t ns = nm * NZ;
     for (auto* b : {&uh, &vh, &wh, &ruo, &rvo, &rwo, &run, &rvn, &rwn}) b->alloc(ns);
     for (auto* b : {&mu, &mv, &mru, &mrv}) b->alloc(NZ);
-    ph.alloc(ns); rscr.alloc(ns); dscr.alloc(ns);
+    ph.alloc(ns);
+    if (NZ > kPressMaxNZ) { rscr.alloc(ns); dscr.alloc(ns); }  // not inside a graph capture
     e.alloc(ps * (NZ + 2)); re.alloc(ps * NZ);
     Xe.alloc(ns); rem.alloc(ns);
     for (auto& b : mixed) b.alloc(nmix * NZ);
@@ -909,15 +910,47 @@ struct Engine : EngineBase {
     launch(k_e_update_phys<T>, dim3(cdiv(ps * (NZ - 1), 256)), dim3(256), 0, st, e.p + ps, (const T*)re.p,
            ps * (NZ - 1), (T)dtab1, (T)cfg.emin);
   }
-  void press_kernel(const StageArgs& a, bool rhs_in_ph) {
-    if (rhs_in_ph)
-      launch(k_press<T, true>, dim3(cdiv(nm, 128)), dim3(128), 0, st, (const cx<T>*)uh.p, (const cx<T>*)vh.p,
-             (const cx<T>*)wh.p, (const cx<T>*)ruo.p, (const cx<T>*)rvo.p, (const cx<T>*)rwo.p, (const cx<T>*)run.p,
-             (const cx<T>*)rvn.p, (const cx<T>*)rwn.p, ph.p, dscr.p, rscr.p, a);
-    else
-      launch(k_press<T, false>, dim3(cdiv(nm, 128)), dim3(128), 0, st, (const cx<T>*)uh.p, (const cx<T>*)vh.p,
-             (const cx<T>*)wh.p, (const cx<T>*)ruo.p, (const cx<T>*)rvo.p, (const cx<T>*)rwo.p, (const cx<T>*)run.p,
-             (const cx<T>*)rvn.p, (const cx<T>*)rwn.p, ph.p, dscr.p, rscr.p, a);
+  // Pressure solve, with the update of u, v, w and their tendencies when
+  // `update` (the split entry points solve with the right-hand side in ph and
+  // update later).  k_press takes 32 modes a block where the blocks still
+  // fill the device and the inputs of one block per SM stay within about half
+  // of L2 (their second read, for the update, then hits it); else 16, whose
+  // blocks hold half as much and split a column into twice the chunks.  Solve
+  // and update, 16 / 32 modes, against a thread per column and a separate
+  // update: 512x512x64 mixed 428 / 313, 359 us; 384x384x192 mixed 557 / 481,
+  // 718; 256x256x256 mixed 317 / 367, 670; 256x256x128 FP64 223 / 235, 465;
+  // 512x512x256 mixed 1264 / 1473, 1413, FP64 1815 / 2720, 2305; 64x64x64
+  // FP64 14 / 18, 130.  (8 modes: 64-byte rows, 2280 and 2340 us at
+  // 512x512x256.)  More than kPressMaxNZ levels take the one-thread sweep.
+  static constexpr int kPressMaxNZ = 512;
+  template <int MODES, bool RHS, bool UPD> void press_launch(const StageArgs& a) {
+    const int L = (int)cdiv(NZ, 512 / MODES);  // levels of a chunk
+    const int threads = (int)cdiv((size_t)MODES * cdiv(NZ, L), 32) * 32;
+    const size_t smem = (size_t)L * threads * (sizeof(cx<double>) + sizeof(double));
+    set_smem_limit((const void*)k_press<T, MODES, RHS, UPD>, smem);  // the kernel has static shared memory too
+    launch(k_press<T, MODES, RHS, UPD>, dim3((unsigned)(nm / MODES)), dim3((unsigned)threads), smem, st, uh.p, vh.p, wh.p,
+           ruo.p, rvo.p, rwo.p, (const cx<T>*)run.p, (const cx<T>*)rvn.p, (const cx<T>*)rwn.p, ph.p, mu.p, mv.p, mru.p,
+           mrv.p, a, L, err.p);
+  }
+  template <bool RHS, bool UPD> void press_pick(const StageArgs& a) {
+    const size_t inputs = (size_t)32 * NZ * 9 * sizeof(cx<T>) * nsm;  // of one 32-mode block per SM
+    if (nm % 32 == 0 && nm / 32 >= (size_t)nsm && NZ <= 256 && inputs <= (size_t)72 << 20) press_launch<32, RHS, UPD>(a);
+    else press_launch<16, RHS, UPD>(a);
+  }
+  void press_kernel(const StageArgs& a, bool rhs_in_ph, bool update) {
+    if (NZ <= kPressMaxNZ) {
+      if (rhs_in_ph) press_pick<true, false>(a);
+      else press_pick<false, true>(a);
+      return;
+    }
+    auto old = [&](auto k) {
+      launch(k, dim3(cdiv(nm, 128)), dim3(128), 0, st, (const cx<T>*)uh.p, (const cx<T>*)vh.p, (const cx<T>*)wh.p,
+             (const cx<T>*)ruo.p, (const cx<T>*)rvo.p, (const cx<T>*)rwo.p, (const cx<T>*)run.p, (const cx<T>*)rvn.p,
+             (const cx<T>*)rwn.p, ph.p, dscr.p, rscr.p, a);
+    };
+    if (rhs_in_ph) old(k_press_long<T, true>);
+    else old(k_press_long<T, false>);
+    if (update) update_kernel(a, run.p, rvn.p, rwn.p);
   }
   void update_kernel(const StageArgs& a, const cx<T>* rnu, const cx<T>* rnv, const cx<T>* rnw) {
     launch(k_update<T>, dim3(cdiv(nm, 128), NZ), dim3(128), 0, st, uh.p, vh.p, wh.p, (const cx<T>*)ruo.p,
@@ -954,7 +987,7 @@ struct Engine : EngineBase {
   void press() override {
     if (phase != 2) throw std::logic_error("press called before comprhs");
     StageArgs a = args(last_dtab1, 0.0, 0.0, 0, 0);
-    press_kernel(a, true);
+    press_kernel(a, true, false);
     phase = 3;
   }
   void comp2(double dtab1) override {
@@ -971,8 +1004,7 @@ struct Engine : EngineBase {
     StageArgs a = args(dtab1, dtab2, xkmax, istage != 1, mnout && istage == 1);
     comp1_kernels(a);
     e_update(dtab1);
-    press_kernel(a, false);
-    update_kernel(a, run.p, rvn.p, rwn.p);
+    press_kernel(a, false, true);
   }
   void stage(bool mnout, int istage, double dtab1, double dtab2, double xkmax) override {
     if (phase != 0) throw std::logic_error("stage called inside a split comp1..comp2 sequence");
@@ -1184,8 +1216,7 @@ struct Engine : EngineBase {
     LES_CUDA(cudaMemsetAsync(re.p, 0, re.n * sizeof(T), st));
     // one projection: comprhs + press + comp2 with dtab1 = 1, zero tendencies
     StageArgs a = args(1.0, 0.0, 0.0, 0, 0);
-    press_kernel(a, false);
-    update_kernel(a, run.p, rvn.p, rwn.p);
+    press_kernel(a, false, true);
     for (auto* b : {&ruo, &rvo, &rwo}) LES_CUDA(cudaMemsetAsync(b->p, 0, b->n * sizeof(cx<T>), st));
     for (auto* b : {&mru, &mrv}) LES_CUDA(cudaMemsetAsync(b->p, 0, NZ * sizeof(double), st));
     LES_CUDA(cudaMemsetAsync(ph.p, 0, ph.n * sizeof(cx<double>), st));

@@ -39,7 +39,7 @@ struct DeviceTables {
   void* tw32 = nullptr;
 };
 std::map<int, DeviceTables> g_tables;
-std::set<std::pair<const void*, int>> g_smem_set;
+std::map<std::pair<const void*, int>, size_t> g_smem_set;  // largest dynamic shared memory asked for
 }  // namespace
 
 // Twiddle tables of the current (or given) device, built on first use:
@@ -84,9 +84,10 @@ void set_smem_limit(const void* func, size_t bytes) {
   int dev;
   LES_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(g_mu);
-  if (g_smem_set.count({func, dev})) return;
+  size_t& have = g_smem_set[{func, dev}];
+  if (have >= bytes) return;
   LES_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  g_smem_set.insert({func, dev});
+  have = bytes;
 }
 
 }  // namespace les

@@ -23,8 +23,8 @@
 //   k_x_forward, k_y_forward    compress() fused with -d/dx, -d/dy of the
 //                               fluxes; the e part also inverts re
 //   k_e_update                  e = max(e + dtab1*re, emin)
-//   k_press                     comprhs + press (tridv) per (kx, ky), FP64
-//   k_update                    comp2 in spectral space, FP64
+//   k_press                     comprhs + press (tridv) per (kx, ky) and
+//                               comp2 in spectral space, FP64
 #pragma once
 #include <cooperative_groups.h>
 
@@ -883,13 +883,204 @@ k_e_update(const cx<T>* __restrict__ rem, T* __restrict__ re, T* __restrict__ e,
   });
 }
 
-// comprhs + press + tridv for every (kx, ky) column in z, in FP64
-// (comprhs.f90:17-35, press.F90:37-101, tridv.f90:29-53).
+// comprhs + press + tridv for every (kx, ky) column in z, in FP64, and (with
+// UPDATE) comp2's update of u, v, w and their tendencies from the new p
+// (comprhs.f90:17-35, press.F90:37-101, tridv.f90:29-53, comp2.f90:15-43).
 //   rhs = ikx (Ru + u*/dtab1) + iky (Rv + v*/dtab1) + (Q(z) - Q(z-1))/dz,
-//   Q = w*/dtab1 + Rw, u* = u - dtab2*Ru_old (comp1.f90:127).
-// Thomas sweeps use scratch d[z][mode], r[z][mode].
+//   Q = w*/dtab1 + Rw, u* = u - dtab2*Ru_old (comp1.f90:127);
+//   Ru' = Ru - ikx p, Rv' = Rv - iky p, Rw' = Rw - (p(z+1)-p(z))/dz (mean 0),
+//   u = u* + dtab1 Ru', ..., w plane mean removed.  The kx=ky=0 modes of u, v
+//   and their tendencies live in the FP64 shadows mu, mv, mru, mrv.
+// A block owns MODES modes; MODES consecutive threads take one chunk of L
+// levels each, so a column is solved by blockDim/MODES threads: every thread
+// sweeps its chunk with a zero inflow, the chunks' inflows come from a scan
+// of (product of -d, last value) over the chunks, and r, d, p stay in shared
+// memory.  The pivots d = 1/(b - d_prev) depend on the grid alone; a chunk
+// starts from their closed form, d_n = -cosh((n-1/2)t)/cosh((n+1/2)t) with
+// 2 cosh t - 2 = dz^2 (kx^2 + ky^2) (the determinants of the constant band
+// with the wall's first row).  Bound by HBM on large grids (r and d never go
+// there, and the update's second read of the inputs mostly hits L2), by the
+// chain of levels on small ones, which the chunks cut to L + chunks / warp
+// steps: 64x64x64 FP64 130 -> 14 us, 128x128x96 FP64 235 -> 51 us, 512x512x256
+// mixed 1413 -> 1264 us against one thread per column and a separate update.
+template <class T, int MODES, bool RHS_IN_PH, bool UPDATE>
+__global__ void __launch_bounds__(512)
+k_press(cx<T>* __restrict__ uh, cx<T>* __restrict__ vh, cx<T>* __restrict__ wh, cx<T>* __restrict__ ruo,
+        cx<T>* __restrict__ rvo, cx<T>* __restrict__ rwo, const cx<T>* __restrict__ run, const cx<T>* __restrict__ rvn,
+        const cx<T>* __restrict__ rwn, cx<double>* __restrict__ ph, double* mu, double* mv, double* mru, double* mrv,
+        StageArgs a, int L, int* err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double tot[2][16][3][MODES];  // forward, backward; warp; (product, re, im)
+  const int KX = a.KX, NY = a.NY, NZ = a.NZ;
+  const int nm = KX * NY, nt = blockDim.x, tid = threadIdx.x;
+  cx<double>* const R = reinterpret_cast<cx<double>*>(smraw) + tid;                        // R[l nt]: r, then p
+  double* const D = reinterpret_cast<double*>(smraw + (size_t)L * nt * sizeof(cx<double>)) + tid;  // D[l nt]
+  const int md = tid % MODES, c = tid / MODES;
+  const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
+  const int m = blockIdx.x * MODES + md;
+  const int ky = m / KX, kx = m - ky * KX;
+  const bool live = ky != NY / 2 && m != 0;
+  const double xk = a.kx0 * kx, yk = a.ky0 * signed_k(ky, NY);
+  const double dzdz = a.dz * a.dz, kap = dzdz * (xk * xk + yk * yk);
+  const double dtabm = a.dtabm, dtab1 = a.dtab1, dtab2 = a.zeta ? a.dtab2 : 0.0;
+  const int zs = c * L + 1, n = min(L, NZ - zs + 1);  // levels zs .. zs + n - 1 (n <= 0: none)
+  auto at = [&](int z) { return (size_t)(z - 1) * nm + m; };
+  auto ld = [](cx<T> v) { return mk((double)v.x, (double)v.y); };
+  // LB levels' loads in flight at a time
+  constexpr int LB = sizeof(T) == 4 ? 4 : 2;
+  cx<T> u[LB], v[LB], w[LB], uo[LB], vo[LB], wo[LB], un[LB], vn[LB], wn[LB];
+  auto fetch = [&](int l0) {
+#pragma unroll
+    for (int i = 0; i < LB; i++) {
+      const int z = zs + l0 + i;
+      if (l0 + i >= n) break;
+      const size_t o = at(z);
+      u[i] = uh[o]; v[i] = vh[o]; uo[i] = ruo[o]; vo[i] = rvo[o]; un[i] = run[o]; vn[i] = rvn[o];
+      const bool inw = z < NZ;
+      w[i] = inw ? wh[o] : zero_cx<T>(); wo[i] = inw ? rwo[o] : zero_cx<T>(); wn[i] = inw ? rwn[o] : zero_cx<T>();
+    }
+  };
+  // forward sweep of the chunk with zero inflow; pr: product of -d of the
+  // levels zs - 1 .. zs + n - 2
+  double din = -1.0, pr = 1.0;
+  cx<double> rl = mk(0.0, 0.0);
+  if (live && n > 0) {
+    cx<double> qprev = mk(0.0, 0.0);
+    if (!RHS_IN_PH && c > 0) {
+      const size_t o = at(zs - 1);
+      qprev = (ld(wh[o]) - ld(rwo[o]) * dtab2) * dtabm + ld(rwn[o]);
+    }
+    if (c > 0) {
+      const double t = 2.0 * asinh(0.5 * sqrt(kap)), e = exp(-t), n2 = 2.0 * (zs - 1);
+      din = -e * (1.0 + exp(-(n2 - 1.0) * t)) / (1.0 + exp(-(n2 + 1.0) * t));
+    }
+    double dprev = din;
+    for (int l0 = 0; l0 < n; l0 += LB) {
+      if (!RHS_IN_PH) fetch(l0);
+#pragma unroll
+      for (int i = 0; i < LB; i++) {
+        const int l = l0 + i, z = zs + l;
+        if (l >= n) break;
+        cx<double> rhs;
+        if constexpr (RHS_IN_PH) rhs = ph[at(z)];
+        else {
+          const cx<double> gu = ld(un[i]) + (ld(u[i]) - ld(uo[i]) * dtab2) * dtabm;
+          const cx<double> gv = ld(vn[i]) + (ld(v[i]) - ld(vo[i]) * dtab2) * dtabm;
+          const cx<double> q = (ld(w[i]) - ld(wo[i]) * dtab2) * dtabm + ld(wn[i]);
+          rhs = mul_i(gu) * xk + mul_i(gv) * yk + (q - qprev) * a.dzm;
+          qprev = q;
+        }
+        pr *= -dprev;
+        const double d = 1.0 / (-kap - (z == NZ ? 1.0 : 2.0) - dprev);
+        rl = rhs * dzdz - rl * dprev;
+        D[l * nt] = d;
+        R[l * nt] = rl;
+        dprev = d;
+      }
+    }
+  }
+  // inflow of each chunk: exclusive scan of y -> val + pr y over the chunks
+  // below (forward) or above (backward)
+  auto inflow = [&](int dir, double ip, cx<double> iv) -> cx<double> {
+#pragma unroll
+    for (int o = MODES; o < 32; o *= 2) {
+      const int src = dir ? lane + o : lane - o;
+      const double p2 = __shfl_sync(0xffffffffu, ip, src & 31);
+      const cx<double> v2 = mk(__shfl_sync(0xffffffffu, iv.x, src & 31), __shfl_sync(0xffffffffu, iv.y, src & 31));
+      if (src >= 0 && src < 32) {
+        iv = iv + v2 * ip;
+        ip *= p2;
+      }
+    }
+    if (dir ? lane < MODES : lane >= 32 - MODES) {
+      tot[dir][warp][0][md] = ip;
+      tot[dir][warp][1][md] = iv.x;
+      tot[dir][warp][2][md] = iv.y;
+    }
+    __syncthreads();
+    cx<double> y = mk(0.0, 0.0);
+    for (int k = 0; k < (dir ? nwarp - 1 - warp : warp); k++) {
+      const int w = dir ? nwarp - 1 - k : k;
+      y = mk(tot[dir][w][1][md], tot[dir][w][2][md]) + y * tot[dir][w][0][md];
+    }
+    if (MODES == 32) return y;
+    // this chunk's inflow: the neighbour chunk's inclusive value applied to y
+    const int src = dir ? lane + MODES : lane - MODES;
+    const double p2 = __shfl_sync(0xffffffffu, ip, src & 31);
+    const cx<double> v2 = mk(__shfl_sync(0xffffffffu, iv.x, src & 31), __shfl_sync(0xffffffffu, iv.y, src & 31));
+    return (src >= 0 && src < 32) ? v2 + y * p2 : y;
+  };
+  const cx<double> rin = inflow(0, pr, rl);
+  // backward sweep: the forward inflow added on the way (r = r_local + P rin,
+  // P the product of -d down to the chunk's first level), zero p above
+  cx<double> p = mk(0.0, 0.0);
+  double pb = 1.0;
+  if (live && n > 0) {
+    double P = -din;
+    for (int l = 0; l < n; l++) {  // forward products
+      R[l * nt] = R[l * nt] + rin * P;
+      P *= -D[l * nt];
+    }
+    for (int l = n - 1; l >= 0; l--) {
+      const double d = D[l * nt];
+      p = (R[l * nt] - p) * d;
+      R[l * nt] = p;
+      pb *= -d;
+    }
+  }
+  const cx<double> pin = inflow(1, pb, p);  // p of level zs + n
+  if (live && n > 0) {
+    double P = 1.0;
+    for (int l = n - 1; l >= 0; l--) {
+      P *= -D[l * nt];
+      R[l * nt] = R[l * nt] + pin * P;
+    }
+  }
+  bool bad = false;
+  auto t2 = [](cx<double> v) { return mk((T)v.x, (T)v.y); };
+  for (int l0 = 0; l0 < n; l0 += LB) {
+    if (UPDATE && live) fetch(l0);
+#pragma unroll
+    for (int i = 0; i < LB; i++) {
+      const int l = l0 + i, z = zs + l;
+      if (l >= n) break;
+      const size_t o = at(z);
+      const cx<double> p0 = live ? R[l * nt] : mk(0.0, 0.0);
+      ph[o] = p0;
+      if constexpr (UPDATE) {
+        if (live) {
+          const cx<double> rpu = ld(un[i]) - mul_i(p0) * xk, rpv = ld(vn[i]) - mul_i(p0) * yk;
+          const cx<double> nu = ld(u[i]) - ld(uo[i]) * dtab2 + rpu * dtab1;
+          const cx<double> nv = ld(v[i]) - ld(vo[i]) * dtab2 + rpv * dtab1;
+          uh[o] = t2(nu); vh[o] = t2(nv); ruo[o] = t2(rpu); rvo[o] = t2(rpv);
+          bad = bad || !isfinite(nu.x + nu.y + nv.x + nv.y);
+          if (z < NZ) {
+            const cx<double> p1 = l + 1 < n ? R[(l + 1) * nt] : pin;
+            const cx<double> rpw = ld(wn[i]) - (p1 - p0) * a.dzm;
+            const cx<double> nw = ld(w[i]) - ld(wo[i]) * dtab2 + rpw * dtab1;
+            wh[o] = t2(nw); rwo[o] = t2(rpw);
+            bad = bad || !isfinite(nw.x + nw.y);
+          }
+        } else if (m == 0) {
+          const double rpu = (double)run[o].x, rpv = (double)rvn[o].x;
+          const double nu = mu[z - 1] - dtab2 * mru[z - 1] + dtab1 * rpu, nv = mv[z - 1] - dtab2 * mrv[z - 1] + dtab1 * rpv;
+          mu[z - 1] = nu; mv[z - 1] = nv; mru[z - 1] = rpu; mrv[z - 1] = rpv;
+          uh[o] = t2(mk(nu, 0.0)); vh[o] = t2(mk(nv, 0.0));
+          ruo[o] = t2(mk(rpu, 0.0)); rvo[o] = t2(mk(rpv, 0.0));
+          if (z < NZ) { wh[o] = t2(mk(0.0, 0.0)); rwo[o] = t2(mk(0.0, 0.0)); }
+          bad = bad || !isfinite(nu) || !isfinite(nv);
+        }
+      }
+    }
+  }
+  if (UPDATE && bad) atomicOr(err, ERR_NAN);
+}
+
+// The pressure solve of k_press with one thread per column, for more levels
+// than k_press's chunks hold: Thomas sweeps through scratch d[z][mode],
+// r[z][mode].
 template <class T, bool RHS_IN_PH>
-__global__ void k_press(const cx<T>* __restrict__ uh, const cx<T>* __restrict__ vh, const cx<T>* __restrict__ wh,
+__global__ void k_press_long(const cx<T>* __restrict__ uh, const cx<T>* __restrict__ vh, const cx<T>* __restrict__ wh,
                         const cx<T>* __restrict__ ruo, const cx<T>* __restrict__ rvo, const cx<T>* __restrict__ rwo,
                         const cx<T>* __restrict__ run, const cx<T>* __restrict__ rvn, const cx<T>* __restrict__ rwn,
                         cx<double>* __restrict__ ph, double* __restrict__ dscr, cx<double>* __restrict__ rscr,

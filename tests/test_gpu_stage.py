@@ -276,3 +276,25 @@ def test_out_of_order_split_calls_are_rejected(gpu_lib, product):
     with pytest.raises(product.LesError) as ei:
         g.press()
     assert ei.value.code == product.LES_ESTATE
+
+
+@pytest.mark.parametrize("nz", [4, 5, 9, 63, 64, 65, 127, 128, 129, 255, 256, 257, 512, 513])
+def test_pressure_columns_of_every_chunk_length(gpu_lib, product, nz):
+    """The chunked pressure solve and update at the edges of its chunk lengths
+    (2, 4, 8 levels), of its last chunk, and of the one-thread sweep beyond
+    512 levels; fields, tendencies and p against the oracle, and divergence at
+    round-off (the tolerances of the stage tests)."""
+    o, g, _ = make_pair(product, 16, 16, nz, dt=2e-4)
+    for s in (1, 2):
+        o.stage(0, 1, s)
+        g.stage(0, True, s)
+    compare(o, g, 1e-11, 1e-9, "nz %d" % nz)
+    g2 = product.LesGpu(g.cfg)
+    f = g.download()
+    g2.upload(f["u"], f["v"], f["w"], f["e"], f["p"])
+    g.upload(f["u"], f["v"], f["w"], f["e"], f["p"])
+    g.stage(0, True, 1)
+    g2.stage_split(0, True, 1)
+    a, b = g.download(), g2.download()
+    for k in "uvwep":
+        assert relerr(b[k], a[k]) < 1e-12, k
