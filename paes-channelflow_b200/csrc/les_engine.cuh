@@ -55,7 +55,8 @@ extern thread_local KernelTrace* g_trace;
 template <class... KArgs, class... Args>
 inline void launch(void (*k)(KArgs...), dim3 g, dim3 b, size_t smem, cudaStream_t s, Args... args) {
   if (g.x == 0 || g.y == 0 || g.z == 0) return;
-  if (smem > 48 * 1024) set_smem_limit((const void*)k, smem);
+  // 48 KB without the attribute, static shared memory (at most 12 KB) included
+  if (smem > 36 * 1024) set_smem_limit((const void*)k, smem);
   k<<<g, b, smem, s>>>(args...);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw CudaError(std::string("kernel launch: ") + cudaGetErrorString(e), LES_ECUDA);
@@ -200,7 +201,8 @@ struct Engine : EngineBase {
   // fused path (k_row_fused): clip corrections and wall-model planes
   bool fused = false;
   DevBuf<int> clipflag;
-  DevBuf<T> ephys, dEX, dEY, wallpl;
+  DevBuf<unsigned char> rowclip;  // per (level, row block): clipped (k_clip_x_flag)
+  DevBuf<T> ephys, dEX, dEY;
   DevBuf<cx<T>> xout[8];  // Xu1..Xe2 written by k_row_fused (its inputs stay readable)
   DevBuf<double> divacc, sgsacc, wacc, acc;
   // per-(level, block) partial sums of divz and the SGS means, reduced into
@@ -268,13 +270,13 @@ struct Engine : EngineBase {
     if (fused) {
       clipflag.alloc(NZ);
       ephys.alloc(pb * NZ); dEX.alloc(pb * NZ); dEY.alloc(pb * NZ);
-      wallpl.alloc(pb * 4);
+      rowclip.alloc((size_t)MY * NZ);
       for (auto& b : xout) b.alloc(nmix * NZ);
     } else {
       for (auto& b : pad) b.alloc(pb * NZ);
       for (auto& b : flux) b.alloc(pb * NZ);
     }
-    divacc.alloc(NZ); sgsacc.alloc((size_t)NZ * 8); wacc.alloc((size_t)2 * kWallBlocks * 8); acc.alloc((size_t)NZ * 16);
+    divacc.alloc(NZ); sgsacc.alloc((size_t)NZ * 8); wacc.alloc((size_t)2 * std::max<size_t>(kWallBlocks, MY) * 8); acc.alloc((size_t)NZ * 16);
     // one partial per warp of k_row_fused or per 256-point block of k_flux
     nstat_parts = (int)cdiv(pb, 256);
     if (fused)
@@ -323,7 +325,7 @@ struct Engine : EngineBase {
     for (auto& b : mixed) b.release();
     for (auto& b : pad) b.release();
     for (auto& b : flux) b.release();
-    clipflag.release(); ephys.release(); dEX.release(); dEY.release(); wallpl.release();
+    clipflag.release(); ephys.release(); dEX.release(); dEY.release(); rowclip.release();
     for (auto& b : xout) b.release();
     for (auto& b : phys) b.release();
     lgy.release(); ltau.release(); lfeat.release(); fraw.release(); lpart.release(); lnut.release(); lstat.release(); lflag.release(); lcount.release();
@@ -505,7 +507,9 @@ struct Engine : EngineBase {
   }
 
   // ---- the stage ----
-  void comp1_kernels(const StageArgs& a) {
+  // ezeta: apply the zeta part to e here (split entry points); the whole
+  // stage leaves it to e_update
+  void comp1_kernels(const StageArgs& a, bool ezeta) {
     const T dtab2 = (T)a.dtab2;
     // the learned closure reads the stage's start state (u, v, w and, for
     // its fallback test, e before k_e_prep's zeta update)
@@ -514,7 +518,7 @@ struct Engine : EngineBase {
       constexpr int N = decltype(cn)::value;
       using C = RowCfg<N>;
       launch(k_e_prep<T, N>, dim3(cdiv(NY / 2, C::NT), NZ - 1), dim3(C::THREADS), C::template smem<T>(), st, e.p,
-             (const T*)re.p, Xe.p, NY, NZ, dtab2, a.zeta, tw);
+             (const T*)re.p, Xe.p, NY, NZ, dtab2, (int)(ezeta && a.zeta), fused ? clipflag.p : (int*)nullptr, tw);
     });
     with_small(NY, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
@@ -776,49 +780,36 @@ struct Engine : EngineBase {
     launch(k_ldiv<T>, dim3(cdiv(nm, 128), NZ), dim3(128), 0, st, (const cx<T>*)lgy.p, run.p, rvn.p, rwn.p,
            (const cx<T>*)uh.p, (const cx<T>*)vh.p, (const double*)nuf, (const int*)lflag.p, a);
   }
-  // Wall-model plane sums from the physical U, V rows of levels 1 and nnz.
-  void wall_params_from(const T* U, const T* V, size_t upper_off, const StageArgs& a) {
-    (void)upper_off;
-    launch(k_wall_sums<T>, dim3(kWallBlocks, 2), dim3(256), 0, st, U, V, 2, pb, wacc.p);
-    launch(k_wall_final, dim3(1), dim3(32), 0, st, (const double*)wacc.p, (int)kWallBlocks, (const double*)mru.p,
+  void wall_final(int nblk, const StageArgs& a) {
+    launch(k_wall_final, dim3(1), dim3(kWallFinalThreads), 0, st, (const double*)wacc.p, nblk, (const double*)mru.p,
            (const double*)mrv.p, a, (double)pb, 0.4, zody, cfg.ufree, wp.p, err.p);
   }
   void fused_middle(const StageArgs& a) {
-    // clip flags and corrections of max(expand(e), emin)
-    LES_CUDA(cudaMemsetAsync(clipflag.p, 0, NZ * sizeof(int), st));
+    int brows = 1;  // rows of a block of k_clip_x_flag
     with_small(NX, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
       using C = RowCfg<3 * N / 2>;
-      launch(k_clip_flag<T, N>, dim3(cdiv(MY / 2, C::NT), NZ - 1), dim3(C::THREADS), C::template smem<T>(), st,
-             (const cx<T>*)mixed[6].p, clipflag.p, MY, (T)cfg.emin, tw);
-      launch(k_clip_phys<T, N>, dim3(cdiv(MY / 2, C::NT), NZ - 1), dim3(C::THREADS), C::template smem<T>(), st,
-             (const cx<T>*)mixed[6].p, ephys.p, (const int*)clipflag.p, MY, tw);
+      brows = 2 * C::NT;
+      // clip flags and corrections of max(expand(e), emin)
+      launch(k_clip_x_flag<T, N>, dim3(cdiv(MY / 2, C::NT), NZ - 1), dim3(C::THREADS), C::template smem<T>(), st,
+             (const cx<T>*)mixed[6].p, ephys.p, dEX.p, clipflag.p, rowclip.p, MY, (T)cfg.emin, (T)kx0, tw);
+      // wall-model sums of U, V at levels 1 and nnz
+      const unsigned nblk = cdiv(MY, C::NT);
+      launch(k_wall_rows<T, N>, dim3(nblk, 2), dim3(C::THREADS), C::template smem<T>(), st, (const cx<T>*)mixed[0].p,
+             (const cx<T>*)mixed[2].p, MY, NZ, wacc.p, tw);
+      wall_final((int)nblk, a);
     });
     with_small(NY, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
       using C = ColCfg<3 * N / 2, T>;
       launch(k_clipd_y<T, N>, dim3(cdiv(MX / 2, C::TC), NZ - 1), dim3(C::THREADS), C::buf(), st,
-             (const T*)ephys.p, dEY.p, (const int*)clipflag.p, MX, (T)cfg.emin, (T)ky0, tw);
+             (const T*)ephys.p, dEY.p, (const int*)clipflag.p, (const unsigned char*)rowclip.p, brows, MX, (T)cfg.emin,
+             (T)ky0, tw);
     });
-    with_small(NX, [&](auto cn) {
-      constexpr int N = decltype(cn)::value;
-      using C = RowCfg<3 * N / 2>;
-      launch(k_clipd_x<T, N>, dim3(cdiv(MY / 2, C::NT), NZ - 1), dim3(C::THREADS), C::template smem<T>(), st,
-             (const T*)ephys.p, dEX.p, (const int*)clipflag.p, MY, (T)cfg.emin, (T)kx0, tw);
-      // physical U, V at levels 1 and nnz for the wall model: wallpl = [U1, Unz, V1, Vnz]
-      using CR = RowCfg<3 * N / 2>;
-      const int lv[2] = {1, NZ};
-      for (int side = 0; side < 2; side++)
-        for (int fld = 0; fld < 2; fld++)
-          launch(k_row_c2r<T, 3 * N / 2>, dim3(cdiv(MY / 2 + 1, CR::NT)), dim3(CR::THREADS), CR::template smem<T>(),
-                 st, (const cx<T>*)(mixed[fld == 0 ? 0 : 2].p + (size_t)(lv[side] - 1) * nmix),
-                 wallpl.p + (size_t)(2 * fld + side) * pb, MY, KX, tw);
-    });
-    wall_params_from(wallpl.p, wallpl.p + 2 * pb, pb, a);
     // the fused row kernel
     FusedArgs fa{};
     for (int i = 0; i < 8; i++) { fa.in.p[i] = mixed[i].p; fa.out.p[i] = xout[i].p; }
-    fa.dEX = dEX.p; fa.dEY = dEY.p; fa.clipflag = clipflag.p; fa.wp = wp.p;
+    fa.dEX = dEX.p; fa.dEY = dEY.p; fa.clipflag = clipflag.p; fa.rowclip = rowclip.p; fa.wp = wp.p;
     fa.divpart = divpart.p; fa.sgspart = sgspart.p;
     fa.lflag = learned_on() ? lflag.p : nullptr;
     with_small(NX, [&](auto cn) {
@@ -881,8 +872,7 @@ struct Engine : EngineBase {
     {
       launch(k_wall_sums<T>, dim3(kWallBlocks, 2), dim3(256), 0, st, (const T*)pad[0].p, (const T*)pad[3].p, NZ, pb,
              wacc.p);
-      launch(k_wall_final, dim3(1), dim3(32), 0, st, (const double*)wacc.p, (int)kWallBlocks, (const double*)mru.p,
-             (const double*)mrv.p, a, (double)pb, 0.4, zody, cfg.ufree, wp.p, err.p);
+      wall_final((int)kWallBlocks, a);
     }
     Ptr11 fl{};
     for (int i = 0; i < 11; i++) fl.p[i] = flux[i].p;
@@ -897,18 +887,14 @@ struct Engine : EngineBase {
              NZ, (T)kx0, tw);
     });
   }
-  // comp2's e update: re = c2r(rem) with plain stores, then the clipped
-  // elementwise update (a read-modify-write inside the transform's store
-  // phase would serialise on the load latency)
-  void e_update(double dtab1) {
+  // re = c2r(rem), e = max(e - dtab2 re_old + dtab1 re, emin) of a whole stage
+  void e_update(const StageArgs& a) {
     with_small(NX, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
       using C = RowCfg<N>;
-      launch(k_row_c2r<T, N>, dim3(cdiv((size_t)(NZ - 1) * NY / 2 + 1, C::NT)), dim3(C::THREADS),
-             C::template smem<T>(), st, (const cx<T>*)rem.p, re.p, (NZ - 1) * NY, KX, tw);
+      launch(k_e_update<T, N>, dim3(cdiv((size_t)(NZ - 1) * NY / 2, C::NT)), dim3(C::THREADS), C::template smem<T>(), st,
+             (const cx<T>*)rem.p, re.p, e.p + ps, (NZ - 1) * NY, (T)a.dtab1, a.zeta ? (T)a.dtab2 : (T)0, (T)cfg.emin, tw);
     });
-    launch(k_e_update_phys<T>, dim3(cdiv(ps * (NZ - 1), 256)), dim3(256), 0, st, e.p + ps, (const T*)re.p,
-           ps * (NZ - 1), (T)dtab1, (T)cfg.emin);
   }
   // Pressure solve, with the update of u, v, w and their tendencies when
   // `update` (the split entry points solve with the right-hand side in ph and
@@ -927,7 +913,6 @@ struct Engine : EngineBase {
     const int L = (int)cdiv(NZ, 512 / MODES);  // levels of a chunk
     const int threads = (int)cdiv((size_t)MODES * cdiv(NZ, L), 32) * 32;
     const size_t smem = (size_t)L * threads * (sizeof(cx<double>) + sizeof(double));
-    set_smem_limit((const void*)k_press<T, MODES, RHS, UPD>, smem);  // the kernel has static shared memory too
     launch(k_press<T, MODES, RHS, UPD>, dim3((unsigned)(nm / MODES)), dim3((unsigned)threads), smem, st, uh.p, vh.p, wh.p,
            ruo.p, rvo.p, rwo.p, (const cx<T>*)run.p, (const cx<T>*)rvn.p, (const cx<T>*)rwn.p, ph.p, mu.p, mv.p, mru.p,
            mrv.p, a, L, err.p);
@@ -961,7 +946,7 @@ struct Engine : EngineBase {
   double last_dtab1 = 0, last_xkmax = 0;
   void comp1(bool mnout, int istage, double dtab1, double dtab2, double xkmax) override {
     StageArgs a = args(dtab1, dtab2, xkmax, istage != 1, mnout && istage == 1);
-    comp1_kernels(a);
+    comp1_kernels(a, true);
     if (istage != 1)
       launch(k_zeta<T>, dim3(cdiv(nm, 128), NZ), dim3(128), 0, st, uh.p, vh.p, wh.p, (const cx<T>*)ruo.p,
              (const cx<T>*)rvo.p, (const cx<T>*)rwo.p, mu.p, mv.p, (const double*)mru.p, (const double*)mrv.p, a);
@@ -1002,8 +987,8 @@ struct Engine : EngineBase {
   }
   void stage_kernels(bool mnout, int istage, double dtab1, double dtab2, double xkmax) {
     StageArgs a = args(dtab1, dtab2, xkmax, istage != 1, mnout && istage == 1);
-    comp1_kernels(a);
-    e_update(dtab1);
+    comp1_kernels(a, false);
+    e_update(a);
     press_kernel(a, false, true);
   }
   void stage(bool mnout, int istage, double dtab1, double dtab2, double xkmax) override {

@@ -284,6 +284,7 @@ struct FusedArgs {
   const void* dEX;       // clip corrections (padded physical, levels 1..nnz-1)
   const void* dEY;
   const int* clipflag;   // per level 1..nnz-1 (index z-1)
+  const unsigned char* rowclip;  // per level and block of k_clip_x_flag: its rows of dEX are set
   const WallParams* wp;
   double* divpart;  // [level][CTA][warp] partial sums of divz, one writer each
   double* sgspart;  // [level][CTA][warp][6] partial SGS means (stage 1 with mnout)
@@ -509,7 +510,11 @@ k_row_fused(FusedArgs f, StageArgs a, const cx<T>* __restrict__ tw) {
     // ---- phase II: fluxes (k_flux) ----
     double divz_part = 0.0;
     double sgs_part[6] = {0, 0, 0, 0, 0, 0};
+    // the clip corrections: dEY on a flagged level, dEX where the row's block
+    // of k_clip_x_flag clipped (2 NT rows each)
+    constexpr int BR = 2 * RowCfg<MX>::NT;
     const bool clip = (!top) && f.clipflag[le - 1];
+    const bool clipx = clip && f.rowclip[(size_t)(le - 1) * ((MY + BR - 1) / BR) + y / BR];
 #pragma unroll
     for (int q = 0; q < PPT; q++) {
       const int n = tr + TR * q;
@@ -535,7 +540,7 @@ k_row_fused(FusedArgs f, StageArgs a, const cx<T>* __restrict__ tw) {
         cx<T> exy = p[5 * BUF];
         if (clip) {
           const size_t o = ((size_t)(le - 1) * MY + y) * MX + C::x_of(n);
-          exy.x += reinterpret_cast<const T*>(f.dEX)[o];
+          if (clipx) exy.x += reinterpret_cast<const T*>(f.dEX)[o];
           exy.y += reinterpret_cast<const T*>(f.dEY)[o];
         }
         U1 = uv1.x; V1 = uv1.y;
@@ -651,89 +656,81 @@ k_row_fused(FusedArgs f, StageArgs a, const cx<T>* __restrict__ tw) {
   }
 }
 
-// Per-level flag: does max(expand(e), emin) clip anywhere on the padded
-// plane?  Rows of Em (pairs) are inverted and compared with emin.
+// Does max(expand(e), emin) clip, and if so dEX = xderiv(delta), delta =
+// max(emin - E, 0).  A block inverts C::NT row pairs of Em.  rowclip[z-1][block]
+// says whether one of its points lies below emin; only then does it store its
+// rows of E (for k_clipd_y) and dEX and set the level's flag: elsewhere delta
+// and its x derivative are zero.  One kernel instead of a flag pass, a pass
+// for E and one for dEX; a clipping block transforms its rows again, so that
+// the common case keeps nothing (with the first transform's rows kept in
+// shared memory an unclipped 512x512x256 stage took 418 us instead of 134).
 template <class T, int NSX>
-__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS)
-k_clip_flag(const cx<T>* __restrict__ Em, int* __restrict__ flags, int MY, T emin, const cx<T>* __restrict__ tw) {
+__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS, sizeof(T) == 8 ? 3 : 1)
+k_clip_x_flag(const cx<T>* __restrict__ Em, T* __restrict__ E, T* __restrict__ dEX, int* __restrict__ flags,
+              unsigned char* __restrict__ rowclip, int MY, T emin, T kx0, const cx<T>* __restrict__ tw) {
   constexpr int MX = 3 * NSX / 2;
   constexpr int KX = NSX / 2;
   using C = RowCfg<MX>;
   extern __shared__ __align__(16) unsigned char smraw[];
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
   const int z = blockIdx.y + 1;
   const int p0 = blockIdx.x * C::NT, np = MY / 2;
   const cx<T>* in = Em + (size_t)(z - 1) * MY * KX;
-  fft_core<MX, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
-    int p = p0 + t;
-    cx<T> v = zero_cx<T>();
-    if (p < np) {
-      int k = -1;
-      bool mir = false;
-      if (n < KX) k = n;
-      else if (n > MX - KX) { k = MX - n; mir = true; }
-      if (k >= 0) {
-        cx<T> av = in[(size_t)(2 * p) * KX + k], bv = in[(size_t)(2 * p + 1) * KX + k];
-        if (k == 0) { av.y = 0; bv.y = 0; }
-        if (mir) { av = conj(av); bv = conj(bv); }
-        v = mk(av.x - bv.y, av.y + bv.x);
-      }
-    }
-    return v;
-  }, [&](int t, int n, cx<T> v) {
-    int p = p0 + t;
-    if (p < np && (v.x < emin || v.y < emin)) any = 1;
+  auto load = [&](int t, int n) {
+    const int p = p0 + t;
+    int k = -1;
+    bool mir = false;
+    if (n < KX) k = n;
+    else if (n > MX - KX) { k = MX - n; mir = true; }
+    if (p >= np || k < 0) return zero_cx<T>();
+    cx<T> av = in[(size_t)(2 * p) * KX + k], bv = in[(size_t)(2 * p + 1) * KX + k];
+    if (k == 0) { av.y = 0; bv.y = 0; }
+    if (mir) { av = conj(av); bv = conj(bv); }
+    return mk(av.x - bv.y, av.y + bv.x);
+  };
+  bool below = false;
+  fft_core<MX, +1, false, false, false>(C::NT, sm, tw, load, [&](int t, int, cx<T> v) {
+    below = below || (p0 + t < np && (v.x < emin || v.y < emin));
   });
+  const bool any = __syncthreads_or(below);
+  if (threadIdx.x == 0) {
+    rowclip[(size_t)(z - 1) * gridDim.x + blockIdx.x] = any;
+    if (any) atomicOr(flags + (z - 1), 1);
+  }
+  if (!any) return;
+  fft_core<MX, +1, false, false, true>(C::NT, sm, tw, load, NoStore{});
+  const size_t zoff = (size_t)(z - 1) * MY * MX;
+  for (int i = threadIdx.x; i < C::NT * MX; i += C::THREADS) {
+    const int t = i / MX, n = i - t * MX, p = p0 + t;
+    const cx<T> v = sm[i];
+    if (p < np) {
+      E[zoff + (size_t)(2 * p) * MX + n] = v.x;
+      E[zoff + (size_t)(2 * p + 1) * MX + n] = v.y;
+    }
+    sm[i] = mk(tmax(emin - v.x, (T)0), tmax(emin - v.y, (T)0));
+  }
   __syncthreads();
-  if (threadIdx.x == 0 && any) atomicOr(flags + (z - 1), 1);
-}
-
-// Physical E (unclipped) of flagged levels, for the clip corrections.
-template <class T, int NSX>
-__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS)
-k_clip_phys(const cx<T>* __restrict__ Em, T* __restrict__ E, const int* __restrict__ flags, int MY,
-            const cx<T>* __restrict__ tw) {
-  constexpr int MX = 3 * NSX / 2;
-  constexpr int KX = NSX / 2;
-  using C = RowCfg<MX>;
-  const int z = blockIdx.y + 1;
-  if (!flags[z - 1]) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  const int p0 = blockIdx.x * C::NT, np = MY / 2;
-  const cx<T>* in = Em + (size_t)(z - 1) * MY * KX;
-  T* out = E + (size_t)(z - 1) * MY * MX;
-  fft_core<MX, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
-    int p = p0 + t;
-    cx<T> v = zero_cx<T>();
-    if (p < np) {
-      int k = -1;
-      bool mir = false;
-      if (n < KX) k = n;
-      else if (n > MX - KX) { k = MX - n; mir = true; }
-      if (k >= 0) {
-        cx<T> av = in[(size_t)(2 * p) * KX + k], bv = in[(size_t)(2 * p + 1) * KX + k];
-        if (k == 0) { av.y = 0; bv.y = 0; }
-        if (mir) { av = conj(av); bv = conj(bv); }
-        v = mk(av.x - bv.y, av.y + bv.x);
-      }
-    }
-    return v;
-  }, [&](int t, int n, cx<T> v) {
-    int p = p0 + t;
+  fft_core<MX, -1, false, true, true>(C::NT, sm, tw, NoLoad{}, NoStore{});
+  for (int i = threadIdx.x; i < C::NT * MX; i += C::THREADS) {
+    const int k = i % MX;
+    const T kk = (k == 0 || 2 * k == MX) ? (T)0 : kx0 * (T)signed_k(k, MX) / (T)MX;
+    sm[i] = mul_i(sm[i]) * kk;
+  }
+  __syncthreads();
+  fft_core<MX, +1, false, true, false>(C::NT, sm, tw, NoLoad{}, [&](int t, int n, cx<T> d) {
+    const int p = p0 + t;
     if (p >= np) return;
-    out[(size_t)(2 * p) * MX + n] = v.x;
-    out[(size_t)(2 * p + 1) * MX + n] = v.y;
+    dEX[zoff + (size_t)(2 * p) * MX + n] = d.x;
+    dEX[zoff + (size_t)(2 * p + 1) * MX + n] = d.y;
   });
 }
 
-// dEY = yderiv(delta), delta = max(emin - E, 0), flagged levels only.
+// dEY = yderiv(delta), delta = max(emin - E, 0), flagged levels only; rowclip
+// (one byte per brows rows) says where E was stored, delta is zero elsewhere.
 template <class T, int NSY>
 __global__ void __launch_bounds__(ColCfg<3 * NSY / 2, T>::THREADS)
-k_clipd_y(const T* __restrict__ E, T* __restrict__ dEY, const int* __restrict__ flags, int MX, T emin, T ky0,
-          const cx<T>* __restrict__ tw) {
+k_clipd_y(const T* __restrict__ E, T* __restrict__ dEY, const int* __restrict__ flags,
+          const unsigned char* __restrict__ rowclip, int brows, int MX, T emin, T ky0, const cx<T>* __restrict__ tw) {
   constexpr int M = 3 * NSY / 2;
   using C = ColCfg<M, T>;
   if (!flags[blockIdx.y]) return;
@@ -742,12 +739,17 @@ k_clipd_y(const T* __restrict__ E, T* __restrict__ dEY, const int* __restrict__ 
   const size_t zoff = (size_t)blockIdx.y * M * MX;
   const int c0 = blockIdx.x * C::TC, ncp = MX / 2;
   const cx<T>* Ez = reinterpret_cast<const cx<T>*>(E + zoff);
+  __shared__ unsigned char clipped[M];
+  for (int n = threadIdx.x; n < M; n += blockDim.x)
+    clipped[n] = rowclip[(size_t)blockIdx.y * ((M + brows - 1) / brows) + n / brows];
+  __syncthreads();
   fft_core<M, -1, true, false, true>(C::TC, sm, tw, [&](int t, int n) {
     int c = c0 + t;
     cx<T> v = zero_cx<T>();
-    if (c < ncp) {
-      cx<T> ev = Ez[(size_t)n * ncp + c];
-      v = mk(tmax(emin - ev.x, (T)0), tmax(emin - ev.y, (T)0));
+    if (c < ncp) {  // load first, select after: the loads stay independent
+      const cx<T> ev = Ez[(size_t)n * ncp + c];
+      const bool on = clipped[n];
+      v = mk(on ? tmax(emin - ev.x, (T)0) : (T)0, on ? tmax(emin - ev.y, (T)0) : (T)0);
     }
     return v;
   }, NoStore{});
@@ -761,43 +763,6 @@ k_clipd_y(const T* __restrict__ E, T* __restrict__ dEY, const int* __restrict__ 
   fft_core<M, +1, true, true, false>(C::TC, sm, tw, NoLoad{}, [&](int t, int n, cx<T> d) {
     int c = c0 + t;
     if (c < ncp) out[(size_t)n * ncp + c] = d;
-  });
-}
-
-// dEX = xderiv(delta), flagged levels only.
-template <class T, int NSX>
-__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS)
-k_clipd_x(const T* __restrict__ E, T* __restrict__ dEX, const int* __restrict__ flags, int MY, T emin, T kx0,
-          const cx<T>* __restrict__ tw) {
-  constexpr int MX = 3 * NSX / 2;
-  using C = RowCfg<MX>;
-  if (!flags[blockIdx.y]) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  const size_t zoff = (size_t)blockIdx.y * MY * MX;
-  const int p0 = blockIdx.x * C::NT, np = MY / 2;
-  const T* Ez = E + zoff;
-  T* out = dEX + zoff;
-  fft_core<MX, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
-    int p = p0 + t;
-    cx<T> v = zero_cx<T>();
-    if (p < np) {
-      T av = Ez[(size_t)(2 * p) * MX + n], bv = Ez[(size_t)(2 * p + 1) * MX + n];
-      v = mk(tmax(emin - av, (T)0), tmax(emin - bv, (T)0));
-    }
-    return v;
-  }, NoStore{});
-  for (int i = threadIdx.x; i < C::NT * MX; i += blockDim.x) {
-    int t = i / MX, k = i - t * MX;
-    T kk = (k == 0 || 2 * k == MX) ? (T)0 : kx0 * (T)signed_k(k, MX) / (T)MX;
-    sm[t * MX + k] = mul_i(sm[t * MX + k]) * kk;
-  }
-  __syncthreads();
-  fft_core<MX, +1, false, true, false>(C::NT, sm, tw, NoLoad{}, [&](int t, int n, cx<T> d) {
-    int p = p0 + t;
-    if (p >= np) return;
-    out[(size_t)(2 * p) * MX + n] = d.x;
-    out[(size_t)(2 * p + 1) * MX + n] = d.y;
   });
 }
 

@@ -228,13 +228,15 @@ k_col_trunc(const cx<T>* __restrict__ in, cx<T>* __restrict__ out, int KX, T sca
 // ---------------------------------------------------------------------------
 // Stage kernels
 // ---------------------------------------------------------------------------
-// lower/upper ghosts of e (lowerbc.f90:13-17, upperbc.f90:20-24), the
-// zeta part of the stage for e (comp1.f90:131), and the x-transform of e
-// (first half of expand, filter_fftw.f90:262-263).  e has levels 0..NZ+1.
+// lower/upper ghosts of e (lowerbc.f90:13-17, upperbc.f90:20-24), with `zeta`
+// the zeta part of the stage for e (comp1.f90:131; the fused stage leaves it
+// to k_e_update), and the x-transform of e (first half of expand,
+// filter_fftw.f90:262-263).  e has levels 0..NZ+1.  Also clears the level's
+// clip flag (when given) for k_clip_x_flag.
 template <class T, int NX>
 __global__ void __launch_bounds__(RowCfg<NX>::THREADS)
 k_e_prep(T* __restrict__ e, const T* __restrict__ re, cx<T>* __restrict__ Xe, int NY, int NZ, T dtab2, int zeta,
-         const cx<T>* __restrict__ tw) {
+         int* __restrict__ clipflag, const cx<T>* __restrict__ tw) {
   using C = RowCfg<NX>;
   constexpr int KX = NX / 2;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -243,6 +245,7 @@ k_e_prep(T* __restrict__ e, const T* __restrict__ re, cx<T>* __restrict__ Xe, in
   const int p0 = blockIdx.x * C::NT;
   const size_t plane = (size_t)NY * NX;
   T* ez = e + (size_t)z * plane;
+  if (clipflag && blockIdx.x == 0 && threadIdx.x == 0) clipflag[z - 1] = 0;
   fft_core<NX, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
     int p = p0 + t;
     return (p < NY / 2) ? mk(ez[(size_t)(2 * p) * NX + n], ez[(size_t)(2 * p + 1) * NX + n]) : zero_cx<T>();
@@ -256,6 +259,7 @@ k_e_prep(T* __restrict__ e, const T* __restrict__ re, cx<T>* __restrict__ Xe, in
     out[(size_t)(2 * p) * KX + k] = (zk + zm) * (T)0.5;
     out[(size_t)(2 * p + 1) * KX + k] = mk(d.y * (T)0.5, -d.x * (T)0.5);
   }
+  if (!zeta && z != 1 && z != NZ - 1) return;
   for (int i = threadIdx.x; i < C::NT * NX; i += blockDim.x) {
     int t = i / NX, n = i - t * NX, p = p0 + t;
     if (p >= NY / 2) continue;
@@ -502,23 +506,70 @@ __global__ void k_wall_sums(const T* __restrict__ U, const T* __restrict__ V, in
   block_sum_store<8>(s, part + ((size_t)side * gridDim.x + blockIdx.x) * 8);
 }
 
+// As k_wall_sums, straight from the mixed rows of u and v (x-spectral, y
+// physical): block (x, side) transforms C::NT rows of U + iV of level 1 or nnz
+// (one complex transform for both) and sums its points, without storing them.
+template <class T, int NSX>
+__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS)
+k_wall_rows(const cx<T>* __restrict__ Um, const cx<T>* __restrict__ Vm, int MY, int NZ, double* part,
+            const cx<T>* __restrict__ tw) {
+  constexpr int MX = 3 * NSX / 2, KX = NSX / 2;
+  using C = RowCfg<MX>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
+  const int side = blockIdx.y, y0 = blockIdx.x * C::NT;
+  const size_t off = side == 0 ? 0 : (size_t)(NZ - 1) * MY * KX;
+  double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  fft_core<MX, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
+    const int y = y0 + t;
+    int k = -1;
+    bool mir = false;
+    if (n < KX) k = n;
+    else if (n > MX - KX) { k = MX - n; mir = true; }
+    if (y >= MY || k < 0) return zero_cx<T>();
+    cx<T> av = Um[off + (size_t)y * KX + k], bv = Vm[off + (size_t)y * KX + k];
+    if (k == 0) { av.y = 0; bv.y = 0; }
+    if (mir) { av = conj(av); bv = conj(bv); }
+    return mk(av.x - bv.y, av.y + bv.x);
+  }, [&](int t, int, cx<T> uv) {
+    if (y0 + t >= MY) return;
+    const double u = (double)uv.x, v = (double)uv.y, wd = (double)sqrt((T)(uv.x * uv.x + uv.y * uv.y));
+    s[0] += u; s[1] += v; s[2] += wd; s[3] += u * u; s[4] += v * v; s[5] += wd * wd; s[6] += wd * u; s[7] += wd * v;
+  });
+  block_sum_store<8>(s, part + ((size_t)side * gridDim.x + blockIdx.x) * 8);
+}
+
 // Wall-model scalars for both walls (lowerbc.f90:56-124, upperbc.f90:63-122)
 // and the global dudt, dvdt (lowerbc.f90:70-72) from the FP64 mean shadows.
-static __global__ void k_wall_final(const double* __restrict__ part, int nblk, const double* __restrict__ mru,
-                             const double* __restrict__ mrv, StageArgs a, double P, double vk, double zody,
-                             double ufree, WallParams* wp, int* err) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double acc[16];
-  for (int q = 0; q < 16; q++) acc[q] = 0.0;
-  for (int side = 0; side < 2; side++)
-    for (int b = 0; b < nblk; b++)
-      for (int q = 0; q < 8; q++) acc[side * 8 + q] += part[((size_t)side * nblk + b) * 8 + q];
-  double su = 0, sv = 0;
-  for (int z = 0; z < a.NZ; z++) { su += mru[z]; sv += mrv[z]; }
-  wp->dudt = su / a.NZ;
-  wp->dvdt = sv / a.NZ;
-  wp->utau_s = sqrt(a.zl / 2 * sqrt(wp->dvdt * wp->dvdt + (a.forcing - wp->dudt) * (a.forcing - wp->dudt)));
-  for (int side = 0; side < 2; side++) {
+// One block of 18 warps: a warp per sum (16 plane sums, then mru, mrv), each
+// in a fixed order, then one lane per wall.  (One thread for everything: 55
+// us per stage at any size; this 7 us.)
+constexpr int kWallFinalThreads = 18 * 32;
+static __global__ void __launch_bounds__(kWallFinalThreads)
+k_wall_final(const double* __restrict__ part, int nblk, const double* __restrict__ mru,
+             const double* __restrict__ mrv, StageArgs a, double P, double vk, double zody,
+             double ufree, WallParams* wp, int* err) {
+  __shared__ double acc[18];
+  {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double s = 0.0;
+    if (w < 16)
+      for (int b = lane; b < nblk; b += 32) s += part[((size_t)(w >> 3) * nblk + b) * 8 + (w & 7)];
+    else
+      for (int z = lane; z < a.NZ; z += 32) s += w == 16 ? mru[z] : mrv[z];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) acc[w] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x > 1) return;
+  const double su = acc[16], sv = acc[17];
+  if (threadIdx.x == 0) {
+    wp->dudt = su / a.NZ;
+    wp->dvdt = sv / a.NZ;
+    wp->utau_s = sqrt(a.zl / 2 * sqrt(wp->dvdt * wp->dvdt + (a.forcing - wp->dudt) * (a.forcing - wp->dudt)));
+  }
+  {
+    const int side = threadIdx.x;
     const double* s = acc + side * 8;
     WallSide& w = wp->w[side];
     double mU = s[0] / P, mV = s[1] / P;
@@ -838,49 +889,60 @@ k_y_forward(Ptr8 X, Ptr8 rnew, int KX, int NZ, T ky0, T scale, const cx<T>* __re
   }
 }
 
-// comp2's e update (comp2.f90:38) with re from its x-spectral rows:
-// re = c2r(rem), e = max(e + dtab1*re, emin), levels 1..nnz-1.
+// The stage's e update (comp1.f90:131, comp2.f90:38) with re from its
+// x-spectral rows: e = max(e - dtab2*re_old + dtab1*re, emin), re = c2r(rem),
+// levels 1..nnz-1 (nrows = ny (nnz-1) rows; dtab2 = 0 in the first stage).
+// The transform leaves its rows in shared memory; the elementwise pass then
+// reads and writes whole rows, four values a thread, so the loads of e and
+// re are not chained to the transform's stores.
 template <class T, int NX>
 __global__ void __launch_bounds__(RowCfg<NX>::THREADS)
-k_e_update(const cx<T>* __restrict__ rem, T* __restrict__ re, T* __restrict__ e, int NY, T dtab1, T emin,
+k_e_update(const cx<T>* __restrict__ rem, T* __restrict__ re, T* __restrict__ e, int nrows, T dtab1, T dtab2, T emin,
            const cx<T>* __restrict__ tw) {
   using C = RowCfg<NX>;
   constexpr int KX = NX / 2;
   extern __shared__ __align__(16) unsigned char smraw[];
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  const int z = blockIdx.y + 1;
-  const int p0 = blockIdx.x * C::NT;
-  const size_t plane = (size_t)NY * NX;
-  const cx<T>* in = rem + (size_t)(z - 1) * NY * KX;
-  T* rez = re + (size_t)(z - 1) * plane;
-  T* ez = e + (size_t)z * plane;
-  fft_core<NX, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
-    int p = p0 + t;
-    cx<T> v = zero_cx<T>();
-    if (p < NY / 2) {
-      int k = -1;
-      bool mir = false;
-      if (n < KX) k = n;
-      else if (n > KX) { k = NX - n; mir = true; }
-      if (k >= 0) {
-        cx<T> a = in[(size_t)(2 * p) * KX + k], b = in[(size_t)(2 * p + 1) * KX + k];
-        if (k == 0) { a.y = 0; b.y = 0; }
-        if (mir) { a = conj(a); b = conj(b); }
-        v = mk(a.x - b.y, a.y + b.x);
-      }
-    }
-    return v;
-  }, [&](int t, int n, cx<T> v) {
-    int p = p0 + t;
-    if (p >= NY / 2) return;
+  const int p0 = blockIdx.x * C::NT, np = nrows / 2;
+  fft_core<NX, +1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
+    const int p = p0 + t;
+    int k = -1;
+    bool mir = false;
+    if (n < KX) k = n;
+    else if (n > KX) { k = NX - n; mir = true; }
+    if (p >= np || k < 0) return zero_cx<T>();
+    cx<T> a = rem[(size_t)(2 * p) * KX + k], b = rem[(size_t)(2 * p + 1) * KX + k];
+    if (k == 0) { a.y = 0; b.y = 0; }
+    if (mir) { a = conj(a); b = conj(b); }
+    return mk(a.x - b.y, a.y + b.x);
+  }, NoStore{});
+  struct alignas(4 * sizeof(T)) V4 { T v[4]; };
+  constexpr int ITEMS = C::NT * NX / 4;
+#pragma unroll 2
+  for (int i = threadIdx.x; i < ITEMS; i += C::THREADS) {
+    const int t = i / (NX / 4), n = 4 * (i - t * (NX / 4)), p = p0 + t;
+    if (p >= np) continue;
+    const cx<T>* s = sm + t * NX + n;
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-      size_t off = (size_t)(2 * p + r) * NX + n;
-      T rv = r ? v.y : v.x;
-      rez[off] = rv;
-      ez[off] = tmax(ez[off] + dtab1 * rv, emin);
+      const size_t o = ((size_t)(2 * p + r) * NX + n) / 4;
+      V4* ev = reinterpret_cast<V4*>(e) + o;
+      V4* rv = reinterpret_cast<V4*>(re) + o;
+      V4 x = *ev, nr;
+      if (dtab2 != (T)0) {
+        const V4 old = *rv;
+#pragma unroll
+        for (int q = 0; q < 4; q++) x.v[q] = x.v[q] - dtab2 * old.v[q];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        nr.v[q] = r ? s[q].y : s[q].x;
+        x.v[q] = tmax(x.v[q] + dtab1 * nr.v[q], emin);
+      }
+      *ev = x;
+      *rv = nr;
     }
-  });
+  }
 }
 
 // comprhs + press + tridv for every (kx, ky) column in z, in FP64, and (with
