@@ -291,29 +291,26 @@ struct Engine : EngineBase {
     with_small(NY, [&](auto cn) { y_prefetch_setup<decltype(cn)::value>(); });
   }
   // Tensor maps and distances of the y-column prefetches.  The distance is
-  // one resident wave of the kernel (resident blocks per SM x SMs, even so
-  // that a k_y_forward block prefetches for a block of its own cluster rank
-  // and a k_y_inverse field block for a field block); one wave ahead measured
-  // faster than two or more.  Without the driver's tensor-map encoder or
-  // with a geometry the TMA cannot box, the distance stays 0.
+  // one resident wave of the kernel (resident blocks per SM x SMs); one wave
+  // ahead measured faster than two or more.  Without the driver's tensor-map
+  // encoder or with a geometry the TMA cannot box, the distance stays 0.
   template <int N> void y_prefetch_setup() {
-    using CM = ColCfg<3 * N / 2, T>;
-    auto wave = [&](const void* k, size_t smem) -> unsigned {
-      if (smem > 48 * 1024) set_smem_limit(k, smem);
+    using CM = ColPlan<T, 3 * N / 2>;
+    static_assert(ColBox<T, N, CM::TC>::ok && ColBox<T, 3 * N / 2, CM::TC>::ok, "tiles the TMA can box");
+    auto wave = [&](const void* k) -> unsigned {
+      if (CM::smem() > 36 * 1024) set_smem_limit(k, CM::smem());
       int nb = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, CM::THREADS, smem) != cudaSuccess) {
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, CM::THREADS, CM::smem()) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
       }
-      return (unsigned)(nb * nsm) & ~1u;
+      return (unsigned)(nb * nsm);
     };
     void* src[4] = {uh.p, vh.p, wh.p, Xe.p};
-    if (make_col_maps<T, N, CM::TC>(yinv_maps, src, 4, KX, NZ))
-      yinv_pdist = wave((const void*)k_y_inverse<T, N>, CM::buf());
+    if (make_col_maps<T, N, CM::TC>(yinv_maps, src, 4, KX, NZ)) yinv_pdist = wave((const void*)k_y_inverse<T, N>);
     void* X[8];
     for (int i = 0; i < 8; i++) X[i] = fused ? xout[i].p : mixed[i].p;
-    if (make_col_maps<T, 3 * N / 2, CM::TC>(yfwd_maps, X, 8, KX, NZ))
-      yfwd_pdist = wave((const void*)k_y_forward<T, N>, CM::buf() + (size_t)(3 * N / 2) * sizeof(cx<T>));
+    if (make_col_maps<T, 3 * N / 2, CM::TC>(yfwd_maps, X, 8, KX, NZ)) yfwd_pdist = wave((const void*)k_y_forward<T, N>);
   }
   ~Engine() override {
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
@@ -525,11 +522,11 @@ struct Engine : EngineBase {
       using C = ColCfg<N, T>;
       launch(k_col_small<T, N, false>, dim3(cdiv(KX, C::TC), NZ - 1), dim3(C::THREADS), C::buf(), st,
              (const cx<T>*)Xe.p, Xe.p, KX, (T)(1.0 / ((double)NX * NY)), tw);
-      using CM = ColCfg<3 * N / 2, T>;
+      using CM = ColPlan<T, 3 * N / 2>;
       Ptr8 src{}, dst{};
       src.p[0] = uh.p; src.p[1] = vh.p; src.p[2] = wh.p; src.p[3] = Xe.p;
       for (int i = 0; i < 8; i++) dst.p[i] = mixed[i].p;
-      launch(k_y_inverse<T, N>, dim3(2 * cdiv(KX, CM::TC), NZ, 4), dim3(CM::THREADS), CM::buf(), st, src, dst,
+      launch(k_y_inverse<T, N>, dim3(cdiv(KX, CM::TC), NZ, 4), dim3(CM::THREADS), CM::smem(), st, src, dst,
              KX, NZ, (T)ky0, tw, yinv_maps, yinv_pdist);
     });
     if (fused) {
@@ -539,14 +536,12 @@ struct Engine : EngineBase {
     }
     with_small(NY, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
-      using C = ColCfg<3 * N / 2, T>;
+      using C = ColPlan<T, 3 * N / 2>;
       Ptr8 X{};
       for (int i = 0; i < 8; i++) X.p[i] = fused ? xout[i].p : mixed[i].p;  // Xu1..Xe2
       Ptr8 rn{};
       rn.p[0] = run.p; rn.p[1] = rvn.p; rn.p[2] = rwn.p; rn.p[3] = rem.p;
-      // clusters of two CTAs (X1, X2) per column group
-      size_t smem = C::buf() + (size_t)(3 * N / 2) * sizeof(cx<T>);
-      launch(k_y_forward<T, N>, dim3(2 * cdiv(KX, C::TC), NZ, 4), dim3(C::THREADS), smem, st, X, rn, KX, NZ, (T)ky0,
+      launch(k_y_forward<T, N>, dim3(cdiv(KX, C::TC), NZ, 4), dim3(C::THREADS), C::smem(), st, X, rn, KX, NZ, (T)ky0,
              (T)(1.0 / ((double)MX * MY)), tw, yfwd_maps, yfwd_pdist);
     });
     if (learned_on()) learned_post(a);

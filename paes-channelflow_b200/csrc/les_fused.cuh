@@ -23,41 +23,11 @@
 
 namespace les {
 
-// Row transforms of the fused kernel, N = 12 M1.  The inverse runs decimation
-// in frequency, natural order in, permuted order out; the forward transform
-// runs the same passes backwards, permuted in, natural out.  The pointwise
-// phase does not care about the order of the points, so nothing is ever
-// reordered: every pass reads and writes the same elements in place, and a
-// pass needs one team barrier instead of the two of an autosorting pass.
-//   element n = b M1 + r R3 + i   (M1 = R2 R3, b < 12, r < R2, i < R3)
-//   pass 1 (radix 12, over b): thread j = r R3 + i
-//   pass 2 (radix R2, over r): thread (b, i), twiddle W_M1^(r i)
-//   pass 3 (radix R3, over i): thread (b, r); none when R3 = 1
-// The first factor is 12 because a padded row has modes |k| < N/3 only: of
-// pass 1's 12 inputs (outputs, forward) the middle 4 are zero (unwanted) at
-// compile time, and thread j's positive modes j + M1 b and its partner
-// M1 - j's negative ones are mirror images, exchanged by shuffles, so each
-// spectral value is loaded (stored) once.
-// Pass 1's twiddles: for N = 3 * 2^m (PFA) the factor 3 is split off by the
-// prime-factor map (no twiddles; thread j's 3-point transforms are rotated by
-// W_3^s, s = s(j), which costs two real factors per term) and the factor 4
-// needs W_(N/3)^(j k), k = 1..3: three table values a thread instead of
-// eleven.  Else (N = 9 * 2^m) W_N^(b j).  With R2 = 4 pass 2 is exactly three
-// rounds of M1 threads with one i each, again three table values.
+// Row transforms of the fused kernel: fft_inplace.cuh, a team of TP threads
+// per row.
 // Elements are padded by one per PB (one 128-byte group per element offset),
 // with which all passes' accesses at N = 768 are conflict-free, and every
 // address is a per-thread base plus a constant.
-template <int MX> struct RowPlan;
-template <> struct RowPlan<24> { static constexpr int R2 = 2, R3 = 1; };
-template <> struct RowPlan<48> { static constexpr int R2 = 4, R3 = 1; };
-template <> struct RowPlan<96> { static constexpr int R2 = 8, R3 = 1; };
-template <> struct RowPlan<144> { static constexpr int R2 = 12, R3 = 1; };
-template <> struct RowPlan<192> { static constexpr int R2 = 16, R3 = 1; };
-template <> struct RowPlan<288> { static constexpr int R2 = 4, R3 = 6; };
-template <> struct RowPlan<384> { static constexpr int R2 = 4, R3 = 8; };
-template <> struct RowPlan<576> { static constexpr int R2 = 4, R3 = 12; };
-template <> struct RowPlan<768> { static constexpr int R2 = 4, R3 = 16; };
-
 template <class T, int NSX> struct FusedCfg {
   static constexpr int MX = 3 * NSX / 2, KX = NSX / 2;
   static constexpr int R2 = RowPlan<MX>::R2, R3 = RowPlan<MX>::R3, M1 = MX / 12;
@@ -69,20 +39,13 @@ template <class T, int NSX> struct FusedCfg {
   static constexpr int THREADS = TR * ROWS;
   static constexpr int WARPS = THREADS / 32;
   static constexpr int PPT = (MX + TR - 1) / TR;         // points of a thread in phase II
-  static constexpr bool PFA = M1 % 3 != 0;
+  static constexpr bool PFA = InPlace<MX>::PFA;
   static constexpr int PB = sizeof(T) == 4 ? 16 : 8;
   static constexpr int SB = R3 == 1 ? (M1 | 1) : M1 + M1 / PB + (sizeof(T) == 8 ? 1 : 0);  // stride of b
   static constexpr int BUF = 12 * SB + (TP == 8 ? 12 : TP == 2 ? 14 : 0);
   static constexpr int NT1 = PFA ? 3 : 11;               // pass 1 twiddles of a thread
   static constexpr int NTW = NT1 * M1 + (R3 > 1 ? (R2 - 1) * R3 : 0);
-  // x of the point at element n: b = 4 x3 + k4 and kappa = k4 + 4 (r + R2 i)
-  // stand for x mod 3 = x3, x mod N/3 = 3 kappa (PFA); else b + 12 (r + R2 i)
-  static __device__ __forceinline__ int x_of(int n) {
-    const int b = n / M1, m = n - b * M1, o = m / R3 + R2 * (m % R3);
-    if (!PFA) return b + 12 * o;
-    constexpr int Q = 4 * M1, U = Q % 3 == 1 ? Q : 2 * Q;  // U = 1 mod 3, 0 mod Q
-    return ((b >> 2) * U + 3 * ((b & 3) + 4 * o)) % MX;
-  }
+  static __device__ __forceinline__ int x_of(int n) { return InPlace<MX>::x_of(n); }
   static constexpr size_t smem() { return ((size_t)6 * ROWS * BUF + NTW) * sizeof(cx<T>); }
   // Resident CTAs per SM the register budget aims at: 24 warps of <= 80
   // registers in FP32, 12 of <= 168 in FP64.  Tighter budgets spill (FP64 at
@@ -99,107 +62,9 @@ template <class T, int NSX> struct FusedCfg {
   }
 };
 
-// a + s b, one packed instruction in FP32
-template <class T> __device__ __forceinline__ cx<T> axpy(cx<T> a, T s, cx<T> b) { return mk(a.x + s * b.x, a.y + s * b.y); }
-template <> __device__ __forceinline__ cx<float> axpy<float>(cx<float> a, float s, cx<float> b) {
-  cx<float> r;
-  asm("{\n\t.reg .b64 a, b, s, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 s, {%6, %6};\n\t"
-      "fma.rn.f32x2 r, b, s, a;\n\tmov.b64 {%0, %1}, r;\n\t}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(s));
-  return r;
-}
-// a + s i b
-template <class T> __device__ __forceinline__ cx<T> axipy(cx<T> a, T s, cx<T> b) { return mk(a.x - s * b.y, a.y + s * b.x); }
-
-// 12-point DFTs as 3 x 4 without inner twiddles (prime-factor maps: input
-// n = 4 a + 3 c, output k = 4 k3 + 9 k4, both mod 12).
-// Inverse with inputs 4..7 zero: x[0..3] inputs 0..3, x[4..7] inputs 8..11.
-template <class T> __device__ __forceinline__ void dft12_padded(const cx<T> (&x)[8], cx<T> (&y)[12]) {
-  constexpr T h = (T)0.5, s3 = (T)0.86602540378443864676372317075293618;
-  cx<T> g[3][4];  // [k3][c]
-  // c = 0: inputs 0, 4, 8;  c = 1: 3, 7, 11 (the second is zero)
-#pragma unroll
-  for (int c = 0; c < 2; c++) {
-    const cx<T> p = c == 0 ? x[0] : x[3], q = c == 0 ? x[4] : x[7];
-    const cx<T> t = axpy<T>(p, -h, q);
-    g[0][c] = p + q;
-    g[1][c] = axipy<T>(t, -s3, q);
-    g[2][c] = axipy<T>(t, s3, q);
-  }
-  {  // c = 2: inputs 6, 10, 2 (the first is zero)
-    const cx<T> s = x[6] + x[2], d = x[6] - x[2], t = s * (-h);
-    g[0][2] = s;
-    g[1][2] = axipy<T>(t, s3, d);
-    g[2][2] = axipy<T>(t, -s3, d);
-  }
-  {  // c = 3: inputs 9, 1, 5 (the third is zero)
-    const cx<T> t = axpy<T>(x[5], -h, x[1]);
-    g[0][3] = x[5] + x[1];
-    g[1][3] = axipy<T>(t, s3, x[1]);
-    g[2][3] = axipy<T>(t, -s3, x[1]);
-  }
-#pragma unroll
-  for (int k3 = 0; k3 < 3; k3++) {
-    Dft<4, +1, T>::run(g[k3]);
-#pragma unroll
-    for (int k4 = 0; k4 < 4; k4++) y[(4 * k3 + 9 * k4) % 12] = g[k3][k4];
-  }
-}
-// Forward with all inputs; the caller leaves outputs 4..7 unused.
-template <class T> __device__ __forceinline__ void dft12_forward(const cx<T> (&x)[12], cx<T> (&y)[12]) {
-  constexpr T h = (T)0.5, s3 = (T)0.86602540378443864676372317075293618;
-  cx<T> g[3][4];
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-#pragma unroll
-    for (int c = 0; c < 4; c++) g[a][c] = x[(4 * a + 3 * c) % 12];
-    Dft<4, -1, T>::run(g[a]);
-  }
-#pragma unroll
-  for (int k4 = 0; k4 < 4; k4++) {
-    const cx<T> s = g[1][k4] + g[2][k4], d = g[1][k4] - g[2][k4], t = axpy<T>(g[0][k4], -h, s);
-    y[(9 * k4) % 12] = g[0][k4] + s;
-    y[(4 + 9 * k4) % 12] = axipy<T>(t, -s3, d);
-    y[(8 + 9 * k4) % 12] = axipy<T>(t, s3, d);
-  }
-}
-
 template <class T> __device__ __forceinline__ cx<T> shfl_cx(unsigned mask, cx<T> v, int src) {
   return mk(__shfl_sync(mask, v.x, src), __shfl_sync(mask, v.y, src));
 }
-
-// Rotated 12-point DFT of pass 1 for N = 3 * 2^m: 3-point transforms over a
-// (input n = j + M1 (c + 4 a), rotated by W_3^(s_c x3), s_c = s + c M1 u mod 3
-// with u = (N/3)^-1 mod 3), then 4-point transforms over c; output b = 4 x3 + k4.
-// w[s] = W_3^(s(j) + s) for s = 0..2.
-template <class T, int M1> struct Dft12Pfa {
-  static constexpr int U = (4 * M1) % 3, STEP = (U * M1) % 3;  // u = Q^-1 = Q mod 3
-  // inverse, inputs 4..7 zero: x[0..3] inputs 0..3, x[4..7] inputs 8..11
-  static __device__ __forceinline__ void padded(const cx<T> (&x)[8], const cx<T> (&w)[3], cx<T> (&y)[12]) {
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const cx<T> p = x[c], q = x[4 + c], al = w[(c * STEP) % 3], be = w[(c * STEP + 2) % 3];
-      const cx<T> re = axpy<T>(p * al.x, be.x, q), im = axpy<T>(p * al.y, be.y, q);
-      y[c] = p + q;
-      y[4 + c] = mk(re.x - im.y, re.y + im.x);
-      y[8 + c] = mk(re.x + im.y, re.y - im.x);
-    }
-#pragma unroll
-    for (int k3 = 0; k3 < 3; k3++) Dft<4, +1, T>::run(y + 4 * k3);
-  }
-  // forward, outputs 0..3 and 8..11 (z[0..3], z[4..7])
-  static __device__ __forceinline__ void forward(cx<T> (&y)[12], const cx<T> (&w)[3], cx<T> (&z)[8]) {
-#pragma unroll
-    for (int k3 = 0; k3 < 3; k3++) Dft<4, -1, T>::run(y + 4 * k3);
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const cx<T> s = y[4 + c] + y[8 + c], d = y[4 + c] - y[8 + c], al = w[(c * STEP) % 3], be = w[(c * STEP + 2) % 3];
-      z[c] = axipy<T>(axpy<T>(y[c], al.x, s), -al.y, d);
-      z[4 + c] = axipy<T>(axpy<T>(y[c], be.x, s), -be.y, d);
-    }
-  }
-};
 
 // Passes 2 and 3 of a team's transform in its buffer.  t = thread of the
 // team.  INV: pass 2 then 3; else 3 then 2, with the conjugate twiddles.
@@ -314,7 +179,7 @@ template <> __device__ __forceinline__ float tke_sqrt<float>(float e) {
 // 64x64x64 FP64 168 -> 47 us.
 template <class T, int NSX>
 __global__ void __launch_bounds__(FusedCfg<T, NSX>::THREADS, FusedCfg<T, NSX>::CTAS)
-k_row_fused(FusedArgs f, StageArgs a, const cx<T>* __restrict__ tw) {
+k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageArgs a, const cx<T>* __restrict__ tw) {
   using C = FusedCfg<T, NSX>;
   constexpr int MX = C::MX, KX = C::KX, M1 = C::M1, R2 = C::R2, R3 = C::R3, TP = C::TP, TR = C::TR;
   constexpr int BUF = C::BUF, SB = C::SB, PPT = C::PPT;
@@ -367,12 +232,8 @@ k_row_fused(FusedArgs f, StageArgs a, const cx<T>* __restrict__ tw) {
   if (!act) j = 0;
   cx<T>* pj = buf + C::off(j);
   const cx<T>* twj = tw1 + j;
-  cx<T> w3[3];  // W_3^(s(j) + 0, 1, 2), s(j) = j u mod 3 (PFA)
-#pragma unroll
-  for (int s = 0; s < 3; s++) {
-    const int e = (j * Dft12Pfa<T, M1>::U + s) % 3;
-    w3[s] = mk(e ? (T)-0.5 : (T)1, e == 0 ? (T)0 : (e == 1 ? (T)1 : (T)-1) * (T)0.86602540378443864676372317075293618);
-  }
+  cx<T> w3[3];
+  InPlace<MX>::rotations(j, w3);
 
   const T dzm = (T)a.dzm, todzm = (T)a.todzm, emin = (T)a.emin;
   const T xkmax = (T)a.xkmax, nu = (T)a.nu, c01 = (T)0.1 * (T)a.dsl;

@@ -26,9 +26,8 @@
 //   k_press                     comprhs + press (tridv) per (kx, ky) and
 //                               comp2 in spectral space, FP64
 #pragma once
-#include <cooperative_groups.h>
-
 #include "fft_core.cuh"
+#include "fft_inplace.cuh"
 #include "les_tma.cuh"
 
 namespace les {
@@ -280,45 +279,168 @@ k_e_prep(T* __restrict__ e, const T* __restrict__ re, cx<T>* __restrict__ Xe, in
 struct Ptr8 { void* p[8]; };
 struct Ptr12 { void* p[12]; };
 
+// Column transforms along y on the padded grid (M = 3 NS/2 = 12 M1, small
+// length NS = 8 M1): a CTA owns TC columns (64-byte row segments) and M1
+// threads per column, thread = (column t, j).  In place (fft_inplace.cuh),
+// two shared-memory tiles (two transforms side by side, one pair of barriers
+// for both).  Element n sits at row b SB + r SR + i of its tile; SR is odd,
+// so that neighbouring threads' rows alternate between the two halves of the
+// banks in every pass, and every address is a base plus a constant.
+template <class T, int M> struct ColPlan {
+  using P = InPlace<M>;
+  static constexpr int M1 = P::M1, R2 = P::R2, R3 = P::R3, NS = 8 * M1;
+  static constexpr int TCB = sizeof(T) == 8 ? 4 : 8;
+  static constexpr int TC = TCB * ((64 + TCB * M1 - 1) / (TCB * M1));  // at least 64 threads
+  static constexpr int THREADS = TC * M1;
+  static constexpr int SR = R3 > 1 ? R3 + 1 : 1, SB = R3 > 1 ? R2 * SR : (M1 | 1);
+  static constexpr int BUF = 12 * SB * TC;
+  static constexpr size_t smem() { return (size_t)2 * BUF * sizeof(cx<T>); }
+  // CTAs per SM the register budget aims at (both tiles' shared memory allows it)
+  static constexpr int CTAS = (sizeof(T) == 8 ? 512 : 1024) / THREADS;
+  static __device__ __forceinline__ int off(int m) { return R3 > 1 ? (m / R3) * SR + m % R3 : m; }
+  // this thread's pass 2 twiddles W_M1^(r i), r = 1..3
+  static __device__ __forceinline__ void twiddles2(const cx<T>* tw, int q, cx<T> (&w)[4]) {
+    if constexpr (R3 > 1) {
+      const cx<T>* g = tw + tw_off(M);
+#pragma unroll
+      for (int r = 1; r < 4; r++) w[r] = g[12 * r * (q % R3)];
+    }
+  }
+  // pass 2 of NB blocks b (12 padded, 8 small) of a tile, R3 > 1
+  template <int NB, bool INV> static __device__ __forceinline__ void pass2(cx<T>* buf, const cx<T> (&w)[4], int q) {
+    static_assert(R3 == 1 || R2 == 4, "rounds of M1 threads");
+    cx<T>* p = buf + (size_t)((q / R3) * SB + q % R3) * TC;
+#pragma unroll
+    for (int jj = 0; jj < NB / 4; jj++) {
+      cx<T> v[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        v[r] = p[(4 * jj * SB + r * SR) * TC];
+        if (!INV && r > 0) v[r] = cmul(v[r], w[r]);
+      }
+      Dft<4, INV ? +1 : -1, T>::run(v);
+#pragma unroll
+      for (int r = 0; r < 4; r++) p[(4 * jj * SB + r * SR) * TC] = (INV && r > 0) ? cmul(v[r], conj(w[r])) : v[r];
+    }
+  }
+  // last pass of an inverse transform of NB blocks: store(row, value); rows in
+  // the order of the padded map (NB = 12) or b + NB (r + R2 i)
+  template <int NB, class StoreF> static __device__ __forceinline__ void last(const cx<T>* buf, int q, StoreF store) {
+    constexpr int R = R3 > 1 ? R3 : R2, ITEMS = R3 > 1 ? NB * R2 : NB;
+#pragma unroll
+    for (int it = 0; it < (ITEMS + M1 - 1) / M1; it++) {
+      const int u = q + it * M1;
+      if (ITEMS % M1 != 0 && u >= ITEMS) break;
+      const int b = R3 > 1 ? u / R2 : u, r = R3 > 1 ? u % R2 : 0;
+      const cx<T>* p = buf + (size_t)(b * SB + r * SR) * TC;
+      cx<T> v[R];
+#pragma unroll
+      for (int i = 0; i < R; i++) v[i] = p[i * TC];
+      Dft<R, +1, T>::run(v);
+      const int x0 = NB == 12 ? P::x_of(b * M1 + r * R3) : b + NB * r;
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        int x = x0 + NB * (R3 > 1 ? R2 : 1) * i;
+        if (NB == 12 && P::PFA) x = x >= M ? x - M : x;
+        store(x, v[i]);
+      }
+    }
+  }
+  // first pass of a forward transform of the padded rows load(row)
+  template <class LoadF> static __device__ __forceinline__ void first(cx<T>* buf, int q, LoadF load) {
+    constexpr int R = R3 > 1 ? R3 : R2, ITEMS = R3 > 1 ? 12 * R2 : 12;
+#pragma unroll
+    for (int it = 0; it < (ITEMS + M1 - 1) / M1; it++) {
+      const int u = q + it * M1;
+      if (ITEMS % M1 != 0 && u >= ITEMS) break;
+      const int b = R3 > 1 ? u / R2 : u, r = R3 > 1 ? u % R2 : 0;
+      cx<T>* p = buf + (size_t)(b * SB + r * SR) * TC;
+      const int x0 = P::x_of(b * M1 + r * R3);
+      cx<T> v[R];
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        int x = x0 + 12 * (R3 > 1 ? R2 : 1) * i;
+        if (P::PFA) x = x >= M ? x - M : x;
+        v[i] = load(x);
+      }
+      Dft<R, -1, T>::run(v);
+#pragma unroll
+      for (int i = 0; i < R; i++) p[i * TC] = v[i];
+    }
+  }
+};
+
+// Pass 1 twiddles of thread j: W_(M/3)^(k j), k = 1..3 (PFA), or W_M^(b j).
+template <class T, int M> struct ColTw1 {
+  static constexpr int NT = InPlace<M>::PFA ? 3 : 11;
+  cx<T> w[NT];
+  __device__ __forceinline__ ColTw1(const cx<T>* tw, int j) {
+    const cx<T>* g = tw + tw_off(M);
+#pragma unroll
+    for (int k = 0; k < NT; k++) w[k] = g[(InPlace<M>::PFA ? 3 : 1) * (k + 1) * j];
+  }
+  __device__ __forceinline__ cx<T> of(int b) const { return InPlace<M>::PFA ? w[(b & 3) ? (b & 3) - 1 : 0] : w[b ? b - 1 : 0]; }
+  static __device__ __forceinline__ bool one(int b) { return InPlace<M>::PFA ? (b & 3) == 0 : b == 0; }
+};
+
 // expand() of u, v, w, e in y fused with d/dy: for field f = blockIdx.z
 // (u, v, w, e), out[2f] = IFFT_M(pad(s)) and out[2f+1] = IFFT_M(i*ky*pad(s)),
-// TC columns per block.  The field and its derivative go to separate blocks
-// (h = blockIdx.x & 1), adjacent in launch order so that the second reads
-// the columns from L2: half the block of a paired form, so that two blocks
-// share an SM and one's loads overlap the other's transform and stores
-// (measured 22% faster in FP32 than TC paired transforms per block).
-// Thread 0 of a field block first has the TMA prefetch into L2 the columns
-// of the field block `pdist` blocks ahead (les_tma.cuh; maps: tensor maps of
-// src[0..3] as [NZ*NS][KX] rows; pdist 0 prefetches nothing).
+// TC columns per block, both from one load of the columns (8 values a
+// thread).  Thread 0 first has the TMA prefetch into L2 the columns of the
+// block `pdist` blocks ahead (les_tma.cuh; maps: tensor maps of src[0..3] as
+// [NZ*NS][KX] rows; pdist 0 prefetches nothing).
 template <class T, int NS>
-__global__ void __launch_bounds__(ColCfg<3 * NS / 2, T>::THREADS)
-k_y_inverse(Ptr8 src, Ptr8 dst, int KX, int NZ, T ky0, const cx<T>* __restrict__ tw,
+__global__ void __launch_bounds__(ColPlan<T, 3 * NS / 2>::THREADS, ColPlan<T, 3 * NS / 2>::CTAS)
+k_y_inverse(const __grid_constant__ Ptr8 src, const __grid_constant__ Ptr8 dst, int KX, int NZ, T ky0, const cx<T>* __restrict__ tw,
             const __grid_constant__ ColMaps maps, unsigned pdist) {
   constexpr int M = 3 * NS / 2;
-  using C = ColCfg<M, T>;
-  if ((blockIdx.x & 1) == 0)
-    prefetch_tile_ahead<T, NS, C::TC>(maps, pdist, [&](unsigned bx, unsigned by, unsigned bz, int& q, int& cg,
-                                                       int& row0) {
-      q = (int)bz; cg = (int)(bx >> 1); row0 = (int)by * NS;
-      return !(bz >= 2 && (int)by + 1 == NZ);
-    });
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  const int f = blockIdx.z, h = blockIdx.x & 1, z = blockIdx.y + 1;
-  if (f >= 2 && z == NZ) return;
-  const int kx0 = (blockIdx.x >> 1) * C::TC;
-  const cx<T>* in = reinterpret_cast<const cx<T>*>(src.p[f]) + (size_t)(z - 1) * NS * KX;
-  cx<T>* out = reinterpret_cast<cx<T>*>(dst.p[2 * f + h]) + (size_t)(z - 1) * M * KX;
-  fft_core<M, +1, true, false, false>(C::TC, sm, tw, [&](int t, int n) {
-    const int kx = kx0 + t;
-    const int ky = (n < NS / 2) ? n : ((n > NS) ? n - NS / 2 : -1);
-    cx<T> v = (kx < KX && ky >= 0) ? in[(size_t)ky * KX + kx] : zero_cx<T>();
-    if (h) v = mul_i(v) * (ky0 * (T)signed_k(n, M));
-    return v;
-  }, [&](int t, int n, cx<T> v) {
-    const int kx = kx0 + t;
-    if (kx < KX) out[(size_t)n * KX + kx] = v;
+  using C = ColPlan<T, M>;
+  constexpr int TC = C::TC, M1 = C::M1;
+  prefetch_tile_ahead<T, NS, TC>(maps, pdist, [&](unsigned bx, unsigned by, unsigned bz, int& q, int& cg, int& row0) {
+    q = (int)bz; cg = (int)bx; row0 = (int)by * NS;
+    return !(bz >= 2 && (int)by + 1 == NZ);
   });
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int f = blockIdx.z, z = blockIdx.y + 1;
+  if (f >= 2 && z == NZ) return;
+  const int t = threadIdx.x % TC, j = threadIdx.x / TC;
+  const int kx = blockIdx.x * TC + t;
+  const bool in = kx < KX;
+  cx<T>* buf = reinterpret_cast<cx<T>*>(smraw) + t;
+  const cx<T>* s = reinterpret_cast<const cx<T>*>(src.p[f]) + (size_t)(z - 1) * NS * KX + (in ? kx : 0);
+  cx<T> x[8], w2[4];
+#pragma unroll
+  for (int m = 0; m < 8; m++) x[m] = (m == 4 && j == 0) ? zero_cx<T>() : s[(j + M1 * m) * KX];  // no Nyquist mode
+  const ColTw1<T, M> tw1(tw, j);
+  C::twiddles2(tw, j, w2);
+  cx<T> w3[3];
+  InPlace<M>::rotations(j, w3);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    cx<T> v[12];
+    if (h) {
+#pragma unroll
+      for (int m = 0; m < 8; m++) x[m] = mul_i(x[m]) * (ky0 * (T)(m < 4 ? j + M1 * m : j + M1 * m - NS));
+    }
+    if constexpr (InPlace<M>::PFA) Dft12Pfa<T, M1>::padded(x, w3, v);
+    else dft12_padded<T>(x, v);
+    cx<T>* p = buf + h * C::BUF + C::off(j) * TC;
+#pragma unroll
+    for (int b = 0; b < 12; b++) p[b * C::SB * TC] = ColTw1<T, M>::one(b) ? v[b] : cmul(v[b], conj(tw1.of(b)));
+  }
+  __syncthreads();
+  if constexpr (C::R3 > 1) {
+    C::template pass2<12, true>(buf, w2, j);
+    C::template pass2<12, true>(buf + C::BUF, w2, j);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    cx<T>* out = reinterpret_cast<cx<T>*>(dst.p[2 * f + h]) + (size_t)(z - 1) * M * KX + kx;
+    C::template last<12>(buf + h * C::BUF, j, [&](int row, cx<T> v) {
+      if (in) out[row * KX] = v;
+    });
+  }
 }
 
 // expand() in x fused with d/dx: six paired inverse row transforms give
@@ -327,7 +449,7 @@ k_y_inverse(Ptr8 src, Ptr8 dst, int KX, int NZ, T ky0, const cx<T>* __restrict__
 // WY, E, EX, EY.  blockIdx.z = group.
 template <class T, int NSX>
 __global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS)
-k_x_inverse(Ptr8 src, Ptr12 dst, int MY, int NZ, T kx0, const cx<T>* __restrict__ tw) {
+k_x_inverse(const __grid_constant__ Ptr8 src, const __grid_constant__ Ptr12 dst, int MY, int NZ, T kx0, const cx<T>* __restrict__ tw) {
   constexpr int MX = 3 * NSX / 2;
   constexpr int KX = NSX / 2;
   using C = RowCfg<MX>;
@@ -781,7 +903,7 @@ k_flux(Ptr12 in, Ptr11 out, StageArgs a, const WallParams* __restrict__ wpp, dou
 // in: A,B,C,D,G,F,H,Pu,Pv,Pw,Pe; out: Xu1,Xu2,Xv1,Xv2,Xw1,Xw2,Xe1,Xe2
 template <class T, int NSX>
 __global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS)
-k_x_forward(Ptr11 in, Ptr8 out, int MY, int NZ, T kx0, const cx<T>* __restrict__ tw) {
+k_x_forward(const __grid_constant__ Ptr11 in, const __grid_constant__ Ptr8 out, int MY, int NZ, T kx0, const cx<T>* __restrict__ tw) {
   constexpr int MX = 3 * NSX / 2;
   constexpr int KX = NSX / 2;
   using C = RowCfg<MX>;
@@ -823,70 +945,99 @@ k_x_forward(Ptr11 in, Ptr8 out, int MY, int NZ, T kx0, const cx<T>* __restrict__
 // compress() in y fused with -d/dy: for field f (u, v, w, e)
 //   R^(ky) = (FFT_M(X1) - i ky FFT_M(X2)) / (MX*MY) at the kept ky,
 // rw's plane mean removed (comp1.f90:172).  R^ of u, v, w is written to
-// rnew[f]; for e, re = IFFT_N(R^) (x-spectral) is written to rnew[3].
-// A cluster of two CTAs per column group (blockIdx.x = 2 group + rank):
-// rank 0 transforms X1, rank 1 X2, each into its own shared memory; after a
-// cluster barrier each rank combines half of the kept ky rows, reading the
-// other rank's transform through distributed shared memory (for e, rank 0
-// combines all rows in place and runs the inverse N-point transform after a
-// second cluster barrier).  Half the shared memory and threads of a CTA that
-// held both transforms: FP64 2.6% faster, FP32 unchanged.  Thread 0 first
-// has the TMA prefetch into L2 the columns of the block `pdist` blocks
-// ahead (les_tma.cuh; maps: tensor maps of X[0..7] as [NZ*M][KX] rows;
-// pdist 0 prefetches nothing).
+// rnew[f]; for e, re = IFFT_NS(R^) (x-spectral) is written to rnew[3].
+// TC columns per block (ColPlan); X1 and X2 go through the two tiles, the
+// rows loaded in the permuted order, and meet in the registers of thread j,
+// whose eight kept outputs are ky = j + M1 m: for e these are also the inputs
+// of the inverse transform's radix-8 first pass.  Thread 0 first has the TMA
+// prefetch into L2 the columns of the block `pdist` blocks ahead (les_tma.cuh;
+// maps: tensor maps of X[0..7] as [NZ*M][KX] rows; pdist 0 prefetches nothing).
 template <class T, int NS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ColCfg<3 * NS / 2, T>::THREADS)
-k_y_forward(Ptr8 X, Ptr8 rnew, int KX, int NZ, T ky0, T scale, const cx<T>* __restrict__ tw,
+__global__ void __launch_bounds__(ColPlan<T, 3 * NS / 2>::THREADS, ColPlan<T, 3 * NS / 2>::CTAS)
+k_y_forward(const __grid_constant__ Ptr8 X, const __grid_constant__ Ptr8 rnew, int KX, int NZ, T ky0, T scale, const cx<T>* __restrict__ tw,
             const __grid_constant__ ColMaps maps, unsigned pdist) {
   constexpr int M = 3 * NS / 2;
-  using C = ColCfg<M, T>;
-  constexpr int TC = C::TC;
-  prefetch_tile_ahead<T, M, TC>(maps, pdist, [&](unsigned bx, unsigned by, unsigned bz, int& q, int& cg, int& row0) {
-    q = 2 * (int)bz + (int)(bx & 1); cg = (int)(bx >> 1); row0 = (int)by * M;
-    return !(bz >= 2 && (int)by + 1 == NZ);
-  });
+  using C = ColPlan<T, M>;
+  constexpr int TC = C::TC, M1 = C::M1;
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+    prefetch_tile_ahead<T, M, TC>(maps, pdist, [&](unsigned bx, unsigned by, unsigned bz, int& q, int& cg, int& row0) {
+      q = 2 * (int)bz + h; cg = (int)bx; row0 = (int)by * M;
+      return !(bz >= 2 && (int)by + 1 == NZ);
+    });
   extern __shared__ __align__(16) unsigned char smraw[];
-  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-  const int rank = (int)cluster.block_rank();
   const int f = blockIdx.z, z = blockIdx.y + 1;
   if (f >= 2 && z == NZ) return;
-  const int kx0 = (blockIdx.x >> 1) * TC;
-  const cx<T>* Xs = (const cx<T>*)X.p[2 * f + rank] + (size_t)(z - 1) * M * KX;
-  // the twiddles of the M-point transform staged in shared memory (measured
-  // faster here than reading them through L1)
-  const cx<T>* tws = stage_twiddles<M>(sm + (size_t)TC * M, tw);
-  fft_core_tab<M, -1, true, false, true>(TC, sm, tws, [&](int t, int n) {
-    int kx = kx0 + t;
-    return (kx < KX) ? Xs[(size_t)n * KX + kx] : zero_cx<T>();
-  }, NoStore{});
-  cluster.sync();
-  const cx<T>* s1 = cluster.map_shared_rank(sm, 0);
-  const cx<T>* s2 = cluster.map_shared_rank(sm, 1);
-  cx<T>* dst = (cx<T>*)rnew.p[f] + (size_t)(z - 1) * NS * KX;
-  constexpr int ITEMS = TC * NS;
-  const int lo = (f == 3) ? 0 : rank * (ITEMS / 2);
-  const int hi = (f == 3) ? (rank == 0 ? ITEMS : 0) : lo + ITEMS / 2;
-  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    int t = i % TC, ky = i / TC, kx = kx0 + t;
-    int n = (ky < NS / 2) ? ky : ky + NS / 2;
-    cx<T> v = zero_cx<T>();
-    if (ky != NS / 2) {
-      cx<T> y1 = s1[n * TC + t], y2 = s2[n * TC + t];
-      T kk = ky0 * (T)signed_k(ky, NS);
-      v = mk(y1.x + kk * y2.y, y1.y - kk * y2.x) * scale;
-      if (f == 2 && kx == 0 && ky == 0) v = zero_cx<T>();
+  const int t = threadIdx.x % TC, j = threadIdx.x / TC;
+  const int kx = blockIdx.x * TC + t;
+  const bool in = kx < KX;
+  cx<T>* buf = reinterpret_cast<cx<T>*>(smraw) + t;
+  cx<T> w2[4];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const cx<T>* s = reinterpret_cast<const cx<T>*>(X.p[2 * f + h]) + (size_t)(z - 1) * M * KX + (in ? kx : 0);
+    C::first(buf + h * C::BUF, j, [&](int row) { return s[row * KX]; });
+  }
+  C::twiddles2(tw, j, w2);
+  __syncthreads();
+  if constexpr (C::R3 > 1) {
+    C::template pass2<12, false>(buf, w2, j);
+    C::template pass2<12, false>(buf + C::BUF, w2, j);
+    __syncthreads();
+  }
+  const ColTw1<T, M> tw1(tw, j);
+  cx<T> w3[3], R[8];
+  InPlace<M>::rotations(j, w3);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const cx<T>* p = buf + h * C::BUF + C::off(j) * TC;
+    cx<T> v[12], o[8];
+#pragma unroll
+    for (int b = 0; b < 12; b++) v[b] = ColTw1<T, M>::one(b) ? p[b * C::SB * TC] : cmul(p[b * C::SB * TC], tw1.of(b));
+    if constexpr (InPlace<M>::PFA) Dft12Pfa<T, M1>::forward(v, w3, o);
+    else {
+      cx<T> y[12];
+      dft12_forward<T>(v, y);
+#pragma unroll
+      for (int m = 0; m < 4; m++) { o[m] = y[m]; o[4 + m] = y[8 + m]; }
     }
-    if (f < 3) { if (kx < KX) dst[(size_t)ky * KX + kx] = v; }
-    else sm[ky * TC + t] = v;
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+      if (h == 0) R[m] = o[m];
+      else {
+        const T kk = ky0 * (T)(m < 4 ? j + M1 * m : j + M1 * m - NS);
+        R[m] = mk(R[m].x + kk * o[m].y, R[m].y - kk * o[m].x) * scale;
+      }
+    }
   }
-  cluster.sync();
-  if (f == 3 && rank == 0) {
-    fft_core<NS, +1, true, true, false>(TC, sm, tw, NoLoad{}, [&](int t, int n, cx<T> v) {
-      int kx = kx0 + t;
-      if (kx < KX) dst[(size_t)n * KX + kx] = v;
-    });
+  if (j == 0) {
+    R[4] = zero_cx<T>();  // Nyquist
+    if (f == 2 && kx == 0) R[0] = zero_cx<T>();
   }
+  cx<T>* dst = reinterpret_cast<cx<T>*>(rnew.p[f]) + (size_t)(z - 1) * NS * KX + kx;
+  if (f < 3) {
+#pragma unroll
+    for (int m = 0; m < 8; m++)
+      if (in) dst[(j + M1 * m) * KX] = R[m];
+    return;
+  }
+  // e: inverse transform of length NS = 8 M1 in the first tile (thread j's
+  // pass 1 writes the elements it has just read)
+  Dft<8, +1, T>::run(R);
+  {
+    const cx<T>* g = tw + tw_off(NS);
+    cx<T>* p = buf + C::off(j) * TC;
+#pragma unroll
+    for (int b = 0; b < 8; b++) p[b * C::SB * TC] = b ? cmul(R[b], conj(g[b * j])) : R[b];
+  }
+  __syncthreads();
+  if constexpr (C::R3 > 1) {
+    C::template pass2<8, true>(buf, w2, j);
+    __syncthreads();
+  }
+  C::template last<8>(buf, j, [&](int row, cx<T> v) {
+    if (in) dst[row * KX] = v;
+  });
 }
 
 // The stage's e update (comp1.f90:131, comp2.f90:38) with re from its

@@ -1,19 +1,17 @@
 // les_tma.cuh -- L2 prefetch of y-column tiles by the tensor memory
 // accelerator (TMA).
 //
-// The y-column transforms (k_y_inverse, k_y_forward) read one column tile
-// per CTA: TC complex columns of an x-spectral array, every row of one level
-// (NS spectral rows, or M = 3NS/2 padded rows), 64-byte row segments with a
-// row stride of KX complex values.  A CTA loads its tile, transforms it and
-// stores the result, so DRAM idles while the resident CTAs compute.  Here
-// thread 0 of each CTA first asks the TMA to bring the tile of the CTA
-// `pdist` blocks later in launch order (about one resident wave ahead) into
-// L2 (cp.async.bulk.prefetch.tensor): that tile's DRAM reads overlap this
-// wave's transforms, and its CTA later finds its columns in L2.  A prefetch
-// has no destination in shared memory and nothing waits on it; the results
-// are those of the kernels without it (checked bit for bit on B200 at
-// 512x512x256: FP64 k_y_forward 3.65 -> 3.44 ms, k_y_inverse 2.11 -> 2.00 ms
-// per stage; FP32 about 1%; two or more waves ahead was slower than one).
+// The y-column transforms (k_y_inverse, k_y_forward) read column tiles: TC
+// complex columns of an x-spectral array, every row of one level (NS spectral
+// rows, or M = 3NS/2 padded rows), 64-byte row segments with a row stride of
+// KX complex values.  A CTA loads its tile, transforms it and stores the
+// result, so DRAM idles while the resident CTAs compute.  Here thread 0 of
+// each CTA first asks the TMA to bring the tile of the CTA `pdist` blocks
+// later in launch order (one resident wave ahead) into L2
+// (cp.async.bulk.prefetch.tensor): that tile's DRAM reads overlap this wave's
+// transforms, and its CTA later finds its columns in L2.  A prefetch has no
+// destination in shared memory and nothing waits on it; the results are those
+// of the kernels without it.
 //
 // The arrays are described to the TMA as 2-D tensors of real elements:
 // dim 0 the 2KX reals of one row, dim 1 all rows of all levels.  A tile is
