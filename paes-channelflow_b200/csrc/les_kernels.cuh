@@ -285,7 +285,14 @@ struct Ptr12 { void* p[12]; };
 // two shared-memory tiles (two transforms side by side, one pair of barriers
 // for both).  Element n sits at row b SB + r SR + i of its tile; SR is odd,
 // so that neighbouring threads' rows alternate between the two halves of the
-// banks in every pass, and every address is a base plus a constant.
+// banks in every pass, and every address is a base plus a constant.  The
+// pointer arrays are __grid_constant__: indexed by blockIdx.z, a plain struct
+// parameter was copied to local memory by every thread (a quarter of the
+// kernels' time).  Per stage at 512x512x256, against one two-pass transform
+// per CTA: k_y_inverse FP32 1.09 -> 0.92 ms, FP64 2.03 -> 1.89; k_y_forward
+// 1.87 -> 1.21, 3.43 -> 2.32 ms (HBM floors 0.66 and 1.31); at 64x64x64 FP64
+// 18 -> 11 and 28 -> 12 us.  Bound by load latency and the load/store path
+// (64-byte rows) at about half of DRAM's peak.
 template <class T, int M> struct ColPlan {
   using P = InPlace<M>;
   static constexpr int M1 = P::M1, R2 = P::R2, R3 = P::R3, NS = 8 * M1;
