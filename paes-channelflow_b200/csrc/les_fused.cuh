@@ -25,9 +25,12 @@ namespace les {
 
 // Row transforms of the fused kernel: fft_inplace.cuh, a team of TP threads
 // per row.
-// Elements are padded by one per PB (one 128-byte group per element offset),
-// with which all passes' accesses at N = 768 are conflict-free, and every
-// address is a per-thread base plus a constant.
+// Element (b, r, i) sits at b SB + r SR + i; SR and SB come from counting the
+// wavefronts of every pass over a warp's lanes (FP32: 16 lanes a wavefront,
+// FP64: 8): with them all passes but pass 1 are conflict-free for R3 >= 8, and
+// every address is a per-thread base plus a constant.  (One pad element per
+// 128 bytes instead took 2.2 times the minimum at 576 points in FP32, 1.7 times
+// in FP64, 1.3 at 384 and 1.7 at 288.)
 template <class T, int NSX> struct FusedCfg {
   static constexpr int MX = 3 * NSX / 2, KX = NSX / 2;
   static constexpr int R2 = RowPlan<MX>::R2, R3 = RowPlan<MX>::R3, M1 = MX / 12;
@@ -40,8 +43,9 @@ template <class T, int NSX> struct FusedCfg {
   static constexpr int WARPS = THREADS / 32;
   static constexpr int PPT = (MX + TR - 1) / TR;         // points of a thread in phase II
   static constexpr bool PFA = InPlace<MX>::PFA;
-  static constexpr int PB = sizeof(T) == 4 ? 16 : 8;
-  static constexpr int SB = R3 == 1 ? (M1 | 1) : M1 + M1 / PB + (sizeof(T) == 8 ? 1 : 0);  // stride of b
+  static constexpr bool F32 = sizeof(T) == 4;
+  static constexpr int SR = R3 == 16 ? 17 : R3 == 12 ? 15 : R3 == 8 ? 9 : R3 == 6 ? (F32 ? 7 : 6) : 1;
+  static constexpr int SB = R3 == 1 ? (M1 | 1) : R2 * SR + (R3 == 6 && !F32 ? 1 : 0);
   static constexpr int BUF = 12 * SB + (TP == 8 ? 12 : TP == 2 ? 14 : 0);
   static constexpr int NT1 = PFA ? 3 : 11;               // pass 1 twiddles of a thread
   static constexpr int NTW = NT1 * M1 + (R3 > 1 ? (R2 - 1) * R3 : 0);
@@ -53,12 +57,15 @@ template <class T, int NSX> struct FusedCfg {
   // passes' shared-memory latency uncovered (FP32 at 12 warps: 512x512x32
   // 719 -> 885 us).
   static constexpr int CTAS = (sizeof(T) == 4 ? 768 : 384) / THREADS;
-  // offset of r R3 + i within b
-  static __device__ __forceinline__ constexpr int off(int m) { return R3 == 1 ? m : m + m / PB; }
-  // address of element n
-  static __device__ __forceinline__ int at(int n) {
-    const int b = n / M1, m = n - b * M1;
-    return b * SB + off(m);
+  // offset of r R3 + i within b, address of element n
+  static __device__ __forceinline__ constexpr int off(int m) { return R3 == 1 ? m : (m / R3) * SR + m % R3; }
+  static __device__ __forceinline__ int at(int n) { return (n / M1) * SB + off(n % M1); }
+  // element of the pointwise phase's point p: in FP32 four neighbouring b run
+  // fastest (SB = 4 mod 16 8-byte banks), else natural order
+  static __device__ __forceinline__ int elem(int p) {
+    if (!F32 || R3 == 1) return p;
+    const int q = p >> 2, i = q % R3, r = (q / R3) % R2, bh = q / M1;
+    return ((p & 3) + 4 * bh) * M1 + r * R3 + i;
   }
 };
 
@@ -75,8 +82,9 @@ template <class T, int NSX, bool INV> struct RowPasses {
     if constexpr (R3 > 1) {
       static_assert(R2 == 4, "three rounds of M1 threads");
       if (TP > M1 && t >= M1) return;
-      const int i = t % R3;
-      cx<T>* p = buf + (t / R3) * C::SB + (i + i / C::PB);
+      // FP32: b runs fastest
+      const int i = C::F32 ? t / 4 : t % R3;
+      cx<T>* p = buf + (C::F32 ? t % 4 : t / R3) * C::SB + i;
       cx<T> w[R2];
 #pragma unroll
       for (int r = 1; r < R2; r++) w[r] = INV ? conj(tw2[(r - 1) * R3 + i]) : tw2[(r - 1) * R3 + i];
@@ -85,12 +93,12 @@ template <class T, int NSX, bool INV> struct RowPasses {
         cx<T> v[R2];
 #pragma unroll
         for (int r = 0; r < R2; r++) {
-          v[r] = p[4 * jj * C::SB + row_off(r, i)];
+          v[r] = p[4 * jj * C::SB + r * C::SR];
           if (!INV && r > 0) v[r] = cmul(v[r], w[r]);
         }
         Dft<R2, INV ? +1 : -1, T>::run(v);
 #pragma unroll
-        for (int r = 0; r < R2; r++) p[4 * jj * C::SB + row_off(r, i)] = (INV && r > 0) ? cmul(v[r], w[r]) : v[r];
+        for (int r = 0; r < R2; r++) p[4 * jj * C::SB + r * C::SR] = (INV && r > 0) ? cmul(v[r], w[r]) : v[r];
       }
     } else {
       constexpr int J = (12 + TP - 1) / TP;
@@ -108,11 +116,6 @@ template <class T, int NSX, bool INV> struct RowPasses {
       }
     }
   }
-  // off(r R3 + i) - off(i): a constant when PB divides R3 or R3 divides PB
-  static __device__ __forceinline__ int row_off(int r, int i) {
-    if (R3 % C::PB == 0 || C::PB % R3 == 0) return r * R3 + (r * R3) / C::PB;
-    return C::off(r * R3 + i) - C::off(i);
-  }
   static __device__ __forceinline__ void pass3(cx<T>* buf, int t) {
     constexpr int ITEMS = 12 * R2, J = (ITEMS + TP - 1) / TP;
 #pragma unroll
@@ -120,18 +123,14 @@ template <class T, int NSX, bool INV> struct RowPasses {
       const int it = t + TP * jj;
       if (J * TP > ITEMS && it >= ITEMS) break;
       const int b = it / R2, r = it - b * R2;
-      cx<T>* p = buf + b * C::SB + C::off(r * R3);
+      cx<T>* p = buf + b * C::SB + r * C::SR;
       cx<T> v[R3];
 #pragma unroll
-      for (int i = 0; i < R3; i++) v[i] = p[col_off(r, i)];
+      for (int i = 0; i < R3; i++) v[i] = p[i];
       Dft<R3, INV ? +1 : -1, T>::run(v);
 #pragma unroll
-      for (int i = 0; i < R3; i++) p[col_off(r, i)] = v[i];
+      for (int i = 0; i < R3; i++) p[i] = v[i];
     }
-  }
-  static __device__ __forceinline__ int col_off(int r, int i) {
-    if (R3 % C::PB == 0 || C::PB % R3 == 0) return i + i / C::PB;
-    return C::off(r * R3 + i) - C::off(r * R3);
   }
 };
 
@@ -332,7 +331,7 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
       for (int q = 0; q < PPT; q++) {
         const int n = tr + TR * q;
         if (PPT * TR > MX && n >= MX) break;
-        const cx<T>* p = rowbuf + C::at(n);
+        const cx<T>* p = rowbuf + C::at(C::elem(n));
         const cx<T> uv = p[0], we = p[BUF];
         U0[q] = uv.x; V0[q] = uv.y; W0[q] = we.x; E0[q] = tmax(we.y, emin);
         if (KEEP) s0[q] = tke_sqrt(E0[q]);
@@ -380,7 +379,7 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
     for (int q = 0; q < PPT; q++) {
       const int n = tr + TR * q;
       if (PPT * TR > MX && n >= MX) break;
-      cx<T>* p = rowbuf + C::at(n);
+      cx<T>* p = rowbuf + C::at(C::elem(n));
       // learned: buffer 2 holds (ux, vy); the other gradients are not needed
       const cx<T> d2 = p[2 * BUF];
       const cx<T> d3 = learned ? mk((T)0, d2.y) : p[3 * BUF];
@@ -400,7 +399,7 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
         const cx<T> wxy = learned ? zero_cx<T>() : p[4 * BUF];
         cx<T> exy = p[5 * BUF];
         if (clip) {
-          const size_t o = ((size_t)(le - 1) * MY + y) * MX + C::x_of(n);
+          const size_t o = ((size_t)(le - 1) * MY + y) * MX + C::x_of(C::elem(n));
           if (clipx) exy.x += reinterpret_cast<const T*>(f.dEX)[o];
           exy.y += reinterpret_cast<const T*>(f.dEY)[o];
         }
