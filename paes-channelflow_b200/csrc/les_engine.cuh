@@ -55,7 +55,7 @@ extern thread_local KernelTrace* g_trace;
 template <class... KArgs, class... Args>
 inline void launch(void (*k)(KArgs...), dim3 g, dim3 b, size_t smem, cudaStream_t s, Args... args) {
   if (g.x == 0 || g.y == 0 || g.z == 0) return;
-  // 48 KB without the attribute, static shared memory (at most 12 KB) included
+  // 48 KB without the attribute, static shared memory (at most 12 KB here) included
   if (smem > 36 * 1024) set_smem_limit((const void*)k, smem);
   k<<<g, b, smem, s>>>(args...);
   cudaError_t e = cudaGetLastError();
@@ -519,15 +519,12 @@ struct Engine : EngineBase {
     });
     with_small(NY, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
-      using C = ColCfg<N, T>;
-      launch(k_col_small<T, N, false>, dim3(cdiv(KX, C::TC), NZ - 1), dim3(C::THREADS), C::buf(), st,
-             (const cx<T>*)Xe.p, Xe.p, KX, (T)(1.0 / ((double)NX * NY)), tw);
       using CM = ColPlan<T, 3 * N / 2>;
       Ptr8 src{}, dst{};
       src.p[0] = uh.p; src.p[1] = vh.p; src.p[2] = wh.p; src.p[3] = Xe.p;
       for (int i = 0; i < 8; i++) dst.p[i] = mixed[i].p;
       launch(k_y_inverse<T, N>, dim3(cdiv(KX, CM::TC), NZ, 4), dim3(CM::THREADS), CM::smem(), st, src, dst,
-             KX, NZ, (T)ky0, tw, yinv_maps, yinv_pdist);
+             KX, NZ, (T)ky0, (T)(1.0 / ((double)NX * NY)), tw, yinv_maps, yinv_pdist);
     });
     if (fused) {
       fused_middle(a);
@@ -908,6 +905,7 @@ struct Engine : EngineBase {
     const int L = (int)cdiv(NZ, 512 / MODES);  // levels of a chunk
     const int threads = (int)cdiv((size_t)MODES * cdiv(NZ, L), 32) * 32;
     const size_t smem = (size_t)L * threads * (sizeof(cx<double>) + sizeof(double));
+    set_smem_limit((const void*)k_press<T, MODES, RHS, UPD>, smem);  // its static tables take up to 24 KB more
     launch(k_press<T, MODES, RHS, UPD>, dim3((unsigned)(nm / MODES)), dim3((unsigned)threads), smem, st, uh.p, vh.p, wh.p,
            ruo.p, rvo.p, rwo.p, (const cx<T>*)run.p, (const cx<T>*)rvn.p, (const cx<T>*)rwn.p, ph.p, mu.p, mv.p, mru.p,
            mrv.p, a, L, err.p);

@@ -201,27 +201,23 @@ static int op_guard(F&& fn) {
 }
 
 
-// Scratch of the expand / compress / deal entry points: stream-ordered
-// allocations released on the same stream.
-template <class T>
-static void with_scratch(size_t n1, size_t n2, cudaStream_t s, const std::function<void(cx<T>*, cx<T>*)>& fn) {
-  void* a = nullptr;
-  void* b = nullptr;
-  LES_CUDA(cudaMallocAsync(&a, std::max<size_t>(n1, 1) * sizeof(cx<T>), s));
-  cudaError_t e2 = cudaMallocAsync(&b, std::max<size_t>(n2, 1) * sizeof(cx<T>), s);
-  if (e2 != cudaSuccess) {
-    cudaFreeAsync(a, s);
-    throw CudaError("cudaMallocAsync", LES_ENOMEM);
+// Scratch of the expand / compress / deal entry points: n1 and n2 complex
+// values (null for 0) in one stream-ordered allocation, released on the same
+// stream.
+template <class T, class F> static void with_scratch(size_t n1, size_t n2, cudaStream_t s, F&& fn) {
+  if (n1 + n2 == 0) {
+    fn((cx<T>*)nullptr, (cx<T>*)nullptr);
+    return;
   }
+  cx<T>* a = nullptr;
+  LES_CUDA(cudaMallocAsync((void**)&a, (n1 + n2) * sizeof(cx<T>), s));
   try {
-    fn((cx<T>*)a, (cx<T>*)b);
+    fn(n1 ? a : (cx<T>*)nullptr, n2 ? a + n1 : (cx<T>*)nullptr);
   } catch (...) {
     cudaFreeAsync(a, s);
-    cudaFreeAsync(b, s);
     throw;
   }
   LES_CUDA(cudaFreeAsync(a, s));
-  LES_CUDA(cudaFreeAsync(b, s));
 }
 
 
@@ -450,13 +446,18 @@ int les_op_expand(const void* xs, void* xl, int nx, int ny, int howmany, int rea
     return LES_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   size_t n1 = (size_t)howmany * ny * (nx / 2), n2 = (size_t)howmany * (3 * ny / 2) * (nx / 2);
+  // the spectral rows fit in the output unless it overlaps the input or is
+  // not aligned to a complex value
+  const size_t ns = (size_t)howmany * nx * ny * real_bytes;
+  const bool apart = (const char*)xl + ns / 4 * 9 <= (const char*)xs || (const char*)xs + ns <= (const char*)xl;
+  const bool direct = apart && (uintptr_t)xl % (2 * real_bytes) == 0;
   return op_guard([&] {
     if (real_bytes == 8)
-      with_scratch<double>(n1, n2, s, [&](cx<double>* a, cx<double>* b) {
+      with_scratch<double>(direct ? 0 : n1, direct ? 0 : n2, s, [&](cx<double>* a, cx<double>* b) {
         op_expand<double>((const double*)xs, (double*)xl, nx, ny, howmany, s, a, b);
       });
     else
-      with_scratch<float>(n1, n2, s, [&](cx<float>* a, cx<float>* b) {
+      with_scratch<float>(direct ? 0 : n1, direct ? 0 : n2, s, [&](cx<float>* a, cx<float>* b) {
         op_expand<float>((const float*)xs, (float*)xl, nx, ny, howmany, s, a, b);
       });
   });
@@ -466,13 +467,14 @@ int les_op_compress(const void* xl, void* xs, int nx, int ny, int howmany, int r
     return LES_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   size_t n1 = (size_t)howmany * ny * (nx / 2), n2 = (size_t)howmany * (3 * ny / 2) * (nx / 2);
+  const bool direct = (uintptr_t)xs % (2 * real_bytes) == 0;  // the input is read before the output is written
   return op_guard([&] {
     if (real_bytes == 8)
-      with_scratch<double>(n1, n2, s, [&](cx<double>* a, cx<double>* b) {
+      with_scratch<double>(direct ? 0 : n1, n2, s, [&](cx<double>* a, cx<double>* b) {
         op_compress<double>((const double*)xl, (double*)xs, nx, ny, howmany, s, a, b);
       });
     else
-      with_scratch<float>(n1, n2, s, [&](cx<float>* a, cx<float>* b) {
+      with_scratch<float>(direct ? 0 : n1, n2, s, [&](cx<float>* a, cx<float>* b) {
         op_compress<float>((const float*)xl, (float*)xs, nx, ny, howmany, s, a, b);
       });
   });
@@ -480,12 +482,12 @@ int les_op_compress(const void* xl, void* xs, int nx, int ny, int howmany, int r
 int les_op_deal(void* x, int nx, int ny, int howmany, int real_bytes, void* stream) {
   if (!x || howmany <= 0 || check_rb(real_bytes) || !supported_small(nx) || !supported_small(ny)) return LES_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
-  size_t n1 = (size_t)howmany * ny * (nx / 2);
+  const size_t n1 = (uintptr_t)x % (2 * real_bytes) == 0 ? 0 : (size_t)howmany * ny * (nx / 2);
   return op_guard([&] {
     if (real_bytes == 8)
-      with_scratch<double>(n1, 1, s, [&](cx<double>* a, cx<double>*) { op_deal<double>((double*)x, nx, ny, howmany, s, a); });
+      with_scratch<double>(n1, 0, s, [&](cx<double>* a, cx<double>*) { op_deal<double>((double*)x, nx, ny, howmany, s, a); });
     else
-      with_scratch<float>(n1, 1, s, [&](cx<float>* a, cx<float>*) { op_deal<float>((float*)x, nx, ny, howmany, s, a); });
+      with_scratch<float>(n1, 0, s, [&](cx<float>* a, cx<float>*) { op_deal<float>((float*)x, nx, ny, howmany, s, a); });
   });
 }
 int les_op_tridv(void* bdar, int ny, int n, int real_bytes, void* stream) {

@@ -147,6 +147,69 @@ k_row_c2r(const cx<T>* __restrict__ in, T* __restrict__ out, int nrows, int KIN,
   });
 }
 
+// Where an operator keeps the x-spectral rows of its planes: row r of plane p
+// at p ps + r rs complex values (rows per plane: ny).
+struct RowLayout {
+  int ny;
+  long long rs, ps;
+  __device__ __forceinline__ long long at(int row) const { return (long long)(row / ny) * ps + (long long)(row % ny) * rs; }
+};
+
+// k_row_r2c and k_row_c2r with the spectral rows in a given layout, which may
+// lie inside the real rows' own buffer (row r's modes at the start of row r):
+// a block reads its rows before it writes them, and no other block touches
+// them.  So expand and deal need no scratch.
+template <class T, int N>
+__global__ void __launch_bounds__(RowCfg<N>::THREADS)
+k_op_row_r2c(const T* in, cx<T>* out, int nrows, int K, RowLayout lo, const cx<T>* __restrict__ tw) {
+  using C = RowCfg<N>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
+  const int p0 = blockIdx.x * C::NT, npair = (nrows + 1) / 2;
+  fft_core<N, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
+    const int p = p0 + t;
+    if (p >= npair) return zero_cx<T>();
+    return mk(in[(size_t)(2 * p) * N + n], (2 * p + 1 < nrows) ? in[(size_t)(2 * p + 1) * N + n] : (T)0);
+  }, NoStore{});
+  for (int i = threadIdx.x; i < C::NT * K; i += blockDim.x) {
+    const int t = i / K, k = i - t * K, p = p0 + t;
+    if (p >= npair) continue;
+    const cx<T> zk = sm[t * N + k], zm = conj(sm[t * N + (N - k) % N]);
+    const cx<T> d = zk - zm;
+    out[lo.at(2 * p) + k] = (zk + zm) * (T)0.5;
+    if (2 * p + 1 < nrows) out[lo.at(2 * p + 1) + k] = mk(d.y * (T)0.5, -d.x * (T)0.5);
+  }
+}
+template <class T, int N>
+__global__ void __launch_bounds__(RowCfg<N>::THREADS)
+k_op_row_c2r(const cx<T>* in, T* out, int nrows, int K, RowLayout li, const cx<T>* __restrict__ tw) {
+  using C = RowCfg<N>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
+  const int p0 = blockIdx.x * C::NT, npair = (nrows + 1) / 2;
+  const int row = 2 * (p0 + (int)(threadIdx.x / Split<N>::N2));  // of the transform this thread loads
+  const long long ra = row < nrows ? li.at(row) : 0, rb = row + 1 < nrows ? li.at(row + 1) : 0;
+  fft_core<N, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
+    const int p = p0 + t;
+    int k = n;
+    bool mir = false;
+    if (k >= K) {
+      if (N - k < K && N - k > 0) { k = N - k; mir = true; }
+      else k = -1;
+    }
+    if (p >= npair || k < 0) return zero_cx<T>();
+    cx<T> a = in[ra + k], b = (2 * p + 1 < nrows) ? in[rb + k] : zero_cx<T>();
+    if (k == 0) { a.y = 0; b.y = 0; }
+    if (mir) { a = conj(a); b = conj(b); }
+    return mk(a.x - b.y, a.y + b.x);
+  }, [&](int t, int n, cx<T> v) {
+    const int p = p0 + t;
+    if (p >= npair) return;
+    out[(size_t)(2 * p) * N + n] = v.x;
+    if (2 * p + 1 < nrows) out[(size_t)(2 * p + 1) * N + n] = v.y;
+  });
+}
+
 // Columns of x-spectral planes [plane][N][KX] (KX columns) -> forward DFT
 // along y, times `scale`, Nyquist row N/2 dropped (deal semantics).
 // With INV = true: inverse DFT, no scaling.
@@ -168,59 +231,6 @@ k_col_small(const cx<T>* __restrict__ in, cx<T>* __restrict__ out, int KX, T sca
     if (kx >= KX) return;
     if (!INV) v = (DROP && k == N / 2) ? zero_cx<T>() : v * scale;
     out[plane + (size_t)k * KX + kx] = v;
-  });
-}
-
-// Padding / truncation between the small (N) and padded (M = 3N/2) y-grid,
-// on x-spectral columns.
-//   PAD:   small spectrum column (N) -> inverse DFT of the zero-padded
-//          column (M) [expand]
-//   TRUNC: padded column (M) -> forward DFT, keep |ky| < N/2, times scale,
-//          inverse DFT of the small column (N) [compress]
-template <class T, int NS>
-__global__ void __launch_bounds__(ColCfg<3 * NS / 2, T>::THREADS)
-k_col_pad(const cx<T>* __restrict__ in, cx<T>* __restrict__ out, int KX, const cx<T>* __restrict__ tw) {
-  constexpr int M = 3 * NS / 2;
-  using C = ColCfg<M, T>;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  const int kx0 = blockIdx.x * C::TC;
-  const cx<T>* src = in + (size_t)blockIdx.y * NS * KX;
-  cx<T>* dst = out + (size_t)blockIdx.y * M * KX;
-  fft_core<M, +1, true, false, false>(C::TC, sm, tw, [&](int t, int n) {
-    int kx = kx0 + t;
-    int ky = (n < NS / 2) ? n : ((n > NS) ? n - NS / 2 : -1);
-    return (kx < KX && ky >= 0) ? src[(size_t)ky * KX + kx] : zero_cx<T>();
-  }, [&](int t, int n, cx<T> v) {
-    int kx = kx0 + t;
-    if (kx < KX) dst[(size_t)n * KX + kx] = v;
-  });
-}
-
-template <class T, int NS>
-__global__ void __launch_bounds__(ColCfg<3 * NS / 2, T>::THREADS)
-k_col_trunc(const cx<T>* __restrict__ in, cx<T>* __restrict__ out, int KX, T scale, const cx<T>* __restrict__ tw) {
-  constexpr int M = 3 * NS / 2;
-  using C = ColCfg<M, T>;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  cx<T>* sm2 = sm + C::TC * M;
-  const int kx0 = blockIdx.x * C::TC;
-  const cx<T>* src = in + (size_t)blockIdx.y * M * KX;
-  cx<T>* dst = out + (size_t)blockIdx.y * NS * KX;
-  fft_core<M, -1, true, false, true>(C::TC, sm, tw, [&](int t, int n) {
-    int kx = kx0 + t;
-    return (kx < KX) ? src[(size_t)n * KX + kx] : zero_cx<T>();
-  }, NoStore{});
-  for (int i = threadIdx.x; i < C::TC * NS; i += blockDim.x) {
-    int t = i % C::TC, ky = i / C::TC;
-    int n = (ky < NS / 2) ? ky : ky + NS / 2;
-    sm2[ky * C::TC + t] = (ky == NS / 2) ? zero_cx<T>() : sm[n * C::TC + t] * scale;
-  }
-  __syncthreads();
-  fft_core<NS, +1, true, true, false>(C::TC, sm2, tw, NoLoad{}, [&](int t, int n, cx<T> v) {
-    int kx = kx0 + t;
-    if (kx < KX) dst[(size_t)n * KX + kx] = v;
   });
 }
 
@@ -353,27 +363,63 @@ template <class T, int M> struct ColPlan {
       }
     }
   }
-  // first pass of a forward transform of the padded rows load(row)
-  template <class LoadF> static __device__ __forceinline__ void first(cx<T>* buf, int q, LoadF load) {
-    constexpr int R = R3 > 1 ? R3 : R2, ITEMS = R3 > 1 ? 12 * R2 : 12;
+  // first pass of a forward transform of NB blocks, rows load(row)
+  template <int NB, class LoadF> static __device__ __forceinline__ void first(cx<T>* buf, int q, LoadF load) {
+    constexpr int R = R3 > 1 ? R3 : R2, ITEMS = R3 > 1 ? NB * R2 : NB;
 #pragma unroll
     for (int it = 0; it < (ITEMS + M1 - 1) / M1; it++) {
       const int u = q + it * M1;
       if (ITEMS % M1 != 0 && u >= ITEMS) break;
       const int b = R3 > 1 ? u / R2 : u, r = R3 > 1 ? u % R2 : 0;
       cx<T>* p = buf + (size_t)(b * SB + r * SR) * TC;
-      const int x0 = P::x_of(b * M1 + r * R3);
+      const int x0 = NB == 12 ? P::x_of(b * M1 + r * R3) : b + NB * r;
       cx<T> v[R];
 #pragma unroll
       for (int i = 0; i < R; i++) {
-        int x = x0 + 12 * (R3 > 1 ? R2 : 1) * i;
-        if (P::PFA) x = x >= M ? x - M : x;
+        int x = x0 + NB * (R3 > 1 ? R2 : 1) * i;
+        if (NB == 12 && P::PFA) x = x >= M ? x - M : x;
         v[i] = load(x);
       }
       Dft<R, -1, T>::run(v);
 #pragma unroll
       for (int i = 0; i < R; i++) p[i * TC] = v[i];
     }
+  }
+  // Forward transform of length NS of the rows load(row): thread j ends with
+  // the modes ky = j + M1 m, m = 0..7, times scale, Nyquist removed.  One or
+  // two barriers; the caller may then write the elements (b, j) without one.
+  template <class LoadF>
+  static __device__ __forceinline__ void forward_small(cx<T>* buf, const cx<T>* tw, const cx<T> (&w2)[4], int j, T scale,
+                                                       LoadF load, cx<T> (&R)[8]) {
+    first<8>(buf, j, load);
+    __syncthreads();
+    if constexpr (R3 > 1) {
+      pass2<8, false>(buf, w2, j);
+      __syncthreads();
+    }
+    const cx<T>* g = tw + tw_off(NS);
+    const cx<T>* p = buf + off(j) * TC;
+#pragma unroll
+    for (int b = 0; b < 8; b++) R[b] = b ? cmul(p[b * SB * TC], g[b * j]) : p[0];
+    Dft<8, -1, T>::run(R);
+#pragma unroll
+    for (int m = 0; m < 8; m++) R[m] = (m == 4 && j == 0) ? zero_cx<T>() : R[m] * scale;
+  }
+  // Inverse of it: the modes in registers to rows store(row, value).
+  template <class StoreF>
+  static __device__ __forceinline__ void inverse_small(cx<T>* buf, const cx<T>* tw, const cx<T> (&w2)[4], int j,
+                                                       cx<T> (&R)[8], StoreF store) {
+    Dft<8, +1, T>::run(R);
+    const cx<T>* g = tw + tw_off(NS);
+    cx<T>* p = buf + off(j) * TC;
+#pragma unroll
+    for (int b = 0; b < 8; b++) p[b * SB * TC] = b ? cmul(R[b], conj(g[b * j])) : R[b];
+    __syncthreads();
+    if constexpr (R3 > 1) {
+      pass2<8, true>(buf, w2, j);
+      __syncthreads();
+    }
+    last<8>(buf, j, store);
   }
 };
 
@@ -390,15 +436,50 @@ template <class T, int M> struct ColTw1 {
   static __device__ __forceinline__ bool one(int b) { return InPlace<M>::PFA ? (b & 3) == 0 : b == 0; }
 };
 
+// Pass 1 of the padded inverse transform of thread j's modes x (ky = j + M1 m)
+// into a tile.
+template <class T, int M>
+__device__ __forceinline__ void col_pad_pass1(cx<T>* buf, int j, const cx<T> (&x)[8], const ColTw1<T, M>& tw1,
+                                              const cx<T> (&w3)[3]) {
+  using C = ColPlan<T, M>;
+  cx<T> v[12];
+  if constexpr (InPlace<M>::PFA) Dft12Pfa<T, C::M1>::padded(x, w3, v);
+  else dft12_padded<T>(x, v);
+  cx<T>* p = buf + C::off(j) * C::TC;
+#pragma unroll
+  for (int b = 0; b < 12; b++) p[b * C::SB * C::TC] = ColTw1<T, M>::one(b) ? v[b] : cmul(v[b], conj(tw1.of(b)));
+}
+// Last pass of the padded forward transform: thread j's kept modes.
+template <class T, int M>
+__device__ __forceinline__ void col_trunc_pass1(const cx<T>* buf, int j, const ColTw1<T, M>& tw1, const cx<T> (&w3)[3],
+                                                cx<T> (&o)[8]) {
+  using C = ColPlan<T, M>;
+  const cx<T>* p = buf + C::off(j) * C::TC;
+  cx<T> v[12];
+#pragma unroll
+  for (int b = 0; b < 12; b++)
+    v[b] = ColTw1<T, M>::one(b) ? p[b * C::SB * C::TC] : cmul(p[b * C::SB * C::TC], tw1.of(b));
+  if constexpr (InPlace<M>::PFA) Dft12Pfa<T, C::M1>::forward(v, w3, o);
+  else {
+    cx<T> y[12];
+    dft12_forward<T>(v, y);
+#pragma unroll
+    for (int m = 0; m < 4; m++) { o[m] = y[m]; o[4 + m] = y[8 + m]; }
+  }
+}
+
 // expand() of u, v, w, e in y fused with d/dy: for field f = blockIdx.z
 // (u, v, w, e), out[2f] = IFFT_M(pad(s)) and out[2f+1] = IFFT_M(i*ky*pad(s)),
 // TC columns per block, both from one load of the columns (8 values a
-// thread).  Thread 0 first has the TMA prefetch into L2 the columns of the
+// thread).  u, v, w come as spectra; e as the x-spectral rows of k_e_prep,
+// whose y transform (times `scale`) is the block's first step: it ends with
+// the modes in the registers where the others are loaded.  Thread 0 first has the TMA prefetch into L2 the columns of the
 // block `pdist` blocks ahead (les_tma.cuh; maps: tensor maps of src[0..3] as
 // [NZ*NS][KX] rows; pdist 0 prefetches nothing).
 template <class T, int NS>
 __global__ void __launch_bounds__(ColPlan<T, 3 * NS / 2>::THREADS, ColPlan<T, 3 * NS / 2>::CTAS)
-k_y_inverse(const __grid_constant__ Ptr8 src, const __grid_constant__ Ptr8 dst, int KX, int NZ, T ky0, const cx<T>* __restrict__ tw,
+k_y_inverse(const __grid_constant__ Ptr8 src, const __grid_constant__ Ptr8 dst, int KX, int NZ, T ky0, T scale,
+            const cx<T>* __restrict__ tw,
             const __grid_constant__ ColMaps maps, unsigned pdist) {
   constexpr int M = 3 * NS / 2;
   using C = ColPlan<T, M>;
@@ -416,24 +497,22 @@ k_y_inverse(const __grid_constant__ Ptr8 src, const __grid_constant__ Ptr8 dst, 
   cx<T>* buf = reinterpret_cast<cx<T>*>(smraw) + t;
   const cx<T>* s = reinterpret_cast<const cx<T>*>(src.p[f]) + (size_t)(z - 1) * NS * KX + (in ? kx : 0);
   cx<T> x[8], w2[4];
+  if (f < 3) {
 #pragma unroll
-  for (int m = 0; m < 8; m++) x[m] = (m == 4 && j == 0) ? zero_cx<T>() : s[(j + M1 * m) * KX];  // no Nyquist mode
+    for (int m = 0; m < 8; m++) x[m] = (m == 4 && j == 0) ? zero_cx<T>() : s[(j + M1 * m) * KX];  // no Nyquist mode
+  }
   const ColTw1<T, M> tw1(tw, j);
   C::twiddles2(tw, j, w2);
   cx<T> w3[3];
   InPlace<M>::rotations(j, w3);
+  if (f == 3) C::forward_small(buf, tw, w2, j, scale, [&](int row) { return s[row * KX]; }, x);
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    cx<T> v[12];
     if (h) {
 #pragma unroll
       for (int m = 0; m < 8; m++) x[m] = mul_i(x[m]) * (ky0 * (T)(m < 4 ? j + M1 * m : j + M1 * m - NS));
     }
-    if constexpr (InPlace<M>::PFA) Dft12Pfa<T, M1>::padded(x, w3, v);
-    else dft12_padded<T>(x, v);
-    cx<T>* p = buf + h * C::BUF + C::off(j) * TC;
-#pragma unroll
-    for (int b = 0; b < 12; b++) p[b * C::SB * TC] = ColTw1<T, M>::one(b) ? v[b] : cmul(v[b], conj(tw1.of(b)));
+    col_pad_pass1<T, M>(buf + h * C::BUF, j, x, tw1, w3);
   }
   __syncthreads();
   if constexpr (C::R3 > 1) {
@@ -983,7 +1062,7 @@ k_y_forward(const __grid_constant__ Ptr8 X, const __grid_constant__ Ptr8 rnew, i
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     const cx<T>* s = reinterpret_cast<const cx<T>*>(X.p[2 * f + h]) + (size_t)(z - 1) * M * KX + (in ? kx : 0);
-    C::first(buf + h * C::BUF, j, [&](int row) { return s[row * KX]; });
+    C::template first<12>(buf + h * C::BUF, j, [&](int row) { return s[row * KX]; });
   }
   C::twiddles2(tw, j, w2);
   __syncthreads();
@@ -997,17 +1076,8 @@ k_y_forward(const __grid_constant__ Ptr8 X, const __grid_constant__ Ptr8 rnew, i
   InPlace<M>::rotations(j, w3);
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    const cx<T>* p = buf + h * C::BUF + C::off(j) * TC;
-    cx<T> v[12], o[8];
-#pragma unroll
-    for (int b = 0; b < 12; b++) v[b] = ColTw1<T, M>::one(b) ? p[b * C::SB * TC] : cmul(p[b * C::SB * TC], tw1.of(b));
-    if constexpr (InPlace<M>::PFA) Dft12Pfa<T, M1>::forward(v, w3, o);
-    else {
-      cx<T> y[12];
-      dft12_forward<T>(v, y);
-#pragma unroll
-      for (int m = 0; m < 4; m++) { o[m] = y[m]; o[4 + m] = y[8 + m]; }
-    }
+    cx<T> o[8];
+    col_trunc_pass1<T, M>(buf + h * C::BUF, j, tw1, w3, o);
 #pragma unroll
     for (int m = 0; m < 8; m++) {
       if (h == 0) R[m] = o[m];
@@ -1028,23 +1098,68 @@ k_y_forward(const __grid_constant__ Ptr8 X, const __grid_constant__ Ptr8 rnew, i
       if (in) dst[(j + M1 * m) * KX] = R[m];
     return;
   }
-  // e: inverse transform of length NS = 8 M1 in the first tile (thread j's
-  // pass 1 writes the elements it has just read)
-  Dft<8, +1, T>::run(R);
-  {
-    const cx<T>* g = tw + tw_off(NS);
-    cx<T>* p = buf + C::off(j) * TC;
-#pragma unroll
-    for (int b = 0; b < 8; b++) p[b * C::SB * TC] = b ? cmul(R[b], conj(g[b * j])) : R[b];
-  }
-  __syncthreads();
-  if constexpr (C::R3 > 1) {
-    C::template pass2<8, true>(buf, w2, j);
-    __syncthreads();
-  }
-  C::template last<8>(buf, j, [&](int row, cx<T> v) {
+  // e: inverse transform of length NS in the first tile (thread j writes the
+  // elements it has just read)
+  C::inverse_small(buf, tw, w2, j, R, [&](int row, cx<T> v) {
     if (in) dst[row * KX] = v;
   });
+}
+
+// Columns of the operator entry points (x-spectral planes, one per
+// blockIdx.y), TC columns per block: forward y transform of length NS (times
+// `scale`, Nyquist dropped) or of the padded rows cut to the kept modes
+// (FROM_PAD), then the inverse transform back, padded (TO_PAD) or not, without
+// leaving the block: expand, compress and deal in one column kernel each (src
+// may be dst: a block reads its columns before it writes them).
+template <class T, int NS, bool FROM_PAD, bool TO_PAD>
+__global__ void __launch_bounds__(ColPlan<T, 3 * NS / 2>::THREADS, ColPlan<T, 3 * NS / 2>::CTAS)
+k_col_resize(const cx<T>* src, cx<T>* dst, int KX, RowLayout ls, RowLayout ld, T scale, const cx<T>* __restrict__ tw) {
+  constexpr int M = 3 * NS / 2;
+  using C = ColPlan<T, M>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int t = threadIdx.x % C::TC, j = threadIdx.x / C::TC;
+  const int kx = blockIdx.x * C::TC + t;
+  const bool in = kx < KX;
+  cx<T>* buf = reinterpret_cast<cx<T>*>(smraw) + t;
+  src += blockIdx.y * ls.ps + (in ? kx : 0);
+  dst += blockIdx.y * ld.ps + kx;
+  const int rs = (int)ls.rs, rd = (int)ld.rs;
+  auto load = [&](int row) { return src[row * rs]; };
+  auto store = [&](int row, cx<T> v) {
+    if (in) dst[row * rd] = v;
+  };
+  cx<T> w2[4], R[8];
+  C::twiddles2(tw, j, w2);
+  if constexpr (FROM_PAD) {
+    C::template first<12>(buf, j, load);
+    __syncthreads();
+    if constexpr (C::R3 > 1) {
+      C::template pass2<12, false>(buf, w2, j);
+      __syncthreads();
+    }
+    const ColTw1<T, M> tw1(tw, j);
+    cx<T> w3[3];
+    InPlace<M>::rotations(j, w3);
+    col_trunc_pass1<T, M>(buf, j, tw1, w3, R);
+#pragma unroll
+    for (int m = 0; m < 8; m++) R[m] = (m == 4 && j == 0) ? zero_cx<T>() : R[m] * scale;
+  } else {
+    C::forward_small(buf, tw, w2, j, scale, load, R);
+  }
+  if constexpr (TO_PAD) {
+    const ColTw1<T, M> tw1(tw, j);
+    cx<T> w3[3];
+    InPlace<M>::rotations(j, w3);
+    col_pad_pass1<T, M>(buf, j, R, tw1, w3);
+    __syncthreads();
+    if constexpr (C::R3 > 1) {
+      C::template pass2<12, true>(buf, w2, j);
+      __syncthreads();
+    }
+    C::template last<12>(buf, j, store);
+  } else {
+    C::inverse_small(buf, tw, w2, j, R, store);
+  }
 }
 
 // The stage's e update (comp1.f90:131, comp2.f90:38) with re from its

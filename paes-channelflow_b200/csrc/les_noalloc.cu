@@ -89,31 +89,29 @@ const NoAllocDevice& noalloc_setup(int dev) {
   return g_noalloc_dev.emplace(dev, d).first->second;
 }
 
-// Same four launches as op_expand, on the static scratch.
+// Same three launches as op_expand, on the static scratch.
 template <class T>
 void expand_static(const T* in, T* out, int nx, int ny, int howmany, cudaStream_t s, const cx<T>* tw, cx<T>* t1,
                    cx<T>* t2) {
   const int KX = nx / 2, MY = 3 * ny / 2;
+  const RowLayout l1{ny, KX, (long long)ny * KX}, l2{MY, KX, (long long)MY * KX};
   with_small(nx, [&](auto cn) {
     constexpr int N = decltype(cn)::value;
     using C = RowCfg<N>;
-    launch(k_row_r2c<T, N>, dim3(cdiv(howmany * ny / 2 + 1, C::NT)), dim3(C::THREADS), C::template smem<T>(), s, in,
-           t1, howmany * ny, KX, tw);
+    launch(k_op_row_r2c<T, N>, dim3(cdiv((howmany * ny + 1) / 2, C::NT)), dim3(C::THREADS), C::template smem<T>(), s, in, t1,
+           howmany * ny, KX, l1, tw);
   });
   with_small(ny, [&](auto cn) {
     constexpr int N = decltype(cn)::value;
-    using C = ColCfg<N, T>;
-    launch(k_col_small<T, N, false>, dim3(cdiv(KX, C::TC), howmany), dim3(C::THREADS), C::buf(), s,
-           (const cx<T>*)t1, t1, KX, (T)(1.0 / ((double)nx * ny)), tw);
-    using CM = ColCfg<3 * N / 2, T>;
-    launch(k_col_pad<T, N>, dim3(cdiv(KX, CM::TC), howmany), dim3(CM::THREADS), CM::buf(), s, (const cx<T>*)t1, t2,
-           KX, tw);
+    using C = ColPlan<T, 3 * N / 2>;
+    launch(k_col_resize<T, N, false, true>, dim3(cdiv(KX, C::TC), howmany), dim3(C::THREADS), C::smem() / 2, s,
+           (const cx<T>*)t1, t2, KX, l1, l2, (T)(1.0 / ((double)nx * ny)), tw);
   });
   with_small(nx, [&](auto cn) {
-    constexpr int N = decltype(cn)::value;
-    using C = RowCfg<3 * N / 2>;
-    launch(k_row_c2r<T, 3 * N / 2>, dim3(cdiv(howmany * MY / 2 + 1, C::NT)), dim3(C::THREADS),
-           C::template smem<T>(), s, (const cx<T>*)t2, out, howmany * MY, KX, tw);
+    constexpr int N = 3 * decltype(cn)::value / 2;
+    using C = RowCfg<N>;
+    launch(k_op_row_c2r<T, N>, dim3(cdiv((howmany * MY + 1) / 2, C::NT)), dim3(C::THREADS), C::template smem<T>(), s,
+           (const cx<T>*)t2, out, howmany * MY, KX, l2, tw);
   });
 }
 

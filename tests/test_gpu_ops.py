@@ -71,3 +71,38 @@ def test_fma_probe_rates(gpu_lib, product):
     f64 = product.fma_rate(8)
     assert f32 > 1e12 and f64 > 1e12
     assert f32 > f64
+
+
+@pytest.mark.parametrize("nx,ny,planes", [(16, 16, 1), (64, 96, 3), (192, 32, 2)])
+def test_operators_in_unaligned_and_overlapping_buffers(gpu_lib, product, nx, ny, planes):
+    """The spectral rows of expand, compress and deal live in the output where
+    its alignment and the input allow it, in scratch otherwise: both give the
+    same bits."""
+    import torch
+    lib = product.lib()
+    for dt in (torch.float64, torch.float32):
+        rb = torch.empty(0, dtype=dt).element_size()
+        a = torch.randn((planes, ny, nx), dtype=dt, device="cuda")
+        b = torch.randn((planes, 3 * ny // 2, 3 * nx // 2), dtype=dt, device="cuda")
+        e, c, d = product.expand(a), product.compress(b), product.deal(a)
+        s = torch.cuda.current_stream().cuda_stream
+
+        def shifted(t):  # a view one real past an aligned address
+            return torch.empty(t.numel() + 1, dtype=dt, device="cuda")[1:].view(t.shape)
+
+        out = shifted(e)
+        assert lib.les_op_expand(a.data_ptr(), out.data_ptr(), nx, ny, planes, rb, s) == 0
+        assert torch.equal(out, e)
+        out = shifted(c)
+        assert lib.les_op_compress(b.data_ptr(), out.data_ptr(), nx, ny, planes, rb, s) == 0
+        assert torch.equal(out, c)
+        out = shifted(a)
+        out.copy_(a)
+        assert lib.les_op_deal(out.data_ptr(), nx, ny, planes, rb, s) == 0
+        assert torch.equal(out, d)
+        # the input at the head, and at the tail, of the output
+        for at in (0, e.numel() - a.numel()):
+            buf = torch.zeros(e.numel(), dtype=dt, device="cuda")
+            buf[at: at + a.numel()] = a.reshape(-1)
+            assert lib.les_op_expand(buf.data_ptr() + at * rb, buf.data_ptr(), nx, ny, planes, rb, s) == 0
+            assert torch.equal(buf.view(e.shape), e)

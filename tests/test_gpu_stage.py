@@ -298,3 +298,27 @@ def test_pressure_columns_of_every_chunk_length(gpu_lib, product, nz):
     a, b = g.download(), g2.download()
     for k in "uvwep":
         assert relerr(b[k], a[k]) < 1e-12, k
+
+
+@pytest.mark.parametrize("nx,ny,nz,imodel", [(96, 128, 45, 4), (128, 128, 20, 3), (128, 96, 33, 3)])
+def test_pressure_columns_in_wide_blocks(gpu_lib, product, nx, ny, nz, imodel):
+    """Grids with enough columns for the pressure solve's wide blocks, through
+    the whole stage and the six entry points: what the solve and its update
+    write (u, v, w, p and their tendencies), to the tolerances of the stage
+    tests."""
+    o, g, f = make_pair(product, nx, ny, nz, imodel=imodel)
+    g2 = product.LesGpu(g.cfg)
+    g2.upload(f["u"], f["v"], f["w"], f["e"], f["p"])
+    o.stage(0, 1, 1)
+    g.stage(0, True, 1)
+    g2.stage_split(0, True, 1)
+    fo, to_ = o.get_fields(), o.get_tendencies()
+    vscale = np.abs(fo["u"]).max()
+    rscale = max(np.abs(to_[k]).max() for k in ("ru", "rv", "rw"))
+    for h in (g, g2):
+        fg, tg = h.download(), h.download_tendencies()
+        for k in "uvw":
+            assert relerr(fg[k], fo[k], vscale) < 1e-11, k
+        for k in ("ru", "rv", "rw"):
+            assert relerr(tg[k], to_[k], rscale) < 1e-9, k
+        assert relerr(fg["p"], fo["p"]) < 1e-9
