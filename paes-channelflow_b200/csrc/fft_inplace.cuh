@@ -158,4 +158,29 @@ template <int N> struct InPlace {
   }
 };
 
+template <class T> __device__ __forceinline__ cx<T> shfl_cx(unsigned mask, cx<T> v, int src) {
+  return mk(__shfl_sync(mask, v.x, src), __shfl_sync(mask, v.y, src));
+}
+
+// A row's team of TP threads (M1 rounded up to a power of two): thread t's
+// pass 1 index j (M1: none) and the lane of its mirror partner M1 - j.  A
+// team of two warps splits j so that both are in the same warp.
+template <int M1, int TP> __device__ __forceinline__ void mirror_lanes(int t, int lane, int& j, int& partner) {
+  if (TP <= 32) {
+    j = t;
+    partner = (lane & ~(TP - 1)) | (t == 0 || t >= M1 ? t : M1 - t);
+  } else {
+    constexpr int H = M1 / 4;
+    const int l = t & 31;
+    if (t < 32) {
+      j = l < H ? l : (l == H ? 2 * H : l + 2 * H);
+      partner = (l == 0 || l == H || l >= 2 * H) ? l : 2 * H - l;
+    } else {
+      j = l < H ? H + l : l + H + 1;
+      partner = l >= 2 * H ? l : 2 * H - 1 - l;
+    }
+    if (l >= 2 * H) j = M1;
+  }
+}
+
 }  // namespace les

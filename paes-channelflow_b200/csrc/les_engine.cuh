@@ -605,21 +605,22 @@ struct Engine : EngineBase {
   void learned_features_into(void* feat, bool raw) {
     with_small(NY, [&](auto cn) {
       constexpr int NN = decltype(cn)::value;
-      using C = LgyCfg<NN, T>;
-      launch(k_lgrad_y<T, NN>, dim3(2 * cdiv(KX, C::H), NZ, 3), dim3(C::THREADS), C::smem(), st, (const cx<T>*)uh.p,
+      using C = ColPlan<T, 3 * NN / 2>;
+      launch(k_lgrad_y<T, NN>, dim3(cdiv(KX, C::TC), NZ, 3), dim3(C::THREADS), C::smem(), st, (const cx<T>*)uh.p,
              (const cx<T>*)vh.p, (const cx<T>*)wh.p, lgy.p, KX, NZ, (T)ky0, tw);
     });
     const T inv_h = (T)(2.0 / cfg.zl);
     with_small(NX, [&](auto cn) {
       constexpr int NN = decltype(cn)::value;
-      using L = LgxCfg<NN>;
+      using L = LgxCfg<T, NN>;
       const unsigned grid = cdiv((size_t)NZ * NY, L::RB);
+      const int pd = L::CTAS * nsm;
       if (raw)
-        launch(k_lgrad_x<T, NN, true>, dim3(grid), dim3(L::THREADS), L::template smem<T>(), st, (const cx<T>*)lgy.p,
-               feat, mlp, NY, NZ, (T)kx0, (T)dzm, (T)dsl, (T)dz, (T)cfg.zl, inv_h, tw);
+        launch(k_lgrad_x<T, NN, true>, dim3(grid), dim3(L::THREADS), L::smem(), st, (const cx<T>*)lgy.p,
+               feat, mlp, NY, NZ, (T)kx0, (T)dzm, (T)dsl, (T)dz, (T)cfg.zl, inv_h, pd, tw);
       else
-        launch(k_lgrad_x<T, NN, false>, dim3(grid), dim3(L::THREADS), L::template smem<T>(), st, (const cx<T>*)lgy.p,
-               feat, mlp, NY, NZ, (T)kx0, (T)dzm, (T)dsl, (T)dz, (T)cfg.zl, inv_h, tw);
+        launch(k_lgrad_x<T, NN, false>, dim3(grid), dim3(L::THREADS), L::smem(), st, (const cx<T>*)lgy.p,
+               feat, mlp, NY, NZ, (T)kx0, (T)dzm, (T)dsl, (T)dz, (T)cfg.zl, inv_h, pd, tw);
     });
   }
   // raw (unnormalised) features of the current state, f32 [N][16]

@@ -69,10 +69,6 @@ template <class T, int NSX> struct FusedCfg {
   }
 };
 
-template <class T> __device__ __forceinline__ cx<T> shfl_cx(unsigned mask, cx<T> v, int src) {
-  return mk(__shfl_sync(mask, v.x, src), __shfl_sync(mask, v.y, src));
-}
-
 // Passes 2 and 3 of a team's transform in its buffer.  t = thread of the
 // team.  INV: pass 2 then 3; else 3 then 2, with the conjugate twiddles.
 template <class T, int NSX, bool INV> struct RowPasses {
@@ -209,24 +205,8 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
   const int bar = 1 + team;
   const unsigned mask = TP >= 32 ? 0xffffffffu : ((1u << (TP & 31)) - 1u) << (lane & ~(TP - 1));
 
-  // pass 1: this thread's j and the lane of its mirror partner M1 - j.  A
-  // team of two warps splits j so that both are in the same warp.
   int j, partner;
-  if (TP <= 32) {
-    j = t;
-    partner = (lane & ~(TP - 1)) | (t == 0 || t >= M1 ? t : M1 - t);
-  } else {
-    constexpr int H = M1 / 4;
-    const int l = t & 31;
-    if (t < 32) {
-      j = l < H ? l : (l == H ? 2 * H : l + 2 * H);
-      partner = (l == 0 || l == H || l >= 2 * H) ? l : 2 * H - l;
-    } else {
-      j = l < H ? H + l : l + H + 1;
-      partner = l >= 2 * H ? l : 2 * H - 1 - l;
-    }
-    if (l >= 2 * H) j = M1;
-  }
+  mirror_lanes<M1, TP>(t, lane, j, partner);
   const bool act = (TP == M1) || j < M1;
   if (!act) j = 0;
   cx<T>* pj = buf + C::off(j);

@@ -52,53 +52,69 @@
 
 namespace les {
 
-// Blocks of k_lgrad_y: H = ColCfg's column count (64-byte row segments of
-// the spectra), H transforms: the field or its y derivative.
-template <int N, class T> struct LgyCfg {
-  static constexpr int H = ColCfg<N, T>::TC;
-  static constexpr int THREADS = H * Split<N>::N2;
-  static constexpr size_t smem() { return (size_t)H * N * sizeof(cx<T>); }
-};
-
 // y-inverse rows gy[f][z][y][kx], f = 0..5: U, UY, V, VY, W, WY.  A block
-// takes H columns of one component (blockIdx.z: u, v, w) at one level and
-// transforms the field (d = blockIdx.x & 1 = 0) or its y derivative (d = 1);
-// the two blocks of a column group are adjacent in launch order, so the
-// second reads the spectral values from L2.
+// takes the columns of ColPlan (64-byte segments) of one component
+// (blockIdx.z: u, v, w) at one level, loads the modes once and transforms the
+// field and its y derivative in the two tiles.  512x512x64 FP32: 348 us with
+// the two in separate blocks, 172 us so; bound by HBM (0.60 GB, 53% of the copy
+// rate) and load latency.
 template <class T, int N>
-__global__ void __launch_bounds__(LgyCfg<N, T>::THREADS)
+__global__ void __launch_bounds__(ColPlan<T, 3 * N / 2>::THREADS, ColPlan<T, 3 * N / 2>::CTAS)
 k_lgrad_y(const cx<T>* __restrict__ uh, const cx<T>* __restrict__ vh, const cx<T>* __restrict__ wh,
           cx<T>* __restrict__ gy, int KX, int NZ, T ky0, const cx<T>* __restrict__ tw) {
-  constexpr int H = LgyCfg<N, T>::H;
+  using C = ColPlan<T, 3 * N / 2>;
+  constexpr int M1 = C::M1, TC = C::TC;
   extern __shared__ __align__(16) unsigned char smraw[];
-  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  const int z = blockIdx.y + 1;
-  const int c = blockIdx.z, d = blockIdx.x & 1;
-  const int c0 = (blockIdx.x >> 1) * H;
+  const int z = blockIdx.y + 1, c = blockIdx.z;
+  const int t = threadIdx.x % TC, j = threadIdx.x / TC;
+  const int kx = blockIdx.x * TC + t;
+  const bool in = kx < KX, zero = (c == 2 && z == NZ);  // w(nnz) = 0
   const size_t nm = (size_t)N * KX;
-  const cx<T>* src = (c == 0 ? uh : (c == 1 ? vh : wh)) + (size_t)(z - 1) * nm;
-  const bool zero = (c == 2 && z == NZ);  // w(nnz) = 0
-  cx<T>* out = gy + ((size_t)(2 * c + d) * NZ + (z - 1)) * nm;
-  fft_core<N, +1, true, false, false>(H, sm, tw, [&](int t, int n) -> cx<T> {
-    const int kx = c0 + t;
-    if (kx >= KX || n == N / 2 || zero) return zero_cx<T>();
-    const cx<T> v = src[(size_t)n * KX + kx];
-    return d ? mul_i(v) * (ky0 * (T)signed_k(n, N)) : v;
-  }, [&](int t, int k, cx<T> v) {
-    const int kx = c0 + t;
-    if (kx < KX) out[(size_t)k * KX + kx] = v;
-  });
+  cx<T>* buf = reinterpret_cast<cx<T>*>(smraw) + t;
+  const cx<T>* s = (c == 0 ? uh : (c == 1 ? vh : wh)) + (size_t)(z - 1) * nm + (in ? kx : 0);
+  cx<T> x[8], w2[4];
+#pragma unroll
+  for (int m = 0; m < 8; m++) x[m] = (zero || (m == 4 && j == 0)) ? zero_cx<T>() : s[(j + M1 * m) * KX];
+  C::twiddles2(tw, j, w2);
+  const cx<T>* g = tw + tw_off(N);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    cx<T> v[8];
+#pragma unroll
+    for (int m = 0; m < 8; m++) v[m] = h ? mul_i(x[m]) * (ky0 * (T)(m < 4 ? j + M1 * m : j + M1 * m - N)) : x[m];
+    Dft<8, +1, T>::run(v);
+    cx<T>* p = buf + h * C::BUF + C::off(j) * TC;
+#pragma unroll
+    for (int b = 0; b < 8; b++) p[b * C::SB * TC] = b ? cmul(v[b], conj(g[b * j])) : v[b];
+  }
+  __syncthreads();
+  if constexpr (C::R3 > 1) {
+    C::template pass2<8, true>(buf, w2, j);
+    C::template pass2<8, true>(buf + C::BUF, w2, j);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    cx<T>* out = gy + ((size_t)(2 * c + h) * NZ + (z - 1)) * nm + kx;
+    C::template last<8>(buf + h * C::BUF, j, [&](int row, cx<T> v) {
+      if (in) out[row * KX] = v;
+    });
+  }
 }
 
-// Rows per block of k_lgrad_x: five transforms per row, about 256 threads.
-template <int NX> struct LgxCfg {
-  static constexpr int N1 = Split<NX>::N1, N2 = Split<NX>::N2, M12 = N1 > N2 ? N1 : N2;
-  static constexpr int RB = (256 / (5 * M12)) > 0 ? (256 / (5 * M12)) : 1;
-  static constexpr int THREADS = 5 * RB * M12;
-  static constexpr int BUF = smem_fft_elems<NX, false>(5 * RB);
-  // transform buffer + the staged spectra (direct and mirrored combination
-  // of each of the 5*RB transforms at kx < NX/2)
-  template <class T> static constexpr size_t smem() { return (size_t)(BUF + 10 * RB * (NX / 2)) * sizeof(cx<T>); }
+// Blocks of k_lgrad_x: five teams of TP threads per row, one per transform
+// (length NX = 8 M1, 8 values a thread, in place: radix 8, R2, R3), RB rows.
+template <class T, int NX> struct LgxCfg {
+  using P = InPlace<3 * NX / 2>;
+  static constexpr int M1 = P::M1, R2 = P::R2, R3 = P::R3;
+  static constexpr int TP = M1 <= 2 ? 2 : M1 <= 4 ? 4 : M1 <= 8 ? 8 : M1 <= 16 ? 16 : M1 <= 32 ? 32 : 64;
+  static constexpr int RB = TP >= 32 ? 1 : 32 / TP;  // 160 or 320 threads
+  static constexpr int THREADS = 5 * TP * RB;
+  static constexpr int SR = R3 > 1 ? R3 + 1 : 1, SB = R3 > 1 ? R2 * SR : (M1 | 1);
+  static constexpr int BUF = 8 * SB;
+  static constexpr int CTAS = (sizeof(T) == 4 ? 960 : 480) / THREADS;
+  static constexpr size_t smem() { return (size_t)5 * RB * BUF * sizeof(cx<T>); }
+  static __device__ __forceinline__ int off(int m) { return R3 > 1 ? (m / R3) * SR + m % R3 : m; }
 };
 
 // Cap of the wall-distance input z_w / Delta: farther from the wall than
@@ -112,17 +128,31 @@ constexpr float kZwCap = 16.0f;
 // bf16 high part (column 11) and remainder (column 12), zeros in 13..15.
 // x order: (ux, vx, wx, uy, vy, wy, uz, vz, wz) / |G|, min(z_w/Delta,
 // kZwCap), z_w / h.
+// The block's rows are consecutive (level, y) rows, one transform per team:
+// (ux, vx), (wx, uy), (vy, wy), (uz, vz), (wz, 0).  Thread j of a team makes
+// the modes k = j + M1 m, m = 0..3, of A + iB in registers; its partner M1 - j
+// needs their mirror images for its own negative modes (shuffles).  The
+// outputs stay permuted in shared memory (x = b + 8 (r + R2 i)); the feature
+// pass walks them in an order its half-warps read without conflicts.  Thread 0
+// to 5 first prefetch the six rows of the block a resident wave ahead into L2.
+// 512x512x64 FP32 412 -> 375 us, 256x192x99 164 -> 108 us, 384x384x64 343 -> 275
+// us against a two-pass transform with the combinations staged in shared
+// memory; bound by the load/store path (74%) and load latency.
 template <class T, int NX, bool RAW>
-__global__ void __launch_bounds__(LgxCfg<NX>::THREADS)
+__global__ void __launch_bounds__(LgxCfg<T, NX>::THREADS, LgxCfg<T, NX>::CTAS)
 k_lgrad_x(const cx<T>* __restrict__ gy, void* __restrict__ feat, const MlpDev* __restrict__ P, int NY, int NZ,
-          T kx0, T dzm, T delta, T dz, T zl, T inv_h, const cx<T>* __restrict__ tw) {
-  using L = LgxCfg<NX>;
-  constexpr int KX = NX / 2, RB = L::RB;
+          T kx0, T dzm, T delta, T dz, T zl, T inv_h, int pdist, const cx<T>* __restrict__ tw) {
+  using L = LgxCfg<T, NX>;
+  constexpr int KX = NX / 2, RB = L::RB, M1 = L::M1, TP = L::TP, R2 = L::R2, R3 = L::R3;
   extern __shared__ __align__(16) unsigned char smraw[];
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
   const int R = NZ * NY;
   const size_t plane = (size_t)R * KX;
   const int r0 = blockIdx.x * RB;
+  // L2 prefetch of the rows of the block one resident wave ahead (its z - 1
+  // and z + 1 rows were or will be its neighbours' own)
+  if (threadIdx.x < 6 && pdist > 0 && r0 + (pdist + 1) * RB <= R)
+    tma::prefetch_l2(gy + threadIdx.x * plane + (size_t)(r0 + pdist * RB) * KX, RB * KX * (unsigned)sizeof(cx<T>));
   // level (0-based) and y of the block's first row; row r0 + rr is at
   // y0 + rr, carried into the next level past NY - 1 (RB <= NY)
   const int zb = r0 / NY, y0 = r0 - zb * NY;
@@ -131,50 +161,114 @@ k_lgrad_x(const cx<T>* __restrict__ gy, void* __restrict__ feat, const MlpDev* _
     z = zb;
     if (y >= NY) { y -= NY; z++; }
   };
-  // row of field f at level k (1..NZ) and y
-  auto rowp = [&](int f, int k, int y) -> const cx<T>* { return gy + (size_t)f * plane + ((size_t)(k - 1) * NY + y) * KX; };
-  // Stage 1: the spectral combinations a + i b of the five transforms of
-  // each row at kx = 0..KX-1, loaded once (coalesced along kx), kept as the
-  // direct value (position kx) and the conjugate-symmetric one (NX - kx).
-  cx<T>* zd = sm + L::BUF;             // [5*RB][KX]
-  cx<T>* zm = zd + (size_t)5 * RB * KX;  // [5*RB][KX]
-  for (int i = threadIdx.x; i < 5 * RB * KX; i += blockDim.x) {
-    const int t = i / KX, k = i - t * KX;
-    const int rr = t / 5, j = t - 5 * rr;
-    cx<T> d = zero_cx<T>(), m = zero_cx<T>();
-    if (r0 + rr < R) {
-      int z, y;
-      row_zy(rr, z, y);
-      z += 1;
+  const int lane = threadIdx.x & 31;
+  const int tm = threadIdx.x / TP, t = threadIdx.x % TP;  // team: rr = tm / 5, transform tm % 5
+  const int rr0 = tm / 5, f = tm - 5 * rr0;
+  const unsigned mask = TP >= 32 ? 0xffffffffu : ((1u << (TP & 31)) - 1u) << (lane & ~(TP - 1));
+  int j, partner;
+  mirror_lanes<M1, TP>(t, lane, j, partner);
+  const bool act = TP == M1 || j < M1;
+  if (!act) j = 0;
+  cx<T>* buf = sm + (size_t)tm * L::BUF;
+  {
+    cx<T> x[4], mir[4], v[8];
+    int z = 0, y = 0;
+    row_zy(rr0, z, y);
+    z += 1;
+    const bool on = r0 + rr0 < R;
+    if (!on) { z = 1; y = 0; }
+    // modes of field q at level k (1..NZ)
+    auto row = [&](int q, int k) { return gy + (size_t)q * plane + ((size_t)(k - 1) * NY + y) * KX + j; };
+    // field A = sa ga(za1) + sb ga(za0), and B likewise: two rows each, with a
+    // zero factor where there is only one
+    // (ux, vx) one row each times i kx; (wx, uy): W at z and z-1 averaged times
+    // i kx, UY; (vy, wy): VY, WY averaged; (uz, vz): vertical differences;
+    // (wz, 0): vertical difference of W
+    const int zu = z < NZ ? z + 1 : NZ, zd = z > 1 ? z - 1 : 1;
+    const T cz = (z == 1 || z == NZ) ? dzm : (T)0.5 * dzm;
+    const bool w1 = z <= NZ - 1, w0 = z >= 2;  // W(z), W(z-1) nonzero
+    const int qa = f == 0 ? 0 : f == 1 ? 4 : f == 2 ? 3 : f == 3 ? 0 : 4;
+    const int qb = f == 0 ? 2 : f == 1 ? 1 : f == 2 ? 5 : 2;
+    const bool wa = f == 1 || f == 4, wb = f == 2, dif = f == 3;
+    const cx<T>* A1 = row(qa, dif ? zu : z);
+    const cx<T>* A0 = row(qa, dif ? zd : (z > 1 ? z - 1 : 1));
+    const cx<T>* B1 = row(qb, dif ? zu : z);
+    const cx<T>* B0 = row(qb, dif ? zd : (z > 1 ? z - 1 : 1));
+    const bool a1 = !wa || w1, a0 = dif || (wa && w0), b1 = f != 4 && (!wb || w1), b0 = dif || (wb && w0);
+    const cx<T> zero = zero_cx<T>();
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int k = j + M1 * m;
+      const cx<T> pa1 = a1 ? A1[M1 * m] : zero, pa0 = a0 ? A0[M1 * m] : zero;
+      const cx<T> pb1 = b1 ? B1[M1 * m] : zero, pb0 = b0 ? B0[M1 * m] : zero;
       const T xk = kx0 * (T)k;
-      auto wl = [&](int f, int kk) -> cx<T> { return (kk >= 1 && kk <= NZ - 1) ? rowp(f, kk, y)[k] : zero_cx<T>(); };
-      auto vz = [&](int f) -> cx<T> {
-        if (z == 1) return (rowp(f, 2, y)[k] - rowp(f, 1, y)[k]) * dzm;
-        if (z == NZ) return (rowp(f, NZ, y)[k] - rowp(f, NZ - 1, y)[k]) * dzm;
-        return (rowp(f, z + 1, y)[k] - rowp(f, z - 1, y)[k]) * ((T)0.5 * dzm);
-      };
       cx<T> a, b;
-      switch (j) {
-        case 0: a = mul_i(rowp(0, z, y)[k]) * xk; b = mul_i(rowp(2, z, y)[k]) * xk; break;      // ux, vx
-        case 1: a = mul_i(wl(4, z) + wl(4, z - 1)) * ((T)0.5 * xk); b = rowp(1, z, y)[k]; break; // wx, uy
-        case 2: a = rowp(3, z, y)[k]; b = (wl(5, z) + wl(5, z - 1)) * (T)0.5; break;            // vy, wy
-        case 3: a = vz(0); b = vz(2); break;                                                    // uz, vz
-        default: a = (wl(4, z) - wl(4, z - 1)) * dzm; b = zero_cx<T>(); break;                  // wz
+      switch (f) {
+        case 0: a = mul_i(pa1) * xk; b = mul_i(pb1) * xk; break;             // ux, vx
+        case 1: a = mul_i(pa1 + pa0) * ((T)0.5 * xk); b = pb1; break;        // wx, uy
+        case 2: a = pa1; b = (pb1 + pb0) * (T)0.5; break;                    // vy, wy
+        case 3: a = (pa1 - pa0) * cz; b = (pb1 - pb0) * cz; break;           // uz, vz
+        default: a = (pa1 - pa0) * dzm; b = zero; break;                     // wz
       }
       if (k == 0) { a.y = 0; b.y = 0; }
-      d = mk(a.x - b.y, a.y + b.x);  // a + i b
-      m = mk(a.x + b.y, b.x - a.y);  // conj(a) + i conj(b)
+      x[m] = mk(a.x - b.y, a.y + b.x);    // a + i b
+      mir[m] = mk(a.x + b.y, b.x - a.y);  // conj(a) + i conj(b)
     }
-    zd[i] = d;
-    zm[i] = m;
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      v[m] = x[m];
+      const cx<T> r = shfl_cx(mask, mir[m], partner), own = m < 3 ? mir[m + 1] : zero;
+      v[7 - m] = j == 0 ? own : r;
+    }
+    if (act) {
+      Dft<8, +1, T>::run(v);
+      const cx<T>* g = tw + tw_off(NX);
+      cx<T>* p = buf + L::off(j);
+#pragma unroll
+      for (int b = 0; b < 8; b++) p[b * L::SB] = b ? cmul(v[b], conj(g[b * j])) : v[b];
+    }
+  }
+  auto team_wait = [&]() {
+    if (TP <= 32) __syncwarp(mask);
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + tm), "r"(TP) : "memory");
+  };
+  team_wait();
+  if constexpr (R3 > 1) {
+    if (t < M1) {  // M1 (b, i) pairs, two rounds of four b
+      const int i = t % R3;
+      cx<T>* p = buf + (t / R3) * L::SB + i;
+      const cx<T>* g = tw + tw_off(3 * NX / 2);
+      cx<T> w[4];
+#pragma unroll
+      for (int r = 1; r < 4; r++) w[r] = conj(g[12 * r * i]);
+#pragma unroll
+      for (int jj = 0; jj < 2; jj++) {
+        cx<T> v[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) v[r] = p[4 * jj * L::SB + r * L::SR];
+        Dft<4, +1, T>::run(v);
+#pragma unroll
+        for (int r = 0; r < 4; r++) p[4 * jj * L::SB + r * L::SR] = r ? cmul(v[r], w[r]) : v[r];
+      }
+    }
+    team_wait();
+  }
+  {
+    constexpr int RL = R3 > 1 ? R3 : R2, ITEMS = R3 > 1 ? 8 * R2 : 8;
+#pragma unroll
+    for (int it = 0; it < (ITEMS + TP - 1) / TP; it++) {
+      const int u = t + it * TP;
+      if (ITEMS % TP != 0 && u >= ITEMS) break;
+      cx<T>* p = buf + (R3 > 1 ? (u / R2) * L::SB + (u % R2) * L::SR : u * L::SB);
+      cx<T> v[RL];
+#pragma unroll
+      for (int i = 0; i < RL; i++) v[i] = p[i];
+      Dft<RL, +1, T>::run(v);
+#pragma unroll
+      for (int i = 0; i < RL; i++) p[i] = v[i];
+    }
   }
   __syncthreads();
-  // Stage 2: the inverse transforms from the staged spectra
-  fft_core<NX, +1, false, false, true>(5 * RB, sm, tw, [&](int t, int n) -> cx<T> {
-    if (n < KX) return zd[(size_t)t * KX + n];
-    if (NX - n < KX) return zm[(size_t)t * KX + (NX - n)];
-    return zero_cx<T>();
-  }, NoStore{});
   // the feature normalisation, read once per thread
   float nsh[11], nsc[11];
 #pragma unroll
@@ -182,15 +276,20 @@ k_lgrad_x(const cx<T>* __restrict__ gy, void* __restrict__ feat, const MlpDev* _
     nsh[jj] = RAW ? 0.f : P->in_shift[jj];
     nsc[jj] = RAW ? 1.f : P->in_scale[jj];
   }
-  for (int i = threadIdx.x; i < RB * NX; i += blockDim.x) {
-    const int rr = i / NX, x = i - rr * NX;
+  for (int i = threadIdx.x; i < RB * NX; i += L::THREADS) {
+    const int rr = i / NX, q0 = i - rr * NX;
     if (r0 + rr >= R) continue;
+    // x = b + 8 (r + R2 i); with R2 = 4 a half-warp takes four b and four r
+    // (SB = 4, SR = 1 mod 16 8-byte banks)
+    const int x = R3 > 1 ? (q0 & ~31) | (q0 & 3) | ((q0 & 12) << 1) | ((q0 & 16) >> 2) : q0;
+    const int o = x >> 3;
+    const cx<T>* gp = sm + (size_t)(5 * rr) * L::BUF + (x & 7) * L::SB + (R3 > 1 ? (o % R2) * L::SR + o / R2 : o);
     T g[9];
 #pragma unroll
-    for (int j = 0; j < 5; j++) {
-      const cx<T> v = sm[(size_t)(5 * rr + j) * NX + x];
-      g[2 * j] = v.x;
-      if (j < 4) g[2 * j + 1] = v.y;
+    for (int q = 0; q < 5; q++) {
+      const cx<T> v = gp[q * L::BUF];
+      g[2 * q] = v.x;
+      if (q < 4) g[2 * q + 1] = v.y;
     }
     int z, y;
     row_zy(rr, z, y);
@@ -288,7 +387,7 @@ template <class T> struct MlpOutTau {
   }
 };
 
-// Mean dissipations (per-CTA triples of sums in CTA order: the raw
+// Mean dissipations (per-CTA triples of sums in a fixed order: the raw
 // network's, the applied, the reference) -> flag, status [applied mean,
 // flag, reference mean, raw mean] and the stage counters [stages, stages
 // that used the network].  The network is used when its raw mean
@@ -297,9 +396,15 @@ template <class T> struct MlpOutTau {
 static __global__ void k_learned_flag(const double* __restrict__ part, int nparts, double inv_n_delta, double guard,
                                       int* __restrict__ flag, double* __restrict__ status,
                                       unsigned long long* __restrict__ counts) {
-  if (threadIdx.x != 0) return;
+  // one warp: lanes over the parts, then a fixed tree
   double sr = 0.0, sa = 0.0, sf = 0.0;
-  for (int i = 0; i < nparts; i++) { sr += part[3 * i]; sa += part[3 * i + 1]; sf += part[3 * i + 2]; }
+  for (int i = threadIdx.x; i < nparts; i += 32) { sr += part[3 * i]; sa += part[3 * i + 1]; sf += part[3 * i + 2]; }
+  for (int o = 16; o > 0; o >>= 1) {
+    sr += __shfl_xor_sync(0xffffffffu, sr, o);
+    sa += __shfl_xor_sync(0xffffffffu, sa, o);
+    sf += __shfl_xor_sync(0xffffffffu, sf, o);
+  }
+  if (threadIdx.x != 0) return;
   const double raw = sr * inv_n_delta, applied = sa * inv_n_delta, ref = sf * inv_n_delta;
   int use = (raw >= 0.0) ? 1 : 0;  // NaN -> fallback
   if (guard > 0.0 && !(ref > 0.0 && applied <= guard * ref && guard * applied >= ref)) use = 0;

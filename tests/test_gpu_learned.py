@@ -221,3 +221,64 @@ def test_mma_wait_limit_in_the_learned_stage(gpu_lib, product):
     a, b = g2.download(), g3.download()
     for k in "uvwe":
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(16, 16, 5), (32, 96, 4), (64, 192, 4), (96, 16, 5), (128, 384, 4), (192, 32, 4),
+                                      (256, 64, 4), (384, 128, 4), (512, 256, 4)])
+def test_features_at_every_row_and_column_length(gpu_lib, product, nx, ny, nz):
+    """The gradient transforms of every grid length (rows and columns) against
+    numpy's: f32 output of FP64 gradients to its rounding, of FP32 gradients to
+    the FP32 transforms' error (2e-5 of the largest gradient, as the operator
+    tests) over the smallest |G| of the field (a mean shear keeps it away from
+    zero)."""
+    cfg = product.channel_config(nx, ny, nz, dt=1e-3, re_tau=180.0, imodel=5)
+    rng = np.random.default_rng(nx + ny)
+    dz = cfg.zl / nz
+    z = (np.arange(nz) + 0.5) * dz
+    k = np.arange(1, 4)
+
+    def smooth():  # a few low modes: gradients of order one at every point
+        x, y = np.arange(nx) * cfg.xl / nx, np.arange(ny) * cfg.yl / ny
+        a = np.zeros((nz, ny, nx))
+        for kx in k:
+            for ky in k:
+                c = 0.1 * rng.standard_normal((2, nz))
+                a += (c[0][:, None, None] * np.cos(kx * x)[None, None, :] * np.cos(2 * ky * y)[None, :, None]
+                      + c[1][:, None, None] * np.sin(kx * x)[None, None, :] * np.sin(2 * ky * y)[None, :, None])
+        return a
+
+    u = smooth() + 20.0 * z[:, None, None]
+    v, w = smooth(), smooth()
+    w[-1] = 0.0
+
+    def d(a, axis, n, length):
+        kk = np.fft.fftfreq(n, 1.0 / n) * 2 * np.pi / length
+        kk[n // 2] = 0.0
+        sh = [1, 1, 1]
+        sh[axis] = n
+        return np.fft.ifft(np.fft.fft(a, axis=axis) * (1j * kk).reshape(sh), axis=axis).real
+
+    wl = np.concatenate([np.zeros((1, ny, nx)), w[:-1], np.zeros((1, ny, nx))])  # w-levels 0..nz
+    wc = 0.5 * (wl[1:] + wl[:-1])
+
+    def dzc(a):
+        o = np.empty_like(a)
+        o[1:-1] = (a[2:] - a[:-2]) / (2 * dz)
+        o[0], o[-1] = (a[1] - a[0]) / dz, (a[-1] - a[-2]) / dz
+        return o
+
+    dx, dy = lambda a: d(a, 2, nx, cfg.xl), lambda a: d(a, 1, ny, cfg.yl)
+    g = np.stack([dx(u), dx(v), dx(wc), dy(u), dy(v), dy(wc), dzc(u), dzc(v), (wl[1:] - wl[:-1]) / dz], -1).reshape(-1, 9)
+    G = np.sqrt((g * g).sum(1))
+    zw = np.minimum(z, cfg.zl - z)
+    delta = (cfg.xl / nx * cfg.yl / ny * dz) ** (1.0 / 3.0)
+    ref = np.concatenate([g / G[:, None], np.repeat(np.minimum(zw / delta, 16.0), nx * ny)[:, None],
+                          np.repeat(zw * 2 / cfg.zl, nx * ny)[:, None], (delta * G)[:, None]], 1)
+    for precision, tol in ((8, 1e-6), (4, 2e-5 * np.abs(g).max() / G.min())):
+        cfg.precision = precision
+        h = product.LesGpu(cfg)
+        h.upload(u, v, w, np.full_like(u, 1e-4), None)
+        got = h.learned_features().cpu().numpy().astype(np.float64)
+        assert np.abs(got[:, :12] - ref).max() < tol * np.maximum(1.0, np.abs(ref).max()), precision
+        assert not got[:, 12:].any()
+        h.close()
