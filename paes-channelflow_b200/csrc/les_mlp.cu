@@ -112,7 +112,7 @@ void read_err(les_mlp* m, cudaStream_t s) {
 int train_partials(les_mlp* m, const void* feat, const float* target, long long n, cudaStream_t s) {
   const long long ntiles = (n + 127) / 128;
   const int grid = (int)std::min<long long>(ntiles, m->nsm);
-  launch(k_mlp_train, dim3(grid), dim3(128), kTrainSmemLaunch, s, (const MlpDev*)m->dev, (const uint4*)feat,
+  launch(k_mlp_train, dim3(grid), dim3(kTrainThreads), kTrainSmemLaunch, s, (const MlpDev*)m->dev, (const uint4*)feat,
          (const float4*)target, n, m->part.p, m->lpart.p, m->err.p);
   return grid;
 }
@@ -147,7 +147,7 @@ int les_mlp_create(int device, les_mlp** out) {
     LES_CUDA(cudaMemset(m->dev, 0, sizeof(MlpDev)));
     LES_CUDA(cudaMemcpy(&m->dev->wait_ns, &m->wait_ns, sizeof(m->wait_ns), cudaMemcpyHostToDevice));
     for (auto* b : {&m->master, &m->m1, &m->m2, &m->grad}) b->alloc(kMlpNParam);
-    m->part.alloc((size_t)m->nsm * kMlpNParam);
+    m->part.alloc((size_t)m->nsm * kMlpPart);
     m->lpart.alloc(m->nsm);
     m->err.alloc(1);
   });
@@ -233,7 +233,7 @@ int les_mlp_loss_grad(les_mlp* m, const void* feat, const float* target, long lo
     check_samples(feat, target, n);
     cudaStream_t s = (cudaStream_t)stream;
     const int np = train_partials(m, feat, target, n, s);
-    launch(k_mlp_reduce_adam, dim3(cdiv(kMlpNParam, 256)), dim3(256), 0, s, (const float*)m->part.p, np, grad,
+    launch(k_mlp_reduce_adam, dim3(cdiv(kMlpNParam, 64)), dim3(64), 0, s, (const float*)m->part.p, np, grad,
            m->master.p, m->m1.p, m->m2.p, m->dev, 0, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
     const double l = host_loss(m, np, n, s);
     if (loss) *loss = l;
@@ -250,7 +250,7 @@ int les_mlp_adam_step(les_mlp* m, const void* feat, const float* target, long lo
     m->adam_step++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = (float)(1.0 - std::pow(0.9, m->adam_step)), c2 = (float)(1.0 - std::pow(0.999, m->adam_step));
-    launch(k_mlp_reduce_adam, dim3(cdiv(kMlpNParam, 256)), dim3(256), 0, s, (const float*)m->part.p, np, m->grad.p,
+    launch(k_mlp_reduce_adam, dim3(cdiv(kMlpNParam, 64)), dim3(64), 0, s, (const float*)m->part.p, np, m->grad.p,
            m->master.p, m->m1.p, m->m2.p, m->dev, 1, lr, b1, b2, 1e-8f, c1, c2);
     if (loss) *loss = host_loss(m, np, n, s);
   });

@@ -28,6 +28,7 @@ namespace les {
 constexpr int kMlpIn = 11, kMlpHid = 64, kMlpOut = 6;
 constexpr int kMlpNParam = 9478;
 constexpr int kMlpNNorm = 34;
+constexpr int kMlpPart = 9480;  // stride of the per-CTA gradient partials (rows of W2, W3 16-byte aligned)
 // offsets in the flat parameter vector: W1[64][11], b1, W2[64][64], b2, W3, b3, W4[6][64], b4
 constexpr int kPW1 = 0, kPB1 = 704, kPW2 = 768, kPB2 = 4864, kPW3 = 4928, kPB3 = 9024, kPW4 = 9088, kPB4 = 9472;
 constexpr int ERR_MMA_TIMEOUT = 4;
@@ -86,12 +87,11 @@ __device__ __forceinline__ bool bar_any(int id, int count, bool pred) {
   return r != 0;
 }
 
-// Bias + GELU of the 64 accumulator columns of this thread's lane, written
-// as row r of a K = 64 activation tile.
-__device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float* __restrict__ b, unsigned char* act,
-                                                int r) {
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
+// Bias + GELU of accumulator columns 16c..16c+15 of this thread's lane,
+// written into row r of a K = 64 activation tile.
+__device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float* __restrict__ b, unsigned char* act, int r,
+                                                int c) {
+  {
     float v[16];
     tc::tmem_ld16(taddr + 16 * c, v);
     uint32_t pk[8];
@@ -403,49 +403,60 @@ struct MlpOutRaw {
 };
 
 // ------------------------------------------------------------------------
-// Training: loss and gradient of a batch.  One group (4 warps) per CTA and
-// the whole tensor memory (512 columns):
+// Training: loss and gradient of a batch.  Four groups of 4 warps per CTA, all
+// on one 128-sample tile: every group covers the tile's lanes and takes 16 of
+// the 64 columns of each epilogue (one group alone spent most of a tile in
+// these chains; an Adam step of 65536 samples took 70 us, now 47, same bits).
+// Bound by the chain of 8 products, epilogues and barriers of a tile (3.5 tiles
+// per SM at that batch), tensor pipe 7%.  The whole tensor memory (512
+// columns):
 //   Z1 [0,64) Z2 [64,128) Z3 [128,192) Z4 [192,208) dA3 [208,272)
 //   dW1 [272,288) dW2 [288,352) dW3 [352,416) dW4^T [416,432)
 //   db1 [432,448) db2 [448,464) db3 [464,480)
 // dA2 reuses Z3's columns and dA1 Z2's once those pre-activations are read.
 // Accumulators of M = 64 occupy lanes 0-15 of each 32-lane quarter: row m
 // is lane 32*(m/16) + m%16.
-// Shared memory: parameters, activation tiles A0 (K=16), A1..A3 (K=64),
-// dZ tiles D (K=64) and D4 (K=16), a tile of ones (K=16).
-// Per-CTA outputs: part[blockIdx.x][9478] gradient partial sums (flat
+// The weight-gradient MMAs of a layer are issued after the commit of the dA
+// product the next epilogue waits for, so they run under that epilogue; the
+// commit of the next product covers them.  What they read is not overwritten
+// before it: the dZ tiles alternate, and so do the feature tiles.
+// Shared memory: parameters, two feature tiles A0 (K=16), activation tiles
+// A1..A3 (K=64), two dZ tiles (K=64), D4 (K=16), a tile of ones (K=16).
+// Per-CTA outputs: part[blockIdx.x][kMlpPart] gradient partial sums (flat
 // parameter order) and lpart[blockIdx.x] the loss partial sum.
 // ------------------------------------------------------------------------
-constexpr size_t kTrainSmem = sizeof(MlpDev) + 4096 + 3 * 16384 + 16384 + 4096 + 4096 + 512;
+constexpr int kTrainThreads = 512;
+constexpr size_t kTrainSmem = sizeof(MlpDev) + 2 * 4096 + 3 * 16384 + 2 * 16384 + 4096 + 4096 + 512;
 // keep one CTA per SM: it owns all 512 tensor-memory columns
 constexpr size_t kTrainSmemLaunch = kTrainSmem > 120 * 1024 ? kTrainSmem : 120 * 1024;
 
-static __global__ void __launch_bounds__(128, 1)
+static __global__ void __launch_bounds__(kTrainThreads, 1)
 k_mlp_train(const MlpDev* __restrict__ prm, const uint4* __restrict__ feat, const float4* __restrict__ target,
             long long n, float* __restrict__ part, double* __restrict__ lpart, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smraw_tc[];
   MlpDev* P = reinterpret_cast<MlpDev*>(smraw_tc);
   unsigned char* A0 = smraw_tc + sizeof(MlpDev);
-  unsigned char* A1 = A0 + 4096;
+  unsigned char* A1 = A0 + 2 * 4096;
   unsigned char* A2 = A1 + 16384;
   unsigned char* A3 = A2 + 16384;
   unsigned char* Dt = A3 + 16384;
-  unsigned char* D4 = Dt + 16384;
+  unsigned char* D4 = Dt + 2 * 16384;
   unsigned char* ONES = D4 + 4096;
   uint64_t* barp = reinterpret_cast<uint64_t*>(ONES + 4096);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(barp + 1);
   float* redf = reinterpret_cast<float*>(barp + 2);  // 4 warps x 8 floats
   double* redd = reinterpret_cast<double*>(barp + 2 + 16);
 
-  const int r = threadIdx.x, warp = r >> 5, lane = r & 31;
-  for (int i = r; i < (int)(sizeof(MlpDev) / 16); i += 128)
+  const int tid = threadIdx.x, r = tid & 127, h = tid >> 7, warp = r >> 5, lane = r & 31;  // row, column chunk
+  for (int i = tid; i < (int)(sizeof(MlpDev) / 16); i += kTrainThreads)
     reinterpret_cast<uint4*>(P)[i] = reinterpret_cast<const uint4*>(prm)[i];
   {
     const uint32_t one2 = pack_bf2(1.0f, 1.0f);
-    for (int i = r; i < 4096 / 16; i += 128) reinterpret_cast<uint4*>(ONES)[i] = make_uint4(one2, one2, one2, one2);
+    for (int i = tid; i < 4096 / 16; i += kTrainThreads)
+      reinterpret_cast<uint4*>(ONES)[i] = make_uint4(one2, one2, one2, one2);
   }
-  if (r == 0) tc::mbar_init(barp, 1);
-  if (warp == 0) {
+  if (tid == 0) tc::mbar_init(barp, 1);
+  if (tid < 32) {
     tc::tmem_alloc(tslot, 512);
     tc::tmem_relinquish();
   }
@@ -458,8 +469,8 @@ k_mlp_train(const MlpDev* __restrict__ prm, const uint4* __restrict__ feat, cons
   const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
   const uint32_t cZ1 = 0, cZ2 = 64, cZ3 = 128, cZ4 = 192, cdA3 = 208, cW1 = 272, cW2 = 288, cW3 = 352, cW4 = 416,
                  cB1 = 432, cB2 = 448, cB3 = 464;
-  const uint32_t a0s = tc::smem_addr(A0), a1s = tc::smem_addr(A1), a2s = tc::smem_addr(A2), a3s = tc::smem_addr(A3),
-                 dts = tc::smem_addr(Dt), d4s = tc::smem_addr(D4), ones = tc::smem_addr(ONES);
+  const uint32_t a1s = tc::smem_addr(A1), a2s = tc::smem_addr(A2), a3s = tc::smem_addr(A3), d4s = tc::smem_addr(D4),
+                 ones = tc::smem_addr(ONES);
   const uint32_t w1s = tc::smem_addr(P->w1), w2s = tc::smem_addr(P->w2), w3s = tc::smem_addr(P->w3),
                  w4s = tc::smem_addr(P->w4);
   constexpr uint32_t idB64 = tc::idesc_bf16(128, 64, false, true);   // dA = dZ * W (W read MN-major)
@@ -480,27 +491,27 @@ k_mlp_train(const MlpDev* __restrict__ prm, const uint4* __restrict__ feat, cons
   auto sync_check = [&](bool bad) -> bool {
     tc::fence_async_smem();
     tc::fence_before_sync();
-    return bar_any(1, 128, bad);
+    return bar_any(1, kTrainThreads, bad);
   };
-  // dZ = dA * GELU'(Z + b) for the 64 columns of this lane, into tile Dt
-  auto back_epilogue = [&](uint32_t c_dA, uint32_t c_Z, const float* b) {
+  // dZ = dA * GELU'(Z + b) for this thread's 16 columns, into dZ tile d
+  auto back_epilogue = [&](uint32_t c_dA, uint32_t c_Z, const float* b, int d) {
+    const int c = h;
+    unsigned char* dst = Dt + d * 16384;
+    float da[16], z[16];
+    tc::tmem_ld16(tb + lane_off + c_dA + 16 * c, da);
+    tc::tmem_ld16(tb + lane_off + c_Z + 16 * c, z);
+    uint32_t pk[8];
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      float da[16], z[16];
-      tc::tmem_ld16(tb + lane_off + c_dA + 16 * c, da);
-      tc::tmem_ld16(tb + lane_off + c_Z + 16 * c, z);
-      uint32_t pk[8];
-#pragma unroll
-      for (int j = 0; j < 8; j++)
-        pk[j] = pack_bf2(da[2 * j] * gelu_grad(z[2 * j] + b[16 * c + 2 * j]),
-                         da[2 * j + 1] * gelu_grad(z[2 * j + 1] + b[16 * c + 2 * j + 1]));
-      *reinterpret_cast<uint4*>(Dt + 2 * tc::tile_elem(r, 16 * c, 64)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-      *reinterpret_cast<uint4*>(Dt + 2 * tc::tile_elem(r, 16 * c + 8, 64)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-    }
+    for (int j = 0; j < 8; j++)
+      pk[j] = pack_bf2(da[2 * j] * gelu_grad(z[2 * j] + b[16 * c + 2 * j]),
+                       da[2 * j + 1] * gelu_grad(z[2 * j + 1] + b[16 * c + 2 * j + 1]));
+    *reinterpret_cast<uint4*>(dst + 2 * tc::tile_elem(r, 16 * c, 64)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    *reinterpret_cast<uint4*>(dst + 2 * tc::tile_elem(r, 16 * c + 8, 64)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
   };
   // weight / bias gradient MMAs of a hidden layer: dW (M=64 outputs) over the
-  // tile's 128 samples, A = Dt (MN-major), B = the layer's input tile
-  auto issue_dw = [&](uint32_t c_W, uint32_t c_B, uint32_t in_s, int kin) {
+  // tile's 128 samples, A = dZ tile d (MN-major), B = the layer's input tile
+  auto issue_dw = [&](uint32_t c_W, uint32_t c_B, uint32_t in_s, int kin, int d) {
+    const uint32_t dts = tc::smem_addr(Dt + d * 16384);
     const uint32_t lbo_in = (uint32_t)(kin / 8) * 128;
     const uint32_t id = kin == 64 ? idW64 : idW16;
 #pragma unroll 1
@@ -510,8 +521,9 @@ k_mlp_train(const MlpDev* __restrict__ prm, const uint4* __restrict__ feat, cons
       tc::mma_bf16(tb + c_B, a, tc::sdesc(ones + 2 * 256 * s, 256, 128), idW16, (accw | s) ? 1u : 0u);
     }
   };
-  // dA = Dt * W (M = 128 samples, N = 64 inputs, K = 64 outputs)
-  auto issue_da = [&](uint32_t c_dA, uint32_t w_s) {
+  // dA = dZ * W (M = 128 samples, N = 64 inputs, K = 64 outputs)
+  auto issue_da = [&](uint32_t c_dA, uint32_t w_s, int d) {
+    const uint32_t dts = tc::smem_addr(Dt + d * 16384);
 #pragma unroll
     for (int s = 0; s < 4; s++)
       tc::mma_bf16(tb + c_dA, tc::sdesc(dts + 256 * s, 128, 1024), tc::sdesc(w_s + 2 * 1024 * s, 1024, 128), idB64,
@@ -519,34 +531,39 @@ k_mlp_train(const MlpDev* __restrict__ prm, const uint4* __restrict__ feat, cons
   };
 
   const long long ntiles = (n + 127) / 128;
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  int ab = 0;  // feature tile
+  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ab ^= 1) {
     const long long p = tile * 128 + r;
     const bool valid = p < n;
-    uint4 f0 = make_uint4(0, 0, 0, 0), f1 = f0;
+    unsigned char* A0t = A0 + ab * 4096;
+    const uint32_t a0s = tc::smem_addr(A0t);
     float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
-    if (valid) {
-      f0 = __ldg(feat + 2 * p); f1 = __ldg(feat + 2 * p + 1);
-      t0 = __ldg(target + 2 * p); t1 = __ldg(target + 2 * p + 1);
+    if (h == 0) {
+      uint4 f0 = make_uint4(0, 0, 0, 0), f1 = f0;
+      if (valid) {
+        f0 = __ldg(feat + 2 * p); f1 = __ldg(feat + 2 * p + 1);
+        t0 = __ldg(target + 2 * p); t1 = __ldg(target + 2 * p + 1);
+      }
+      *reinterpret_cast<uint4*>(A0t + 2 * tc::tile_elem(r, 0, 16)) = f0;
+      *reinterpret_cast<uint4*>(A0t + 2 * tc::tile_elem(r, 8, 16)) = f1;
     }
-    *reinterpret_cast<uint4*>(A0 + 2 * tc::tile_elem(r, 0, 16)) = f0;
-    *reinterpret_cast<uint4*>(A0 + 2 * tc::tile_elem(r, 8, 16)) = f1;
     if (sync_check(false)) { failed = true; break; }
     // ---- forward ----
-    if (r == 0) { tc::fence_after_sync(); issue_layer<64, 16>(tb + cZ1, a0s, w1s); tc::mma_commit(barp); }
+    if (tid == 0) { tc::fence_after_sync(); issue_layer<64, 16>(tb + cZ1, a0s, w1s); tc::mma_commit(barp); }
     bool bad = !wait_mma();
-    hidden_epilogue(tb + lane_off + cZ1, P->b1, A1, r);
+    hidden_epilogue(tb + lane_off + cZ1, P->b1, A1, r, h);
     if (sync_check(bad)) { failed = true; break; }
-    if (r == 0) { tc::fence_after_sync(); issue_layer<64, 64>(tb + cZ2, a1s, w2s); tc::mma_commit(barp); }
+    if (tid == 0) { tc::fence_after_sync(); issue_layer<64, 64>(tb + cZ2, a1s, w2s); tc::mma_commit(barp); }
     bad = !wait_mma();
-    hidden_epilogue(tb + lane_off + cZ2, P->b2, A2, r);
+    hidden_epilogue(tb + lane_off + cZ2, P->b2, A2, r, h);
     if (sync_check(bad)) { failed = true; break; }
-    if (r == 0) { tc::fence_after_sync(); issue_layer<64, 64>(tb + cZ3, a2s, w3s); tc::mma_commit(barp); }
+    if (tid == 0) { tc::fence_after_sync(); issue_layer<64, 64>(tb + cZ3, a2s, w3s); tc::mma_commit(barp); }
     bad = !wait_mma();
-    hidden_epilogue(tb + lane_off + cZ3, P->b3, A3, r);
+    hidden_epilogue(tb + lane_off + cZ3, P->b3, A3, r, h);
     if (sync_check(bad)) { failed = true; break; }
-    if (r == 0) { tc::fence_after_sync(); issue_layer<16, 64>(tb + cZ4, a3s, w4s); tc::mma_commit(barp); }
+    if (tid == 0) { tc::fence_after_sync(); issue_layer<16, 64>(tb + cZ4, a3s, w4s); tc::mma_commit(barp); }
     bad = !wait_mma();
-    {
+    if (h == 0) {
       float y[16];
       tc::tmem_ld16(tb + lane_off + cZ4, y);
       const float tg[6] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y};
@@ -565,97 +582,101 @@ k_mlp_train(const MlpDev* __restrict__ prm, const uint4* __restrict__ feat, cons
       *reinterpret_cast<uint4*>(D4 + 2 * tc::tile_elem(r, 8, 16)) = make_uint4(0u, 0u, 0u, 0u);
     }
     if (sync_check(bad)) { failed = true; break; }
-    // ---- backward, layer 4: dW4^T (M = 64 inputs, N = 16 outputs) and dA3 ----
-    if (r == 0) {
+    // ---- backward, layer 4: dA3, then dW4^T (M = 64 inputs, N = 16 outputs) ----
+    if (tid == 0) {
       tc::fence_after_sync();
+      // dA3 = dZ4 * W4: K = 16 outputs, W4 tile read MN-major (rows = outputs)
+      tc::mma_bf16(tb + cdA3, tc::sdesc(d4s, 128, 256), tc::sdesc(w4s, 1024, 128), idB64, 0u);
+      tc::mma_commit(barp);
 #pragma unroll 1
       for (int s = 0; s < 8; s++)
         tc::mma_bf16(tb + cW4, tc::sdesc(a3s + 2 * 1024 * s, 1024, 128), tc::sdesc(d4s + 2 * 256 * s, 256, 128), idW16,
                      (accw | s) ? 1u : 0u);
-      // dA3 = dZ4 * W4: K = 16 outputs, W4 tile read MN-major (rows = outputs)
-      tc::mma_bf16(tb + cdA3, tc::sdesc(d4s, 128, 256), tc::sdesc(w4s, 1024, 128), idB64, 0u);
-      tc::mma_commit(barp);
     }
     bad = !wait_mma();
-    back_epilogue(cdA3, cZ3, P->b3);  // dZ3
+    back_epilogue(cdA3, cZ3, P->b3, 0);  // dZ3
     if (sync_check(bad)) { failed = true; break; }
-    if (r == 0) {
+    if (tid == 0) {
       tc::fence_after_sync();
-      issue_dw(cW3, cB3, a2s, 64);
-      issue_da(cZ3, w3s);  // dA2 into Z3's columns
+      issue_da(cZ3, w3s, 0);  // dA2 into Z3's columns
       tc::mma_commit(barp);
+      issue_dw(cW3, cB3, a2s, 64, 0);
     }
     bad = !wait_mma();
-    back_epilogue(cZ3, cZ2, P->b2);  // dZ2
+    back_epilogue(cZ3, cZ2, P->b2, 1);  // dZ2
     if (sync_check(bad)) { failed = true; break; }
-    if (r == 0) {
+    if (tid == 0) {
       tc::fence_after_sync();
-      issue_dw(cW2, cB2, a1s, 64);
-      issue_da(cZ2, w2s);  // dA1 into Z2's columns
+      issue_da(cZ2, w2s, 1);  // dA1 into Z2's columns
       tc::mma_commit(barp);
+      issue_dw(cW2, cB2, a1s, 64, 1);
     }
     bad = !wait_mma();
-    back_epilogue(cZ2, cZ1, P->b1);  // dZ1
+    back_epilogue(cZ2, cZ1, P->b1, 0);  // dZ1 (the commit above covers dW3's reads of this tile)
     if (sync_check(bad)) { failed = true; break; }
-    if (r == 0) {
+    if (tid == 0) {
       tc::fence_after_sync();
-      issue_dw(cW1, cB1, a0s, 16);
-      tc::mma_commit(barp);
+      issue_dw(cW1, cB1, a0s, 16, 0);
     }
-    bad = !wait_mma();
     accw = 1;
-    if (sync_check(bad)) { failed = true; break; }
   }
-  if (failed && r == 0) {
+  if (!failed) {  // the last weight gradients
+    if (tid == 0) tc::mma_commit(barp);
+    const bool bad = !wait_mma();
+    failed = sync_check(bad);
+  }
+  if (failed && tid == 0) {
     atomicOr(err, ERR_MMA_TIMEOUT);
+    // the outstanding commit, then whatever was issued after it
     tc::mbar_wait(barp, parity ^ 1, kMmaWaitNs);
+    tc::mma_commit(barp);
+    tc::mbar_wait(barp, parity, kMmaWaitNs);
   }
   // ---- per-CTA partial sums ----
-  float* out = part + (size_t)blockIdx.x * kMlpNParam;
+  float* out = part + (size_t)blockIdx.x * kMlpPart;
   if (accw) {
     // M = 64 accumulators: thread (warp q, lane l < 16) holds row 16q + l
     const int m = warp * 16 + lane;
     float v[16];
-    // dW1 [64][11]
-    tc::tmem_ld16(tb + lane_off + cW1, v);
-    if (lane < 16)
-      for (int i = 0; i < kMlpIn; i++) out[kPW1 + m * kMlpIn + i] = v[i];
-    tc::tmem_ld16(tb + lane_off + cB1, v);
-    if (lane < 16) out[kPB1 + m] = v[0];
-    tc::tmem_ld16(tb + lane_off + cB2, v);
-    if (lane < 16) out[kPB2 + m] = v[0];
-    tc::tmem_ld16(tb + lane_off + cB3, v);
-    if (lane < 16) out[kPB3 + m] = v[0];
-#pragma unroll 1
-    for (int c = 0; c < 4; c++) {
-      tc::tmem_ld16(tb + lane_off + cW2 + 16 * c, v);
+    // each group takes 16 columns of dW2 and dW3 and one of the narrow ones
+    if (h == 0) {  // dW1 [64][11]
+      tc::tmem_ld16(tb + lane_off + cW1, v);
       if (lane < 16)
-        for (int i = 0; i < 16; i++) out[kPW2 + m * 64 + 16 * c + i] = v[i];
-      tc::tmem_ld16(tb + lane_off + cW3 + 16 * c, v);
-      if (lane < 16)
-        for (int i = 0; i < 16; i++) out[kPW3 + m * 64 + 16 * c + i] = v[i];
+        for (int i = 0; i < kMlpIn; i++) out[kPW1 + m * kMlpIn + i] = v[i];
+    } else {
+      tc::tmem_ld16(tb + lane_off + (h == 1 ? cB1 : h == 2 ? cB2 : cB3), v);
+      if (lane < 16) out[(h == 1 ? kPB1 : h == 2 ? kPB2 : kPB3) + m] = v[0];
     }
-    // dW4^T: row m = input, columns = outputs
-    tc::tmem_ld16(tb + lane_off + cW4, v);
-    if (lane < 16)
-      for (int o = 0; o < kMlpOut; o++) out[kPW4 + o * 64 + m] = v[o];
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+      tc::tmem_ld16(tb + lane_off + (w ? cW3 : cW2) + 16 * h, v);
+      float4* o = reinterpret_cast<float4*>(out + (w ? kPW3 : kPW2) + m * 64 + 16 * h);
+      if (lane < 16)
+#pragma unroll
+        for (int i = 0; i < 4; i++) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+    if (h == 3) {  // dW4^T: row m = input, columns = outputs
+      tc::tmem_ld16(tb + lane_off + cW4, v);
+      if (lane < 16)
+        for (int o = 0; o < kMlpOut; o++) out[kPW4 + o * 64 + m] = v[o];
+    }
   } else {
-    for (int i = r; i < kPB4; i += 128) out[i] = 0.f;
+    for (int i = tid; i < kPB4; i += kTrainThreads) out[i] = 0.f;
   }
   // db4 and the loss: block sums in a fixed order
 #pragma unroll
   for (int j = 0; j < kMlpOut; j++) {
     float s = db4[j];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) redf[warp * 8 + j] = s;
+    if (h == 0 && lane == 0) redf[warp * 8 + j] = s;
   }
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if (lane == 0) redd[warp] = lsum;
+  if (h == 0 && lane == 0) redd[warp] = lsum;
   tc::fence_before_sync();
   __syncthreads();
-  if (r < kMlpOut) out[kPB4 + r] = redf[r] + redf[8 + r] + redf[16 + r] + redf[24 + r];
-  if (r == 0) lpart[blockIdx.x] = redd[0] + redd[1] + redd[2] + redd[3];
-  if (warp == 0) {
+  if (tid < kMlpOut) out[kPB4 + tid] = redf[tid] + redf[8 + tid] + redf[16 + tid] + redf[24 + tid];
+  if (tid == 0) lpart[blockIdx.x] = redd[0] + redd[1] + redd[2] + redd[3];
+  if (tid < 32) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tb, 512);
   }
@@ -670,8 +691,17 @@ static __global__ void k_mlp_reduce_adam(const float* __restrict__ part, int npa
                                   float c1, float c2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kMlpNParam) return;
+  // 37 partials' loads in flight (148 CTAs in four batches), added in order
+  constexpr int U = 37;
   float g = 0.f;
-  for (int c = 0; c < nparts; c++) g += part[(size_t)c * kMlpNParam + i];
+  for (int c0 = 0; c0 < nparts; c0 += U) {
+    float v[U];
+#pragma unroll
+    for (int c = 0; c < U; c++) v[c] = c0 + c < nparts ? part[(size_t)(c0 + c) * kMlpPart + i] : 0.f;
+#pragma unroll
+    for (int c = 0; c < U; c++)
+      if (c0 + c < nparts) g += v[c];
+  }
   grad[i] = g;
   if (!adam) return;
   const float mm = b1 * m1[i] + (1.f - b1) * g;
