@@ -201,7 +201,7 @@ struct Engine : EngineBase {
   // fused path (k_row_fused): clip corrections and wall-model planes
   bool fused = false;
   DevBuf<int> clipflag;
-  DevBuf<unsigned char> rowclip;  // per (level, row block): clipped (k_clip_x_flag)
+  DevBuf<unsigned char> rowclip;  // per (level, row block): clipped (k_clip_walls)
   DevBuf<T> ephys, dEX, dEY;
   DevBuf<cx<T>> xout[8];  // Xu1..Xe2 written by k_row_fused (its inputs stay readable)
   DevBuf<double> divacc, sgsacc, wacc, acc;
@@ -778,27 +778,25 @@ struct Engine : EngineBase {
            (const double*)mrv.p, a, (double)pb, 0.4, zody, cfg.ufree, wp.p, err.p);
   }
   void fused_middle(const StageArgs& a) {
-    int brows = 1;  // rows of a block of k_clip_x_flag
+    int brows = 1, nwall = 1;  // rows of a clip block, blocks of wall rows per side
     with_small(NX, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
       using C = RowCfg<3 * N / 2>;
       brows = 2 * C::NT;
-      // clip flags and corrections of max(expand(e), emin)
-      launch(k_clip_x_flag<T, N>, dim3(cdiv(MY / 2, C::NT), NZ - 1), dim3(C::THREADS), C::template smem<T>(), st,
-             (const cx<T>*)mixed[6].p, ephys.p, dEX.p, clipflag.p, rowclip.p, MY, (T)cfg.emin, (T)kx0, tw);
-      // wall-model sums of U, V at levels 1 and nnz
-      const unsigned nblk = cdiv(MY, C::NT);
-      launch(k_wall_rows<T, N>, dim3(nblk, 2), dim3(C::THREADS), C::template smem<T>(), st, (const cx<T>*)mixed[0].p,
-             (const cx<T>*)mixed[2].p, MY, NZ, wacc.p, tw);
-      wall_final((int)nblk, a);
+      nwall = (int)cdiv(MY, C::NT);
+      // clip flags and corrections of max(expand(e), emin), and the wall-model
+      // sums of U, V at levels 1 and nnz
+      launch(k_clip_walls<T, N>, dim3(cdiv(MY / 2, C::NT), NZ - 1 + 4), dim3(C::THREADS), C::template smem<T>(), st,
+             (const cx<T>*)mixed[6].p, ephys.p, dEX.p, clipflag.p, rowclip.p, (const cx<T>*)mixed[0].p,
+             (const cx<T>*)mixed[2].p, wacc.p, nwall, MY, NZ, (T)cfg.emin, (T)kx0, tw);
     });
     with_small(NY, [&](auto cn) {
       constexpr int N = decltype(cn)::value;
       using C = ColCfg<3 * N / 2, T>;
-      launch(k_clipd_y<T, N>, dim3(cdiv(MX / 2, C::TC), NZ - 1), dim3(C::THREADS), C::buf(), st,
-             (const T*)ephys.p, dEY.p, (const int*)clipflag.p, (const unsigned char*)rowclip.p, brows, MX, (T)cfg.emin,
-             (T)ky0, tw);
+      launch(k_clipd_y<T, N>, dim3(cdiv(MX / 2, C::TC), NZ - 1), dim3(C::THREADS), C::buf(), st, (const T*)ephys.p,
+             dEY.p, (const int*)clipflag.p, (const unsigned char*)rowclip.p, brows, MX, (T)cfg.emin, (T)ky0, tw);
     });
+    wall_final(nwall, a);
     // the fused row kernel
     FusedArgs fa{};
     for (int i = 0; i < 8; i++) { fa.in.p[i] = mixed[i].p; fa.out.p[i] = xout[i].p; }

@@ -241,7 +241,7 @@ k_col_small(const cx<T>* __restrict__ in, cx<T>* __restrict__ out, int KX, T sca
 // the zeta part of the stage for e (comp1.f90:131; the fused stage leaves it
 // to k_e_update), and the x-transform of e (first half of expand,
 // filter_fftw.f90:262-263).  e has levels 0..NZ+1.  Also clears the level's
-// clip flag (when given) for k_clip_x_flag.
+// clip flag (when given) for k_clip_walls.
 template <class T, int NX>
 __global__ void __launch_bounds__(RowCfg<NX>::THREADS)
 k_e_prep(T* __restrict__ e, const T* __restrict__ re, cx<T>* __restrict__ Xe, int NY, int NZ, T dtab2, int zeta,
@@ -715,17 +715,16 @@ __global__ void k_wall_sums(const T* __restrict__ U, const T* __restrict__ V, in
 }
 
 // As k_wall_sums, straight from the mixed rows of u and v (x-spectral, y
-// physical): block (x, side) transforms C::NT rows of U + iV of level 1 or nnz
-// (one complex transform for both) and sums its points, without storing them.
+// physical): block `blk` of `nblk` transforms C::NT rows of U + iV of level 1
+// (side 0) or nnz (one complex transform for both) and sums its points, without
+// storing them.  Part of k_clip_walls, which has blocks of the same shape.
 template <class T, int NSX>
-__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS)
-k_wall_rows(const cx<T>* __restrict__ Um, const cx<T>* __restrict__ Vm, int MY, int NZ, double* part,
-            const cx<T>* __restrict__ tw) {
+__device__ __forceinline__ void wall_rows_block(const cx<T>* __restrict__ Um, const cx<T>* __restrict__ Vm, int side,
+                                                int blk, int nblk, int MY, int NZ, double* part, cx<T>* sm,
+                                                const cx<T>* __restrict__ tw) {
   constexpr int MX = 3 * NSX / 2, KX = NSX / 2;
   using C = RowCfg<MX>;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-  const int side = blockIdx.y, y0 = blockIdx.x * C::NT;
+  const int y0 = blk * C::NT;
   const size_t off = side == 0 ? 0 : (size_t)(NZ - 1) * MY * KX;
   double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   fft_core<MX, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
@@ -744,7 +743,7 @@ k_wall_rows(const cx<T>* __restrict__ Um, const cx<T>* __restrict__ Vm, int MY, 
     const double u = (double)uv.x, v = (double)uv.y, wd = (double)sqrt((T)(uv.x * uv.x + uv.y * uv.y));
     s[0] += u; s[1] += v; s[2] += wd; s[3] += u * u; s[4] += v * v; s[5] += wd * wd; s[6] += wd * u; s[7] += wd * v;
   });
-  block_sum_store<8>(s, part + ((size_t)side * gridDim.x + blockIdx.x) * 8);
+  block_sum_store<8>(s, part + ((size_t)side * nblk + blk) * 8);
 }
 
 // Wall-model scalars for both walls (lowerbc.f90:56-124, upperbc.f90:63-122)
