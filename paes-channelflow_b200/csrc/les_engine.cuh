@@ -277,8 +277,8 @@ struct Engine : EngineBase {
       for (auto& b : flux) b.alloc(pb * NZ);
     }
     divacc.alloc(NZ); sgsacc.alloc((size_t)NZ * 8); wacc.alloc((size_t)2 * std::max<size_t>(kWallBlocks, MY) * 8); acc.alloc((size_t)NZ * 16);
-    // one partial per warp of k_row_fused or per 256-point block of k_flux
-    nstat_parts = (int)cdiv(pb, 256);
+    // one partial per warp of k_row_fused or k_flux
+    nstat_parts = (int)cdiv(pb, kFluxThreads) * (kFluxThreads / 32);
     if (fused)
       with_small(NX, [&](auto cn) {
         using C = FusedCfg<T, decltype(cn)::value>;
@@ -807,21 +807,22 @@ struct Engine : EngineBase {
       constexpr int N = decltype(cn)::value;
       using C = FusedCfg<T, N>;
       if (fused_chunks == 0)
-        fused_chunks = fused_chunk_count((const void*)k_row_fused<T, N>, C::THREADS, C::smem(), MY / C::ROWS);
+        fused_chunks = chunk_count((const void*)k_row_fused<T, N>, C::THREADS, C::smem(), MY / C::ROWS, 0.5);
       fa.zchunk = (int)cdiv(NZ, fused_chunks);
       launch(k_row_fused<T, N>, dim3(MY / C::ROWS, (unsigned)cdiv(NZ, fa.zchunk)), dim3(C::THREADS), C::smem(), st, fa,
              a, tw);
     });
   }
-  // z chunks of the fused kernel: a CTA walks its rows' chunk with a sliding
-  // window, so chunks only add prologues (about half a level of work each),
-  // while the last wave of CTAs leaves SMs idle.  Minimise waves x (levels
-  // per chunk + 1/2) over 1..NZ chunks, the waves counted with the kernel's
+  // z chunks of the fused kernel and k_flux: a CTA walks its chunk with a
+  // sliding window, so chunks only add prologues (half a level of work each in
+  // the fused kernel, the loads of two levels in k_flux), while the last wave
+  // of CTAs leaves SMs idle.  Minimise waves x (levels per chunk + prologue)
+  // over 1..NZ chunks, the waves counted with the kernel's
   // resident CTAs per SM.  A grid that fits one wave is bound by the latency
   // of a CTA's chain of levels, so its chunks shrink to a level or two
   // (32x32x16: 16 chunks instead of the 2 of an 8-level minimum).
-  int fused_chunks = 0;
-  int fused_chunk_count(const void* kernel, int threads, size_t smem, int rows) {
+  int fused_chunks = 0, flux_chunks = 0;
+  int chunk_count(const void* kernel, int threads, size_t smem, int rows, double prologue) {
     if (smem > 48 * 1024) set_smem_limit(kernel, smem);
     int per_sm = 0;
     LES_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
@@ -830,7 +831,7 @@ struct Engine : EngineBase {
     double best_cost = 0.0;
     for (int c = 1; c <= NZ; c++) {
       const int zc = (int)cdiv(NZ, c), n = (int)cdiv(NZ, zc);
-      const double cost = std::ceil((double)rows * n / resident) * (zc + 0.5);
+      const double cost = std::ceil((double)rows * n / resident) * (zc + prologue);
       if (c == 1 || cost < best_cost) { best = c; best_cost = cost; }
     }
     return best;
@@ -867,8 +868,11 @@ struct Engine : EngineBase {
     }
     Ptr11 fl{};
     for (int i = 0; i < 11; i++) fl.p[i] = flux[i].p;
-    launch(k_flux<T>, dim3(cdiv(pb, 256), NZ), dim3(256), 0, st, pd, fl, a, (const WallParams*)wp.p, divpart.p,
-           sgspart.p);
+    const unsigned nblk = cdiv(pb, kFluxThreads);
+    if (flux_chunks == 0) flux_chunks = chunk_count((const void*)k_flux<T>, kFluxThreads, 0, (int)nblk, 2.0);
+    const int zchunk = (int)cdiv(NZ, flux_chunks);
+    launch(k_flux<T>, dim3(nblk, (unsigned)cdiv(NZ, zchunk)), dim3(kFluxThreads), 0, st, pd, fl, a, (const WallParams*)wp.p,
+           divpart.p, sgspart.p, zchunk);
     Ptr8 X{};
     for (int i = 0; i < 8; i++) X.p[i] = mixed[i].p;  // reuse the mixed buffers
     with_small(NX, [&](auto cn) {

@@ -322,3 +322,30 @@ def test_pressure_columns_in_wide_blocks(gpu_lib, product, nx, ny, nz, imodel):
         for k in ("ru", "rv", "rw"):
             assert relerr(tg[k], to_[k], rscale) < 1e-9, k
         assert relerr(fg["p"], fo["p"]) < 1e-9
+
+
+@pytest.mark.parametrize("clipped", [False, True])
+@pytest.mark.parametrize("nx,ny,nz,imodel,tke", [(16, 32, 4, 4, 0), (96, 128, 5, 4, 1), (96, 128, 8, 3, 1), (128, 96, 13, 4, 0)])
+def test_flux_columns_of_the_unfused_stage(gpu_lib, product, nx, ny, nz, imodel, tke, clipped):
+    """k_flux with one level, several levels and a short last chunk per thread
+    (padded planes of 216 point blocks), and the clip kernels with a TKE that
+    they leave alone and one that they raise.  Tolerances of the unclipped stage
+    tests; e in FP64 only (white noise in e rounds to 2e-5 of it in FP32, by the
+    advective term, whichever way the fluxes are computed)."""
+    rng = np.random.default_rng(nx + nz)
+    e = 1e-3 * rng.random((nz, ny, nx)) ** 4 if clipped else 1e-3 * (1.0 + 0.1 * rng.random((nz, ny, nx)))
+    for precision, tol in ((8, 1e-11), (4, 2e-5)):
+        o, g, f = make_pair(product, nx, ny, nz, precision=precision, amp=0.3, imodel=imodel, tke_production=tke)
+        o.set_fields(e=e)
+        o.deal_fields()
+        f = o.get_fields()
+        g.upload(f["u"], f["v"], f["w"], f["e"], f["p"])
+        for s in (1, 2):
+            o.stage(0, 1, s)
+            g.stage(0, True, s)
+        fo, fg = o.get_fields(), g.download()
+        vscale = np.abs(fo["u"]).max()
+        for k in "uvw":
+            assert relerr(fg[k], fo[k], vscale) < tol, (precision, k)
+        if precision == 8:
+            assert relerr(fg["e"], fo["e"]) < tol
