@@ -805,12 +805,12 @@ k_wall_final(const double* __restrict__ part, int nblk, const double* __restrict
     w.utau = w.vsfc * vk / zody;
     if (w.utau > 10.0) atomicOr(err, ERR_UTAU);
     double tep = fmin(fmax(w.u1xy / w.vsfc, -1.0), 1.0);
-    double thta = acos(tep);
     double ut2 = w.utau * w.utau;
     double sg = copysign(1.0, w.v1xy);
     double sgn_wall = side ? 1.0 : -1.0;
-    w.auuwm = sgn_wall * ut2 * cos(thta);
-    w.auvwm = sgn_wall * ut2 * sin(thta) * sg;
+    // theta = acos(tep): cos(theta) = tep, sin(theta) >= 0
+    w.auuwm = sgn_wall * ut2 * tep;
+    w.auvwm = sgn_wall * ut2 * sqrt((1.0 - tep) * (1.0 + tep)) * sg;
     // fluctuation moments: ufluc = U + ugal - u1xy = U - cu
     double cu = w.u1xy - a.ugal, cv = w.v1xy - a.vgal;
     double Suu = s[3] - 2 * cu * s[0] + P * cu * cu;
