@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <cmath>
+#include <type_traits>
 
 namespace les {
 
@@ -372,8 +373,9 @@ __device__ __forceinline__ void smem_fft(int ntrans, cx<T>* sm, const cx<T>* __r
 // General four-step transform of `ntrans` sequences with one shared-memory
 // transpose.  Input comes from global memory through load(t, n) (pass A
 // issues N1 independent loads per thread before any arithmetic) or, with
-// IN_SMEM, from `sm` in natural layout; output goes to store(t, k, v) or,
-// with OUT_SMEM, back to `sm` in natural layout.
+// IN_SMEM, from `sm` in natural layout (through load(n, v), unless NoLoad);
+// output goes to store(t, k, v) or, with OUT_SMEM, back to `sm` in natural
+// layout.
 //   natural layout: rows  sm[t*N + n];  cols (COLS) sm[n*ntrans + t]
 // Requires blockDim.x >= ntrans*N2 and smem_fft_elems<N, COLS>(ntrans)
 // elements; every thread of the block must call it.  Ends with a
@@ -391,13 +393,25 @@ __device__ __forceinline__ void fft_core_tab(int ntrans, cx<T>* sm, const cx<T>*
     int t = 0, n2 = 0;
     if (COLS) { t = it % ntrans; n2 = it / ntrans; }
     else { t = it / N2; n2 = it - t * N2; }
-    cx<T> v[N1];
+    // Short first passes of rows ask for their twiddles with the data, not after
+    // it; longer ones and columns would pay with resident blocks (up to 256 bytes
+    // and columns too: k_clipd_y of 288 points FP64 155 -> 274 us).
+    constexpr bool EARLY = !COLS && N1 * sizeof(cx<T>) <= 128;
+    cx<T> v[N1], we[EARLY ? N1 : 1];
     if (active) {
+      if constexpr (EARLY) {
+#pragma unroll
+        for (int k1 = 1; k1 < N1; k1++) we[k1] = twn[n2 * k1];
+      }
 #pragma unroll
       for (int n1 = 0; n1 < N1; n1++) {
         const int n = n2 + N2 * n1;
-        if constexpr (IN_SMEM) v[n1] = COLS ? sm[n * ntrans + t] : sm[t * N + n];
-        else v[n1] = load(t, n);
+        if constexpr (IN_SMEM) {
+          v[n1] = COLS ? sm[n * ntrans + t] : sm[t * N + n];
+          if constexpr (std::is_invocable_v<LoadF, int, cx<T>>) v[n1] = load(n, v[n1]);
+        } else {
+          v[n1] = load(t, n);
+        }
       }
     }
     if (IN_SMEM) __syncthreads();
@@ -405,7 +419,7 @@ __device__ __forceinline__ void fft_core_tab(int ntrans, cx<T>* sm, const cx<T>*
       Dft<N1, S, T>::run(v);
 #pragma unroll
       for (int k1 = 0; k1 < N1; k1++) {
-        cx<T> w = twn[n2 * k1];
+        cx<T> w = k1 == 0 ? zero_cx<T>() : EARLY ? we[EARLY ? k1 : 0] : twn[n2 * k1];
         if (S > 0) w.y = -w.y;
         cx<T> r = (k1 == 0) ? v[k1] : cmul(v[k1], w);
         if (COLS) sm[(k1 * N2 + n2) * ntrans + t] = r;
@@ -456,9 +470,7 @@ __device__ __forceinline__ const cx<T>* stage_twiddles(cx<T>* dst, const cx<T>* 
   __syncthreads();
   return dst;
 }
-struct NoLoad {
-  __device__ int operator()(int, int) const { return 0; }
-};
+struct NoLoad {};
 struct NoStore {
   template <class V> __device__ void operator()(int, int, V) const {}
 };

@@ -507,7 +507,7 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
 // The first four block rows sum the wall rows, two block rows a side: a launch
 // less (a 32x32x16 FP64 stage 79.5 -> 74.0 us, 64x64x64 135 -> 126).
 template <class T, int NSX>
-__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS, sizeof(T) == 8 ? 3 : 1)
+__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS, sizeof(T) == 8 ? 3 : 4)
 k_clip_walls(const cx<T>* __restrict__ Em, T* __restrict__ E, T* __restrict__ dEX, int* __restrict__ flags,
              unsigned char* __restrict__ rowclip, const cx<T>* __restrict__ Um, const cx<T>* __restrict__ Vm,
              double* __restrict__ wpart, int nwall, int MY, int NZ, T emin, T kx0, const cx<T>* __restrict__ tw) {
@@ -524,17 +524,11 @@ k_clip_walls(const cx<T>* __restrict__ Em, T* __restrict__ E, T* __restrict__ dE
   const int z = (int)blockIdx.y - 3;
   const int p0 = blockIdx.x * C::NT, np = MY / 2;
   const cx<T>* in = Em + (size_t)(z - 1) * MY * KX;
-  auto load = [&](int t, int n) {
-    const int p = p0 + t;
-    int k = -1;
-    bool mir = false;
-    if (n < KX) k = n;
-    else if (n > MX - KX) { k = MX - n; mir = true; }
-    if (p >= np || k < 0) return zero_cx<T>();
-    cx<T> av = in[(size_t)(2 * p) * KX + k], bv = in[(size_t)(2 * p + 1) * KX + k];
-    if (k == 0) { av.y = 0; bv.y = 0; }
-    if (mir) { av = conj(av); bv = conj(bv); }
-    return mk(av.x - bv.y, av.y + bv.x);
+  const int pl = p0 + (int)(threadIdx.x / Split<MX>::N2);  // the pair this thread loads
+  const cx<T>* ra = in + (size_t)(2 * (pl < np ? pl : p0)) * KX;
+  auto load = [&](int, int n) {
+    const PairMode m = pair_mode<MX>(n, KX);
+    return m.join(ra[m.k], ra[KX + m.k]);
   };
   bool below = false;
   fft_core<MX, +1, false, false, false>(C::NT, sm, tw, load, [&](int t, int, cx<T> v) {
@@ -559,13 +553,7 @@ k_clip_walls(const cx<T>* __restrict__ Em, T* __restrict__ E, T* __restrict__ dE
   }
   __syncthreads();
   fft_core<MX, -1, false, true, true>(C::NT, sm, tw, NoLoad{}, NoStore{});
-  for (int i = threadIdx.x; i < C::NT * MX; i += C::THREADS) {
-    const int k = i % MX;
-    const T kk = (k == 0 || 2 * k == MX) ? (T)0 : kx0 * (T)signed_k(k, MX) / (T)MX;
-    sm[i] = mul_i(sm[i]) * kk;
-  }
-  __syncthreads();
-  fft_core<MX, +1, false, true, false>(C::NT, sm, tw, NoLoad{}, [&](int t, int n, cx<T> d) {
+  fft_core<MX, +1, false, true, false>(C::NT, sm, tw, Derivative<T, MX>(kx0), [&](int t, int n, cx<T> d) {
     const int p = p0 + t;
     if (p >= np) return;
     dEX[zoff + (size_t)(2 * p) * MX + n] = d.x;
@@ -601,14 +589,8 @@ k_clipd_y(const T* __restrict__ E, T* __restrict__ dEY, const int* __restrict__ 
     }
     return v;
   }, NoStore{});
-  for (int i = threadIdx.x; i < C::TC * M; i += blockDim.x) {
-    int t = i % C::TC, k = i / C::TC;
-    T kk = (k == 0 || 2 * k == M) ? (T)0 : ky0 * (T)signed_k(k, M) / (T)M;
-    sm[k * C::TC + t] = mul_i(sm[k * C::TC + t]) * kk;
-  }
-  __syncthreads();
   cx<T>* out = reinterpret_cast<cx<T>*>(dEY + zoff);
-  fft_core<M, +1, true, true, false>(C::TC, sm, tw, NoLoad{}, [&](int t, int n, cx<T> d) {
+  fft_core<M, +1, true, true, false>(C::TC, sm, tw, Derivative<T, M>(ky0), [&](int t, int n, cx<T> d) {
     int c = c0 + t;
     if (c < ncp) out[(size_t)n * ncp + c] = d;
   });

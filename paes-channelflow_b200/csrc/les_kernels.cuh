@@ -79,6 +79,37 @@ constexpr int ERR_NAN = 1, ERR_UTAU = 2;
 template <class T> __device__ __forceinline__ T tmax(T a, T b) { return a > b ? a : b; }
 template <class T> __device__ __forceinline__ T tmin(T a, T b) { return a < b ? a : b; }
 
+// Element n of the length-N sequence A + iB of two real rows, from the K <= N/2 + 1
+// modes of A and B that are kept (the others are zero, the imaginary parts of
+// modes 0 and N/2 ignored): the mode to read, and what to make of it.  The loads
+// need no branch, so a thread's go out together; behind branches they were a chain
+// (expand of 384x384x64 FP64 230 -> 215 us, k_e_update of 512x512x64 147 -> 123,
+// k_clip_walls 110 -> 90).
+struct PairMode {
+  int k;
+  bool mirror, zero, real;
+  template <class T> __device__ __forceinline__ cx<T> join(cx<T> a, cx<T> b) const {
+    if (real) a.y = b.y = (T)0;
+    const cx<T> v = mirror ? mk(a.x + b.y, b.x - a.y) : mk(a.x - b.y, a.y + b.x);
+    return zero ? zero_cx<T>() : v;
+  }
+};
+template <int N> __device__ __forceinline__ PairMode pair_mode(int n, int K) {
+  const bool direct = n < K, mirror = !direct && N - n < K;
+  const int k = direct ? n : mirror ? N - n : 0;
+  return {k, mirror, !direct && !mirror, k == 0 || 2 * k == N};
+}
+// d/dx of a transformed row or column, with the 1/N of the inverse transform
+// (the Nyquist mode dropped), at the inverse transform's loads: a pass over shared
+// memory, a barrier and a division per mode less (384x384x64 FP64: k_op_xderiv 139
+// -> 125 us, k_op_yderiv 205 -> 130).
+template <class T, int N> struct Derivative {
+  T k1;
+  __device__ __forceinline__ explicit Derivative(T k0) : k1(k0 / (T)N) {}
+  __device__ __forceinline__ cx<T> operator()(int k, cx<T> v) const {
+    return (k == 0 || 2 * k == N) ? zero_cx<T>() : mul_i(v) * (k1 * (T)signed_k(k, N));
+  }
+};
 // ---------------------------------------------------------------------------
 // Generic small-grid transforms (upload, download, deal, expand, compress)
 // ---------------------------------------------------------------------------
@@ -93,6 +124,7 @@ k_row_r2c(const T* __restrict__ in, cx<T>* __restrict__ out, int nrows, int KOUT
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
   const int p0 = blockIdx.x * C::NT;
   const int npair = (nrows + 1) / 2;
+  if (p0 >= npair) return;
   fft_core<N, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
     int p = p0 + t;
     cx<T> v = zero_cx<T>();
@@ -120,25 +152,13 @@ k_row_c2r(const cx<T>* __restrict__ in, T* __restrict__ out, int nrows, int KIN,
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
   const int p0 = blockIdx.x * C::NT;
   const int npair = (nrows + 1) / 2;
-  fft_core<N, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
-    int p = p0 + t;
-    cx<T> v = zero_cx<T>();
-    if (p < npair) {
-      int k = n;
-      bool mir = false;
-      if (k >= KIN) {
-        if (N - k < KIN && N - k > 0 && N - k != N / 2) { k = N - k; mir = true; }
-        else k = -1;
-      }
-      if (k >= 0) {
-        cx<T> a = in[(size_t)(2 * p) * KIN + k];
-        cx<T> b = (2 * p + 1 < nrows) ? in[(size_t)(2 * p + 1) * KIN + k] : zero_cx<T>();
-        if (k == 0 || (2 * k == N)) { a.y = 0; b.y = 0; }
-        if (mir) { a = conj(a); b = conj(b); }
-        v = mk(a.x - b.y, a.y + b.x);
-      }
-    }
-    return v;
+  if (p0 >= npair) return;
+  const int row = 2 * (p0 + (int)(threadIdx.x / Split<N>::N2));  // of the transform this thread loads
+  const cx<T>* ra = in + (size_t)(row < nrows ? row : 2 * p0) * KIN;
+  const bool two = row + 1 < nrows;
+  fft_core<N, +1, false, false, false>(C::NT, sm, tw, [&](int, int n) {
+    const PairMode m = pair_mode<N>(n, KIN);
+    return m.join(ra[m.k], two ? ra[KIN + m.k] : zero_cx<T>());
   }, [&](int t, int n, cx<T> v) {
     int p = p0 + t;
     if (p >= npair) return;
@@ -166,6 +186,7 @@ k_op_row_r2c(const T* in, cx<T>* out, int nrows, int K, RowLayout lo, const cx<T
   extern __shared__ __align__(16) unsigned char smraw[];
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
   const int p0 = blockIdx.x * C::NT, npair = (nrows + 1) / 2;
+  if (p0 >= npair) return;
   fft_core<N, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
     const int p = p0 + t;
     if (p >= npair) return zero_cx<T>();
@@ -187,21 +208,14 @@ k_op_row_c2r(const cx<T>* in, T* out, int nrows, int K, RowLayout li, const cx<T
   extern __shared__ __align__(16) unsigned char smraw[];
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
   const int p0 = blockIdx.x * C::NT, npair = (nrows + 1) / 2;
+  if (p0 >= npair) return;
   const int row = 2 * (p0 + (int)(threadIdx.x / Split<N>::N2));  // of the transform this thread loads
-  const long long ra = row < nrows ? li.at(row) : 0, rb = row + 1 < nrows ? li.at(row + 1) : 0;
-  fft_core<N, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
-    const int p = p0 + t;
-    int k = n;
-    bool mir = false;
-    if (k >= K) {
-      if (N - k < K && N - k > 0) { k = N - k; mir = true; }
-      else k = -1;
-    }
-    if (p >= npair || k < 0) return zero_cx<T>();
-    cx<T> a = in[ra + k], b = (2 * p + 1 < nrows) ? in[rb + k] : zero_cx<T>();
-    if (k == 0) { a.y = 0; b.y = 0; }
-    if (mir) { a = conj(a); b = conj(b); }
-    return mk(a.x - b.y, a.y + b.x);
+  const cx<T>* ra = in + li.at(row < nrows ? row : 2 * p0);
+  const bool two = row + 1 < nrows;
+  const cx<T>* rb = two ? in + li.at(row + 1) : ra;
+  fft_core<N, +1, false, false, false>(C::NT, sm, tw, [&](int, int n) {
+    const PairMode m = pair_mode<N>(n, K);
+    return m.join(ra[m.k], two ? rb[m.k] : zero_cx<T>());
   }, [&](int t, int n, cx<T> v) {
     const int p = p0 + t;
     if (p >= npair) return;
@@ -554,25 +568,15 @@ k_x_inverse(const __grid_constant__ Ptr8 src, const __grid_constant__ Ptr12 dst,
   const int y0 = blockIdx.x * C::NT;
   T* outA = reinterpret_cast<T*>(dst.p[oA[g]]) + zoff * MX;
   T* outB = reinterpret_cast<T*>(dst.p[oB[g]]) + zoff * MX;
-  fft_core<MX, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
-    int y = y0 + t;
-    cx<T> v = zero_cx<T>();
-    if (y < MY) {
-      int k = -1;
-      bool mir = false;
-      if (n < KX) k = n;
-      else if (n > MX - KX) { k = MX - n; mir = true; }
-      if (k >= 0) {
-        cx<T> a = A[(size_t)y * KX + k], b = B[(size_t)y * KX + k];
-        T kk = kx0 * (T)k;
-        if (ma) a = mul_i(a) * kk;
-        if (mb) b = mul_i(b) * kk;
-        if (k == 0) { a.y = 0; b.y = 0; }
-        if (mir) { a = conj(a); b = conj(b); }
-        v = mk(a.x - b.y, a.y + b.x);
-      }
-    }
-    return v;
+  const int yl = y0 + (int)(threadIdx.x / Split<MX>::N2);  // the row this thread loads
+  const size_t ro = (size_t)(yl < MY ? yl : y0) * KX;
+  fft_core<MX, +1, false, false, false>(C::NT, sm, tw, [&](int, int n) {
+    const PairMode m = pair_mode<MX>(n, KX);
+    cx<T> a = A[ro + m.k], b = B[ro + m.k];
+    const T kk = kx0 * (T)m.k;
+    if (ma) a = mul_i(a) * kk;
+    if (mb) b = mul_i(b) * kk;
+    return m.join(a, b);
   }, [&](int t, int n, cx<T> v) {
     int y = y0 + t;
     if (y >= MY) return;
@@ -613,14 +617,8 @@ k_clip_y(const T* __restrict__ E, T* __restrict__ EY, int MX, T emin, T ky0, con
     }
     return v;
   }, NoStore{});
-  for (int i = threadIdx.x; i < C::TC * M; i += blockDim.x) {
-    int t = i % C::TC, k = i / C::TC;
-    T kk = (k == 0 || 2 * k == M) ? (T)0 : ky0 * (T)signed_k(k, M) / (T)M;
-    sm[k * C::TC + t] = mul_i(sm[k * C::TC + t]) * kk;
-  }
-  __syncthreads();
   cx<T>* EYz = reinterpret_cast<cx<T>*>(EY + zoff);
-  fft_core<M, +1, true, true, false>(C::TC, sm, tw, NoLoad{}, [&](int t, int n, cx<T> d) {
+  fft_core<M, +1, true, true, false>(C::TC, sm, tw, Derivative<T, M>(ky0), [&](int t, int n, cx<T> d) {
     int c = c0 + t;
     if (c >= ncp) return;
     cx<T> o = EYz[(size_t)n * ncp + c];
@@ -653,13 +651,7 @@ k_clip_x(T* __restrict__ E, T* __restrict__ EX, int MY, T emin, T kx0, const cx<
     }
     return v;
   }, NoStore{});
-  for (int i = threadIdx.x; i < C::NT * MX; i += blockDim.x) {
-    int t = i / MX, k = i - t * MX;
-    T kk = (k == 0 || 2 * k == MX) ? (T)0 : kx0 * (T)signed_k(k, MX) / (T)MX;
-    sm[t * MX + k] = mul_i(sm[t * MX + k]) * kk;
-  }
-  __syncthreads();
-  fft_core<MX, +1, false, true, false>(C::NT, sm, tw, NoLoad{}, [&](int t, int n, cx<T> d) {
+  fft_core<MX, +1, false, true, false>(C::NT, sm, tw, Derivative<T, MX>(kx0), [&](int t, int n, cx<T> d) {
     int p = p0 + t;
     if (p >= np) return;
 #pragma unroll
@@ -741,17 +733,11 @@ __device__ __forceinline__ void wall_rows_block(const cx<T>* __restrict__ Um, co
   const int y0 = blk * C::NT;
   const size_t off = side == 0 ? 0 : (size_t)(NZ - 1) * MY * KX;
   double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  fft_core<MX, +1, false, false, false>(C::NT, sm, tw, [&](int t, int n) {
-    const int y = y0 + t;
-    int k = -1;
-    bool mir = false;
-    if (n < KX) k = n;
-    else if (n > MX - KX) { k = MX - n; mir = true; }
-    if (y >= MY || k < 0) return zero_cx<T>();
-    cx<T> av = Um[off + (size_t)y * KX + k], bv = Vm[off + (size_t)y * KX + k];
-    if (k == 0) { av.y = 0; bv.y = 0; }
-    if (mir) { av = conj(av); bv = conj(bv); }
-    return mk(av.x - bv.y, av.y + bv.x);
+  const int yl = y0 + (int)(threadIdx.x / Split<MX>::N2);  // the row this thread loads
+  const size_t ro = off + (size_t)(yl < MY ? yl : y0) * KX;
+  fft_core<MX, +1, false, false, false>(C::NT, sm, tw, [&](int, int n) {
+    const PairMode m = pair_mode<MX>(n, KX);
+    return m.join(Um[ro + m.k], Vm[ro + m.k]);
   }, [&](int t, int, cx<T> uv) {
     if (y0 + t >= MY) return;
     const double u = (double)uv.x, v = (double)uv.y, wd = (double)sqrt((T)(uv.x * uv.x + uv.y * uv.y));
@@ -1058,10 +1044,10 @@ k_x_forward(const __grid_constant__ Ptr11 in, const __grid_constant__ Ptr8 out, 
   const T* A = (const T*)in.p[sA[g]] + zoff * MX;
   const T* B = sB[g] >= 0 ? (const T*)in.p[sB[g]] + zoff * MX : nullptr;
   const int y0 = blockIdx.x * C::NT;
-  fft_core<MX, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
-    int y = y0 + t;
-    return (y < MY) ? mk(A[(size_t)y * MX + n], B ? B[(size_t)y * MX + n] : (T)0) : zero_cx<T>();
-  }, NoStore{});
+  const int yl = y0 + (int)(threadIdx.x / Split<MX>::N2);  // the row this thread loads
+  const size_t ro = (size_t)(yl < MY ? yl : y0) * MX;
+  fft_core<MX, -1, false, false, true>(C::NT, sm, tw, [&](int, int n) { return mk(A[ro + n], B ? B[ro + n] : (T)0); },
+                                       NoStore{});
   auto O = [&](int j) { return (cx<T>*)out.p[j] + zoff * KX; };
   for (int i = threadIdx.x; i < C::NT * KX; i += blockDim.x) {
     int t = i / KX, k = i - t * KX, y = y0 + t;
@@ -1233,17 +1219,11 @@ k_e_update(const cx<T>* __restrict__ rem, T* __restrict__ re, T* __restrict__ e,
   extern __shared__ __align__(16) unsigned char smraw[];
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
   const int p0 = blockIdx.x * C::NT, np = nrows / 2;
-  fft_core<NX, +1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
-    const int p = p0 + t;
-    int k = -1;
-    bool mir = false;
-    if (n < KX) k = n;
-    else if (n > KX) { k = NX - n; mir = true; }
-    if (p >= np || k < 0) return zero_cx<T>();
-    cx<T> a = rem[(size_t)(2 * p) * KX + k], b = rem[(size_t)(2 * p + 1) * KX + k];
-    if (k == 0) { a.y = 0; b.y = 0; }
-    if (mir) { a = conj(a); b = conj(b); }
-    return mk(a.x - b.y, a.y + b.x);
+  const int pl = p0 + (int)(threadIdx.x / Split<NX>::N2);  // the pair this thread loads
+  const cx<T>* ra = rem + (size_t)(2 * (pl < np ? pl : p0)) * KX;
+  fft_core<NX, +1, false, false, true>(C::NT, sm, tw, [&](int, int n) {
+    const PairMode m = pair_mode<NX>(n, KX);
+    return m.join(ra[m.k], ra[KX + m.k]);
   }, NoStore{});
   struct alignas(4 * sizeof(T)) V4 { T v[4]; };
   constexpr int ITEMS = C::NT * NX / 4;
@@ -1746,18 +1726,13 @@ k_op_xderiv(const T* __restrict__ in, T* __restrict__ out, int nrows, T k0, cons
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
   const int p0 = blockIdx.x * C::NT;
   const int npair = (nrows + 1) / 2;
+  if (p0 >= npair) return;
   fft_core<N, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
     int p = p0 + t;
     return (p < npair) ? mk(in[(size_t)(2 * p) * N + n], (2 * p + 1 < nrows) ? in[(size_t)(2 * p + 1) * N + n] : (T)0)
                        : zero_cx<T>();
   }, NoStore{});
-  for (int i = threadIdx.x; i < C::NT * N; i += blockDim.x) {
-    int t = i / N, k = i - t * N;
-    T kk = (k == 0 || 2 * k == N) ? (T)0 : k0 * (T)signed_k(k, N) / (T)N;
-    sm[t * N + k] = mul_i(sm[t * N + k]) * kk;
-  }
-  __syncthreads();
-  fft_core<N, +1, false, true, false>(C::NT, sm, tw, NoLoad{}, [&](int t, int n, cx<T> v) {
+  fft_core<N, +1, false, true, false>(C::NT, sm, tw, Derivative<T, N>(k0), [&](int t, int n, cx<T> v) {
     int p = p0 + t;
     if (p >= npair) return;
     out[(size_t)(2 * p) * N + n] = v.x;
@@ -1772,18 +1747,15 @@ k_op_yderiv(const T* __restrict__ in, T* __restrict__ out, int n1, T k0, const c
   cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
   const size_t plane = (size_t)blockIdx.y * N * n1;
   const int ncp = (n1 + 1) / 2, c0 = blockIdx.x * C::TC;
-  fft_core<N, -1, true, false, true>(C::TC, sm, tw, [&](int t, int n) {
-    int c = c0 + t;
-    return (c < ncp) ? mk(in[plane + (size_t)n * n1 + 2 * c], (2 * c + 1 < n1) ? in[plane + (size_t)n * n1 + 2 * c + 1] : (T)0)
-                     : zero_cx<T>();
+  const int cl = c0 + (int)(threadIdx.x % C::TC);  // the column pair this thread loads
+  const T* col = in + plane + 2 * (cl < ncp ? cl : c0);
+  const int second = 2 * (cl < ncp ? cl : c0) + 1 < n1 ? 1 : 0;
+  fft_core<N, -1, true, false, true>(C::TC, sm, tw, [&](int, int n) {
+    const T* r = col + (size_t)n * n1;
+    const T b = r[second];
+    return mk(r[0], second ? b : (T)0);
   }, NoStore{});
-  for (int i = threadIdx.x; i < C::TC * N; i += blockDim.x) {
-    int t = i % C::TC, k = i / C::TC;
-    T kk = (k == 0 || 2 * k == N) ? (T)0 : k0 * (T)signed_k(k, N) / (T)N;
-    sm[k * C::TC + t] = mul_i(sm[k * C::TC + t]) * kk;
-  }
-  __syncthreads();
-  fft_core<N, +1, true, true, false>(C::TC, sm, tw, NoLoad{}, [&](int t, int n, cx<T> v) {
+  fft_core<N, +1, true, true, false>(C::TC, sm, tw, Derivative<T, N>(k0), [&](int t, int n, cx<T> v) {
     int c = c0 + t;
     if (c >= ncp) return;
     out[plane + (size_t)n * n1 + 2 * c] = v.x;
