@@ -171,7 +171,8 @@ def algorithmic_bytes(kernel, nx, ny, nz, tb, learned=False):
         "k_clip_x": Lw * pad * 4,
         "k_e_prep": Lw * (3 * small + spec),
         "k_e_update": Lw * (spec + 3 * small),
-        "k_press": nz * (9 * spec + 2 * 24 * nm + 16 * nm),
+        # solve with the velocity update: 9 spectra read, 6 and p written
+        "k_press": nz * (15 * spec + 16 * nm),
         "k_update": nz * (15 * spec + 16 * nm),
         # fused row kernel: reads the 8 mixed inputs, writes the 8 mixed outputs
         "k_row_fused": ((3 * L + 3 * Lw) if learned else (4 * L + 4 * Lw)) * mix + (4 * L + 4 * Lw) * mix,

@@ -13,18 +13,20 @@
 //   "padded" arrays   physical                [z][y][x]
 //
 // One stage (les.F90:254-285) is:
-//   k_e_prep, k_col_fwd_small   e ghosts + zeta update + spectrum of e
+//   k_e_prep                    e ghosts, x spectrum of e
 //   k_y_inverse, k_x_inverse    expand() of u, v, w, e fused with the
 //                               spectral derivatives ux..ey (derivs1/2)
 //   k_clip_y, k_clip_x          derivatives of max(E, emin) - E
-//   k_wall_sums/final           plane means for sufsim / sufsim_upper
+//   k_wall_sums, k_wall_final   plane means for sufsim / sufsim_upper
 //   k_flux                      compadv1, complen, compsgs1, compsgs3
 //                               pointwise, written as flux fields
 //   k_x_forward, k_y_forward    compress() fused with -d/dx, -d/dy of the
-//                               fluxes; the e part also inverts re
+//                               fluxes; the e part also inverts re in y
 //   k_e_update                  e = max(e + dtab1*re, emin)
 //   k_press                     comprhs + press (tridv) per (kx, ky) and
 //                               comp2 in spectral space, FP64
+// The x kernels, the clip kernels, k_wall_sums and k_flux are the unfused
+// middle (Smagorinsky, shear production); les_fused.cuh holds the fused one.
 #pragma once
 #include "fft_core.cuh"
 #include "fft_inplace.cuh"
