@@ -169,8 +169,8 @@ def algorithmic_bytes(kernel, nx, ny, nz, tb, learned=False):
         "k_y_forward": (4 * L + 4 * Lw) * mix + (2 * L + Lw) * spec + Lw * spec,
         "k_clip_y": Lw * pad * 2,
         "k_clip_x": Lw * pad * 4,
-        "k_e_prep": Lw * (3 * small + spec),
-        "k_e_update": Lw * (spec + 3 * small),
+        "k_e_prep": Lw * (small + spec),
+        "k_e_update": Lw * (spec + 4 * small),
         # solve with the velocity update: 9 spectra read, 6 and p written
         "k_press": nz * (15 * spec + 16 * nm),
         "k_update": nz * (15 * spec + 16 * nm),
