@@ -786,7 +786,7 @@ struct Engine : EngineBase {
       nwall = (int)cdiv(MY, C::NT);
       // clip flags and corrections of max(expand(e), emin), and the wall-model
       // sums of U, V at levels 1 and nnz
-      launch(k_clip_walls<T, N>, dim3(cdiv(MY / 2, C::NT), NZ - 1 + 4), dim3(C::THREADS), C::template smem<T>(), st,
+      launch(k_clip_walls<T, N>, dim3(cdiv(MY / 2, C::NT), NZ - 1 + 4), dim3(C::SUM_THREADS), C::template smem<T>(), st,
              (const cx<T>*)mixed[6].p, ephys.p, dEX.p, clipflag.p, rowclip.p, (const cx<T>*)mixed[0].p,
              (const cx<T>*)mixed[2].p, wacc.p, nwall, MY, NZ, (T)cfg.emin, (T)kx0, tw);
     });

@@ -509,7 +509,7 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
 // Registers: 168 (FP64) and 128 (FP32); unbounded, the 768-point FP32 rows take 190
 // and an unclipped 512x512x64 launch 66 us instead of 47.
 template <class T, int NSX>
-__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS, sizeof(T) == 8 ? 3 : 4)
+__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::SUM_THREADS, sizeof(T) == 8 ? 3 : 4)
 k_clip_walls(const cx<T>* __restrict__ Em, T* __restrict__ E, T* __restrict__ dEX, int* __restrict__ flags,
              unsigned char* __restrict__ rowclip, const cx<T>* __restrict__ Um, const cx<T>* __restrict__ Vm,
              double* __restrict__ wpart, int nwall, int MY, int NZ, T emin, T kx0, const cx<T>* __restrict__ tw) {
@@ -544,7 +544,7 @@ k_clip_walls(const cx<T>* __restrict__ Em, T* __restrict__ E, T* __restrict__ dE
   if (!any) return;
   fft_core<MX, +1, false, false, true>(C::NT, sm, tw, load, NoStore{});
   const size_t zoff = (size_t)(z - 1) * MY * MX;
-  for (int i = threadIdx.x; i < C::NT * MX; i += C::THREADS) {
+  for (int i = threadIdx.x; i < C::NT * MX; i += C::SUM_THREADS) {
     const int t = i / MX, n = i - t * MX, p = p0 + t;
     const cx<T> v = sm[i];
     if (p < np) {

@@ -41,6 +41,8 @@ template <int N> struct RowCfg {
   static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
   static constexpr int NT = (128 / N2) > 0 ? (128 / N2) : 1;  // row transforms per CTA
   static constexpr int THREADS = NT * N2;
+  // THREADS rounded up to whole warps, for a kernel that also sums over its block
+  static constexpr int SUM_THREADS = (THREADS + 31) / 32 * 32;
   template <class T> static constexpr size_t smem() { return (size_t)smem_fft_elems<N, false>(NT) * sizeof(cx<T>); }
 };
 template <int N, class T> struct ColCfg {
@@ -667,8 +669,11 @@ k_clip_x(T* __restrict__ E, T* __restrict__ EX, int MY, T emin, T kx0, const cx<
 
 // Block-wide sum of NV doubles per thread, written (not accumulated) to
 // out[q] by thread 0: a fixed reduction order, so results are reproducible.
-template <int NV>
+// The block has THREADS threads, whole warps: a shuffle from a lane that does
+// not exist has no defined value.
+template <int NV, int THREADS>
 __device__ __forceinline__ void block_sum_store(double (&v)[NV], double* out) {
+  static_assert(THREADS % 32 == 0 && THREADS <= 1024, "the shuffles name every lane of every warp");
   __shared__ double red[32][NV];
 #pragma unroll
   for (int q = 0; q < NV; q++)
@@ -679,7 +684,7 @@ __device__ __forceinline__ void block_sum_store(double (&v)[NV], double* out) {
     for (int q = 0; q < NV; q++) red[warp][q] = v[q];
   __syncthreads();
   if (warp == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
+    constexpr int nw = THREADS / 32;
 #pragma unroll
     for (int q = 0; q < NV; q++) {
       double s = (lane < nw) ? red[lane][q] : 0.0;
@@ -701,7 +706,7 @@ static __global__ void __launch_bounds__(256) k_sum_parts(const double* __restri
     for (int q = 0; q < 8; q++)
       if (q < nq) s[q] += part[(z * nparts + p) * nq + q];
   double t[8];
-  block_sum_store<8>(s, t);
+  block_sum_store<8, 256>(s, t);
   if (threadIdx.x == 0)
     for (int q = 0; q < nq; q++) out[z * ostride + q] = t[q];
 }
@@ -710,7 +715,7 @@ static __global__ void __launch_bounds__(256) k_sum_parts(const double* __restri
 // (blockIdx.y = 1): sum U, V, wind, U^2, V^2, wind^2, wind*U, wind*V, one
 // partial per block in part[side][block][8] (summed in order by k_wall_final).
 template <class T>
-__global__ void k_wall_sums(const T* __restrict__ U, const T* __restrict__ V, int NZ, size_t P, double* part) {
+__global__ void __launch_bounds__(256) k_wall_sums(const T* __restrict__ U, const T* __restrict__ V, int NZ, size_t P, double* part) {
   const int side = blockIdx.y;
   const size_t off = side == 0 ? 0 : (size_t)(NZ - 1) * P;
   double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -719,13 +724,15 @@ __global__ void k_wall_sums(const T* __restrict__ U, const T* __restrict__ V, in
     double wd = (double)sqrt((T)(U[off + i] * U[off + i] + V[off + i] * V[off + i]));
     s[0] += u; s[1] += v; s[2] += wd; s[3] += u * u; s[4] += v * v; s[5] += wd * wd; s[6] += wd * u; s[7] += wd * v;
   }
-  block_sum_store<8>(s, part + ((size_t)side * gridDim.x + blockIdx.x) * 8);
+  block_sum_store<8, 256>(s, part + ((size_t)side * gridDim.x + blockIdx.x) * 8);
 }
 
 // As k_wall_sums, straight from the mixed rows of u and v (x-spectral, y
 // physical): block `blk` of `nblk` transforms C::NT rows of U + iV of level 1
 // (side 0) or nnz (one complex transform for both) and sums its points, without
-// storing them.  Part of k_clip_walls, which has blocks of the same shape.
+// storing them.  Part of k_clip_walls, which has blocks of the same shape; the
+// threads that fill the last warp (THREADS is 126 or 120 at six of the nine
+// lengths) transform nothing and add zeros.
 template <class T, int NSX>
 __device__ __forceinline__ void wall_rows_block(const cx<T>* __restrict__ Um, const cx<T>* __restrict__ Vm, int side,
                                                 int blk, int nblk, int MY, int NZ, double* part, cx<T>* sm,
@@ -745,7 +752,7 @@ __device__ __forceinline__ void wall_rows_block(const cx<T>* __restrict__ Um, co
     const double u = (double)uv.x, v = (double)uv.y, wd = (double)sqrt((T)(uv.x * uv.x + uv.y * uv.y));
     s[0] += u; s[1] += v; s[2] += wd; s[3] += u * u; s[4] += v * v; s[5] += wd * wd; s[6] += wd * u; s[7] += wd * v;
   });
-  block_sum_store<8>(s, part + ((size_t)side * nblk + blk) * 8);
+  block_sum_store<8, C::SUM_THREADS>(s, part + ((size_t)side * nblk + blk) * 8);
 }
 
 // Wall-model scalars for both walls (lowerbc.f90:56-124, upperbc.f90:63-122)
@@ -1649,7 +1656,7 @@ __global__ void __launch_bounds__(1024) k_plane_sums(const T* __restrict__ f0, c
     if (f2) s[2] += (double)f2[off + i];
     if (f3) s[3] += (double)f3[off + i];
   }
-  block_sum_store<4>(s, acc + (size_t)blockIdx.y * 8);
+  block_sum_store<4, 1024>(s, acc + (size_t)blockIdx.y * 8);
 }
 
 // Moments of compmn (compmn.F90:29-62) at level iz = blockIdx.y + 1:
@@ -1674,7 +1681,7 @@ __global__ void __launch_bounds__(1024) k_moments(const T* __restrict__ u, const
     s[0] += (double)(ul * ul); s[1] += (double)(vl * vl); s[2] += (double)(w0 * w0);
     s[3] += (double)(ul * w0); s[4] += (double)(vl * w0); s[5] += (double)(ul * vl);
   }
-  block_sum_store<6>(s, acc + (size_t)(iz - 1) * 8);
+  block_sum_store<6, 1024>(s, acc + (size_t)(iz - 1) * 8);
 }
 
 // Max |u|, |v|, |w| for the CFL time step (les.F90:205-207).
