@@ -165,7 +165,7 @@ template <class T> __device__ __forceinline__ cx<T> shfl_cx(unsigned mask, cx<T>
 // A row's team of TP threads (M1 rounded up to a power of two): thread t's
 // pass 1 index j (M1: none) and the lane of its mirror partner M1 - j.  A
 // team of two warps splits j so that both are in the same warp.
-template <int M1, int TP> __device__ __forceinline__ void mirror_lanes(int t, int lane, int& j, int& partner) {
+template <int M1, int TP> __host__ __device__ __forceinline__ void mirror_lanes(int t, int lane, int& j, int& partner) {
   if (TP <= 32) {
     j = t;
     partner = (lane & ~(TP - 1)) | (t == 0 || t >= M1 ? t : M1 - t);
@@ -181,6 +181,13 @@ template <int M1, int TP> __device__ __forceinline__ void mirror_lanes(int t, in
     }
     if (l >= 2 * H) j = M1;
   }
+}
+// The elements (b, j), b < 12, of the forward transform's last pass; p points
+// at (0, j).  A thread without a j reads none: whatever element it named would
+// be another thread's, which may already be writing the next row's pass 1.
+template <int SB, class T, class P> __host__ __device__ __forceinline__ void own_elements(P p, bool act, cx<T> (&v)[12]) {
+#pragma unroll
+  for (int b = 0; b < 12; b++) v[b] = act ? p[b * SB] : mk((T)0, (T)0);
 }
 
 }  // namespace les

@@ -451,18 +451,18 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
       cx<T> zf[8];  // outputs 0..3 and 8..11
       {
         cx<T> v[12];
+        own_elements<SB>((const cx<T>*)pj, act, v);
         if constexpr (C::PFA) {
 #pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const cx<T> w = k ? twj[(k - 1) * M1] : zero_cx<T>();
+          for (int k = 1; k < 4; k++) {
+            const cx<T> w = twj[(k - 1) * M1];
 #pragma unroll
-            for (int b = k; b < 12; b += 4) v[b] = k ? cmul(pj[b * SB], w) : pj[b * SB];
+            for (int b = k; b < 12; b += 4) v[b] = cmul(v[b], w);
           }
           Dft12Pfa<T, M1>::forward(v, w3, zf);
         } else {
-          v[0] = pj[0];
 #pragma unroll
-          for (int b = 1; b < 12; b++) v[b] = cmul(pj[b * SB], twj[(b - 1) * M1]);
+          for (int b = 1; b < 12; b++) v[b] = cmul(v[b], twj[(b - 1) * M1]);
           cx<T> o[12];
           dft12_forward<T>(v, o);
 #pragma unroll
@@ -492,7 +492,8 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
       }
     }
     // no barrier here: the next level's pass 1 writes the elements this
-    // thread's pass 1 read, in the same buffer
+    // thread's last pass read, in the same buffer, and no other thread read
+    // them (own_elements)
   }
 }
 

@@ -2,15 +2,48 @@
 // library dispatches (les_engine.cuh with_small); host code only, checked by
 // tests/test_launch_shapes.py.
 //   clip_walls <NSX> <row transforms' threads> <block>
+//   row <real bytes> <NSX> <thread of the team> <written by the next level's
+//       pass 1> : <read by the forward transform's last pass>
+//       (elements of the row's buffer in k_row_fused)
 #include <cstdio>
-#include "les_kernels.cuh"
+#include <vector>
+#include "les_fused.cuh"
 using namespace les;
 
 template <int NSX> void clip_walls() {
   using C = RowCfg<3 * NSX / 2>;
   printf("clip_walls %d %d %d\n", NSX, C::THREADS, C::SUM_THREADS);
 }
-template <int N> void one() { clip_walls<N>(); }
+// a row of shared memory that notes what is read
+template <class T> struct Noted {
+  std::vector<int>* at;
+  int base;
+  cx<T> operator[](int i) const {
+    at->push_back(base + i);
+    return mk((T)0, (T)0);
+  }
+};
+template <class T, int NSX> void row() {
+  using C = FusedCfg<T, NSX>;
+  for (int t = 0; t < C::TP; t++) {
+    int j, partner;
+    mirror_lanes<C::M1, C::TP>(t, t & 31, j, partner);
+    const bool act = j < C::M1;
+    std::vector<int> read;
+    cx<T> v[12];
+    own_elements<C::SB>(Noted<T>{&read, C::off(act ? j : 0)}, act, v);
+    printf("row %d %d %d", (int)sizeof(T), NSX, t);
+    for (int b = 0; act && b < 12; b++) printf(" %d", C::off(j) + b * C::SB);
+    printf(" :");
+    for (int e : read) printf(" %d", e);
+    printf("\n");
+  }
+}
+template <int N> void one() {
+  clip_walls<N>();
+  row<float, N>();
+  row<double, N>();
+}
 int main() {
   one<16>(); one<32>(); one<64>(); one<96>(); one<128>(); one<192>(); one<256>(); one<384>(); one<512>();
   return 0;

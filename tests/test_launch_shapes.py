@@ -48,3 +48,22 @@ def test_wall_sums_shuffle_between_lanes_that_exist(shapes):
     for n, (threads, block) in rows.items():
         assert threads <= block < threads + 32
         assert tree_sum(block) == block
+
+
+def test_row_elements_have_one_thread(shapes):
+    """k_row_fused has no barrier between a level's last forward pass and the
+    next level's first pass: each element that the one reads must be written by
+    the same thread in the other."""
+    plans = {}
+    for real, nsx, t, *rest in shapes["row"]:
+        cut = rest.index(":")
+        plans.setdefault((int(real), int(nsx)), []).append((rest[:cut], rest[cut + 1:]))
+    assert sorted(plans) == [(r, n) for r in (4, 8) for n in SIZES]
+    for plan, threads in plans.items():
+        owner = {}
+        for t, (written, _) in enumerate(threads):
+            for e in written:
+                assert owner.setdefault(e, t) == t, plan
+        assert len(owner) == 3 * plan[1] // 2, plan
+        for t, (_, read) in enumerate(threads):
+            assert all(owner[e] == t for e in read), (plan, t)
