@@ -1047,8 +1047,8 @@ struct Engine : EngineBase {
     LES_CUDA(cudaMemsetAsync(acc.p, 0, (size_t)NZ * 16 * sizeof(double), st));
     launch(k_plane_sums<T>, dim3(1, NZ), dim3(1024), 0, st, (const T*)phys[0].p, (const T*)phys[1].p,
            (const T*)phys[2].p, (const T*)(e.p + ps), ps, acc.p);
-    launch(k_sum_parts, dim3(NZ), dim3(256), 0, st, (const double*)divpart.p, nstat_parts, 1, divacc.p, 1);
-    launch(k_sum_parts, dim3(NZ), dim3(256), 0, st, (const double*)sgspart.p, nstat_parts, 6, sgsacc.p, 8);
+    launch(k_sum_parts<1>, dim3(NZ), dim3(kSumThreads), 0, st, (const double*)divpart.p, nstat_parts, divacc.p, 1);
+    launch(k_sum_parts<6>, dim3(NZ), dim3(kSumThreads), 0, st, (const double*)sgspart.p, nstat_parts, sgsacc.p, 8);
     std::vector<double> sums((size_t)NZ * 16), mshadow(NZ), vshadow(NZ);
     LES_CUDA(cudaMemcpyAsync(sums.data(), acc.p, sums.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     LES_CUDA(cudaMemcpyAsync(mshadow.data(), mu.p, NZ * sizeof(double), cudaMemcpyDeviceToHost, st));

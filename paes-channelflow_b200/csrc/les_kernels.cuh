@@ -694,21 +694,33 @@ __device__ __forceinline__ void block_sum_store(double (&v)[NV], double* out) {
   }
 }
 
-// Per-level totals of per-block partial sums: one block per level z,
-// out[z*ostride + q] = sum over p < nparts of part[(z*nparts + p)*nq + q],
-// q < nq <= 8, summed in a fixed order.
-static __global__ void __launch_bounds__(256) k_sum_parts(const double* __restrict__ part, int nparts, int nq,
-                                                          double* __restrict__ out, int ostride) {
-  const size_t z = blockIdx.x;
-  double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int p = threadIdx.x; p < nparts; p += blockDim.x)
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      if (q < nq) s[q] += part[(z * nparts + p) * nq + q];
-  double t[8];
-  block_sum_store<8, 256>(s, t);
-  if (threadIdx.x == 0)
-    for (int q = 0; q < nq; q++) out[z * ostride + q] = t[q];
+// Per-level totals of partial sums: one block per level z, out[z*ostride + q] =
+// sum over p < nparts of part[(z*nparts + p)*NQ + q], in a fixed order.
+// Neighbouring threads take neighbouring values (kSumThreads is a multiple of
+// NQ: a thread's are all of quantity t % NQ), several loads in flight, so that a
+// level's partials (one per warp of k_row_fused or k_flux, 442 KB of SGS means
+// at 768x768 points) arrive at the block's bandwidth and not one latency after
+// the other: 32 levels of 512x512 25 -> 8 us (SGS) and 20 -> 4 us (divz) against
+// 256 threads that each took a whole row of NQ values.
+constexpr int kSumThreads = 960;
+template <int NQ>
+__global__ void __launch_bounds__(kSumThreads) k_sum_parts(const double* __restrict__ part, int nparts,
+                                                           double* __restrict__ out, int ostride) {
+  static_assert(kSumThreads % NQ == 0 && kSumThreads % 32 == 0 && NQ <= kSumThreads / 32, "a warp per quantity");
+  __shared__ double red[kSumThreads];
+  const int t = threadIdx.x, n = nparts * NQ;
+  const double* p = part + (size_t)blockIdx.x * n;
+  double s = 0.0;
+#pragma unroll 8
+  for (int i = t; i < n; i += kSumThreads) s += p[i];
+  red[t] = s;
+  __syncthreads();
+  const int q = t >> 5;
+  if (q >= NQ) return;
+  s = 0.0;
+  for (int i = t & 31; i < kSumThreads / NQ; i += 32) s += red[i * NQ + q];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((t & 31) == 0) out[(size_t)blockIdx.x * ostride + q] = s;
 }
 
 // Raw sums over the padded planes U, V at level 1 (blockIdx.y = 0) and nnz

@@ -349,3 +349,27 @@ def test_flux_columns_of_the_unfused_stage(gpu_lib, product, nx, ny, nz, imodel,
             assert relerr(fg[k], fo[k], vscale) < tol, (precision, k)
         if precision == 8:
             assert relerr(fg["e"], fo["e"]) < tol
+
+
+@pytest.mark.parametrize("nx,ny,imodel", [(16, 16, 3), (512, 16, 3), (512, 128, 3), (128, 64, 4)])
+def test_statistics_from_few_and_many_partial_sums(gpu_lib, product, nx, ny, imodel):
+    """divz and the SGS means from 9, 288, 2304 (one partial sum per warp of
+    k_row_fused) and 576 (k_flux) partials a level: less than one round of
+    k_sum_parts' threads, a remainder and several unrolled rounds.  A field
+    with a divergence, so that divz is no round-off; one stage from the same
+    field, tolerance that of one stage's tendencies (1e-9 of the scale)."""
+    o, g, f = make_pair(product, nx, ny, 4, imodel=imodel)
+    o.set_fields(u=f["u"] + 0.5 * np.sin(2 * np.pi * np.arange(nx) / nx)[None, None, :])
+    o.deal_fields()
+    f = o.get_fields()
+    g.upload(f["u"], f["v"], f["w"], f["e"], f["p"])
+    o.stage(0, 1, 1)
+    g.stage(0, True, 1)
+    o.compmn()
+    mo, _ = o.stats()
+    mg, _ = g.stats()
+    assert mo[2].min() > 1e-3
+    assert relerr(mg[2], mo[2]) < 1e-9
+    scale = np.abs(mo[13:19]).max()
+    for r in range(13, 19):
+        assert relerr(mg[r], mo[r], scale) < 1e-9, r
