@@ -893,30 +893,47 @@ struct Engine : EngineBase {
   }
   // Pressure solve, with the update of u, v, w and their tendencies when
   // `update` (the split entry points solve with the right-hand side in ph and
-  // update later).  k_press takes 32 modes a block where the blocks still
-  // fill the device and the inputs of one block per SM stay within about half
-  // of L2 (their second read, for the update, then hits it); else 16, whose
-  // blocks hold half as much and split a column into twice the chunks.  Solve
-  // and update, 16 / 32 modes, against a thread per column and a separate
-  // update: 512x512x64 mixed 428 / 313, 359 us; 384x384x192 mixed 557 / 481,
-  // 718; 256x256x256 mixed 317 / 367, 670; 256x256x128 FP64 223 / 235, 465;
-  // 512x512x256 mixed 1264 / 1473, 1413, FP64 1815 / 2720, 2305; 64x64x64
-  // FP64 14 / 18, 130.  (8 modes: 64-byte rows, 2280 and 2340 us at
-  // 512x512x256.)  More than kPressMaxNZ levels take the one-thread sweep.
+  // update later).  k_press takes `modes` modes a block and chunks of L levels a
+  // thread; a column is modes x cdiv(NZ, L) threads of a block.
+  // L: where the blocks do not fill the device the chain of levels counts, and a
+  // column takes up to 512 / modes threads (64x64x64 FP64 10 us, 11 with L = 4).
+  // Where they do, more threads a column only mean more totals to scan and fewer
+  // loads in flight a thread: L is at least 4 there, on large planes 8 in FP32
+  // (which fetches four levels at a time) and for the solve alone.
+  // 512x512x16 mixed 158 us with L = 1, 69 with 4, 64 with 8 (a thread per column
+  // and a separate update: 89); 512x512x32 FP64 250 -> 188 (292), mixed 207 -> 122
+  // (177); solve alone 512x512x128 249 -> 181 (238).
+  // Blocks of more than 256 and less than about 450 threads leave an SM half empty: they
+  // become two of at most 256 with chunks of up to 8 levels, 16 in wide blocks
+  // (512x512x96 FP64 658 -> 602, mixed 450 -> 384; with 13 levels in FP64, at
+  // 512x512x200, 1329 -> 1602).
+  // Modes: rows of 256 bytes, 16 modes in FP64 and 32 in FP32, on large planes
+  // and while the inputs of one block per SM stay within about half of L2 (their
+  // second read, for the update, then hits it: 512x512x256 mixed 1264 us with 16,
+  // 1473 with 32; 512x512x64 287 and 243); the solve alone 32 up to 32 levels
+  // (512x512x16 23.7 and 21.4 us, 512x512x64 86 and 104).  (8 modes: 64-byte rows,
+  // 2280 and 2340 us at 512x512x256, FP64 1815.)  More than kPressMaxNZ levels take
+  // the one-thread sweep.
   static constexpr int kPressMaxNZ = 512;
-  template <int MODES, bool RHS, bool UPD> void press_launch(const StageArgs& a) {
-    const int L = (int)cdiv(NZ, 512 / MODES);  // levels of a chunk
+  template <int MODES, bool RHS, bool UPD> void press_launch(const StageArgs& a, int L) {
     const int threads = (int)cdiv((size_t)MODES * cdiv(NZ, L), 32) * 32;
-    const size_t smem = (size_t)L * threads * (sizeof(cx<double>) + sizeof(double));
-    set_smem_limit((const void*)k_press<T, MODES, RHS, UPD>, smem);  // its static tables take up to 24 KB more
+    // r (then p) and d of every level, and the totals of every warp
+    const size_t smem = (size_t)L * threads * 3 * sizeof(double) + (size_t)threads / 32 * 6 * MODES * sizeof(double);
     launch(k_press<T, MODES, RHS, UPD>, dim3((unsigned)(nm / MODES)), dim3((unsigned)threads), smem, st, uh.p, vh.p, wh.p,
            ruo.p, rvo.p, rwo.p, (const cx<T>*)run.p, (const cx<T>*)rvn.p, (const cx<T>*)rwn.p, ph.p, mu.p, mv.p, mru.p,
            mrv.p, a, L, err.p);
   }
   template <bool RHS, bool UPD> void press_pick(const StageArgs& a) {
+    const bool f32 = sizeof(T) == 4, fills = nm / 16 >= (size_t)nsm, large = nm / 16 >= (size_t)4 * nsm;
     const size_t inputs = (size_t)32 * NZ * 9 * sizeof(cx<T>) * nsm;  // of one 32-mode block per SM
-    if (nm % 32 == 0 && nm / 32 >= (size_t)nsm && NZ <= 256 && inputs <= (size_t)72 << 20) press_launch<32, RHS, UPD>(a);
-    else press_launch<16, RHS, UPD>(a);
+    const bool wide = large && nm % 32 == 0 && (UPD ? f32 && NZ <= 256 && inputs <= (size_t)72 << 20 : NZ <= 32);
+    const int modes = wide ? 32 : 16, least = !fills ? 1 : large && (f32 || !UPD) ? 8 : 4;
+    int L = std::max(least, (int)cdiv(NZ, 512 / modes));
+    const int threads = modes * (int)cdiv(NZ, L);
+    const int half = (int)cdiv(NZ, 256 / modes);
+    if (fills && threads > 256 && threads < (wide ? 480 : 448) && half <= (wide ? 16 : 8)) L = half;
+    if (wide) press_launch<32, RHS, UPD>(a, L);
+    else press_launch<16, RHS, UPD>(a, L);
   }
   void press_kernel(const StageArgs& a, bool rhs_in_ph, bool update) {
     if (NZ <= kPressMaxNZ) {

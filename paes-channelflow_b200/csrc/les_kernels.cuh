@@ -1293,8 +1293,10 @@ k_e_update(const cx<T>* __restrict__ rem, T* __restrict__ re, T* __restrict__ e,
 // with the wall's first row).  Bound by HBM on large grids (r and d never go
 // there, and the update's second read of the inputs mostly hits L2), by the
 // chain of levels on small ones, which the chunks cut to L + chunks / warp
-// steps: 64x64x64 FP64 130 -> 14 us, 128x128x96 FP64 235 -> 51 us, 512x512x256
-// mixed 1413 -> 1264 us against one thread per column and a separate update.
+// steps: 64x64x64 FP64 120 -> 10 us, 128x128x96 FP64 232 -> 46 us, 512x512x256
+// mixed 1402 -> 1264 us against one thread per column and a separate update.
+// Shared memory goes with the threads and levels of the launch (tables for 16
+// warps in every block left 512x512x8 mixed at 44 us instead of 31).
 template <class T, int MODES, bool RHS_IN_PH, bool UPDATE>
 __global__ void __launch_bounds__(512)
 k_press(cx<T>* __restrict__ uh, cx<T>* __restrict__ vh, cx<T>* __restrict__ wh, cx<T>* __restrict__ ruo,
@@ -1302,13 +1304,15 @@ k_press(cx<T>* __restrict__ uh, cx<T>* __restrict__ vh, cx<T>* __restrict__ wh, 
         const cx<T>* __restrict__ rwn, cx<double>* __restrict__ ph, double* mu, double* mv, double* mru, double* mrv,
         StageArgs a, int L, int* err) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ double tot[2][16][3][MODES];  // forward, backward; warp; (product, re, im)
   const int KX = a.KX, NY = a.NY, NZ = a.NZ;
   const int nm = KX * NY, nt = blockDim.x, tid = threadIdx.x;
   cx<double>* const R = reinterpret_cast<cx<double>*>(smraw) + tid;                        // R[l nt]: r, then p
   double* const D = reinterpret_cast<double*>(smraw + (size_t)L * nt * sizeof(cx<double>)) + tid;  // D[l nt]
   const int md = tid % MODES, c = tid / MODES;
   const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
+  // totals of a warp's chunks: [forward, backward][warp][product, re, im][mode]
+  double* const tots = D - tid + (size_t)L * nt + md;
+  auto tot = [&](int dir, int w, int q) -> double& { return tots[((dir * nwarp + w) * 3 + q) * MODES]; };
   const int m = blockIdx.x * MODES + md;
   const int ky = m / KX, kx = m - ky * KX;
   const bool live = ky != NY / 2 && m != 0;
@@ -1385,15 +1389,15 @@ k_press(cx<T>* __restrict__ uh, cx<T>* __restrict__ vh, cx<T>* __restrict__ wh, 
       }
     }
     if (dir ? lane < MODES : lane >= 32 - MODES) {
-      tot[dir][warp][0][md] = ip;
-      tot[dir][warp][1][md] = iv.x;
-      tot[dir][warp][2][md] = iv.y;
+      tot(dir, warp, 0) = ip;
+      tot(dir, warp, 1) = iv.x;
+      tot(dir, warp, 2) = iv.y;
     }
     __syncthreads();
     cx<double> y = mk(0.0, 0.0);
     for (int k = 0; k < (dir ? nwarp - 1 - warp : warp); k++) {
       const int w = dir ? nwarp - 1 - k : k;
-      y = mk(tot[dir][w][1][md], tot[dir][w][2][md]) + y * tot[dir][w][0][md];
+      y = mk(tot(dir, w, 1), tot(dir, w, 2)) + y * tot(dir, w, 0);
     }
     if (MODES == 32) return y;
     // this chunk's inflow: the neighbour chunk's inclusive value applied to y

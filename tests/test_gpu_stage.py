@@ -373,3 +373,28 @@ def test_statistics_from_few_and_many_partial_sums(gpu_lib, product, nx, ny, imo
     scale = np.abs(mo[13:19]).max()
     for r in range(13, 19):
         assert relerr(mg[r], mo[r], scale) < 1e-9, r
+
+
+@pytest.mark.parametrize("nz", [4, 8, 9, 33, 70, 99])
+def test_pressure_columns_on_large_planes(gpu_lib, product, nz):
+    """The pressure solve where a plane's columns fill the device: chunks of 4
+    and 8 levels, one chunk, a short last one, the columns split for two blocks
+    per SM (70 and 99 levels), blocks of 16 and 32 modes, the whole
+    stage and the six entry points.  Tolerances of the stage tests."""
+    for precision, tol in ((8, 1e-11), (4, 2e-5)):
+        o, g, f = make_pair(product, 192, 128, nz, precision=precision)
+        g2 = product.LesGpu(g.cfg)
+        g2.upload(f["u"], f["v"], f["w"], f["e"], f["p"])
+        for s in (1, 2):
+            o.stage(0, 1, s)
+            g.stage(0, True, s)
+            g2.stage_split(0, True, s)
+        fo = o.get_fields()
+        vscale = np.abs(fo["u"]).max()
+        for h in (g, g2):
+            fg = h.download()
+            for k in "uvw":
+                assert relerr(fg[k], fo[k], vscale) < tol, (precision, k)
+            if precision == 8:
+                assert relerr(fg["p"], fo["p"]) < 1e-9
+            h.close()
