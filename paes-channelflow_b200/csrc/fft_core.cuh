@@ -379,11 +379,19 @@ __device__ __forceinline__ void smem_fft(int ntrans, cx<T>* sm, const cx<T>* __r
 //   natural layout: rows  sm[t*N + n];  cols (COLS) sm[n*ntrans + t]
 // Requires blockDim.x >= ntrans*N2 and smem_fft_elems<N, COLS>(ntrans)
 // elements; every thread of the block must call it.  Ends with a
-// __syncthreads() when OUT_SMEM.  fft_core_tab takes the length-N twiddle
+// __syncthreads() when OUT_SMEM.  With a gate, the transform goes on only if
+// gate(), called by every thread once its inputs are loaded, says so for the
+// whole block; returns whether it did.  fft_core_tab takes the length-N twiddle
 // table itself (e.g. staged in shared memory by stage_twiddles); fft_core
 // reads it from the global table.
-template <int N, int S, bool COLS, bool IN_SMEM, bool OUT_SMEM, class T, class LoadF, class StoreF>
-__device__ __forceinline__ void fft_core_tab(int ntrans, cx<T>* sm, const cx<T>* twn, LoadF load, StoreF store) {
+struct NoLoad {};
+struct NoStore {
+  template <class V> __device__ void operator()(int, int, V) const {}
+};
+struct NoGate {};
+template <int N, int S, bool COLS, bool IN_SMEM, bool OUT_SMEM, class T, class LoadF, class StoreF, class GateF>
+__device__ __forceinline__ bool fft_core_tab(int ntrans, cx<T>* sm, const cx<T>* twn, LoadF load, StoreF store,
+                                             GateF gate) {
   constexpr int N1 = Split<N>::N1;
   constexpr int N2 = Split<N>::N2;
   constexpr int LD = N2 + 1;
@@ -414,6 +422,8 @@ __device__ __forceinline__ void fft_core_tab(int ntrans, cx<T>* sm, const cx<T>*
         }
       }
     }
+    if constexpr (!std::is_same_v<GateF, NoGate>)
+      if (!gate()) return false;
     if (IN_SMEM) __syncthreads();
     if (active) {
       Dft<N1, S, T>::run(v);
@@ -455,11 +465,12 @@ __device__ __forceinline__ void fft_core_tab(int ntrans, cx<T>* sm, const cx<T>*
     }
     if (OUT_SMEM) __syncthreads();
   }
+  return true;
 }
-template <int N, int S, bool COLS, bool IN_SMEM, bool OUT_SMEM, class T, class LoadF, class StoreF>
-__device__ __forceinline__ void fft_core(int ntrans, cx<T>* sm, const cx<T>* __restrict__ tw, LoadF load,
-                                         StoreF store) {
-  fft_core_tab<N, S, COLS, IN_SMEM, OUT_SMEM, T>(ntrans, sm, tw + tw_off(N), load, store);
+template <int N, int S, bool COLS, bool IN_SMEM, bool OUT_SMEM, class T, class LoadF, class StoreF, class GateF = NoGate>
+__device__ __forceinline__ bool fft_core(int ntrans, cx<T>* sm, const cx<T>* __restrict__ tw, LoadF load,
+                                         StoreF store, GateF gate = GateF{}) {
+  return fft_core_tab<N, S, COLS, IN_SMEM, OUT_SMEM, T>(ntrans, sm, tw + tw_off(N), load, store, gate);
 }
 // Copy of the length-N twiddle table into shared memory `dst` (N entries),
 // by the whole block; ends with a barrier.
@@ -470,10 +481,6 @@ __device__ __forceinline__ const cx<T>* stage_twiddles(cx<T>* dst, const cx<T>* 
   __syncthreads();
   return dst;
 }
-struct NoLoad {};
-struct NoStore {
-  template <class V> __device__ void operator()(int, int, V) const {}
-};
 
 // Signed wavenumber index of FFT bin k for length n (k > n/2 -> k - n).
 __host__ __device__ __forceinline__ int signed_k(int k, int n) { return (k > n / 2) ? k - n : k; }

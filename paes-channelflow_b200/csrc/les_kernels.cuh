@@ -592,10 +592,14 @@ k_x_inverse(const __grid_constant__ Ptr8 src, const __grid_constant__ Ptr12 dst,
 // yderiv of delta = max(emin - E, 0) on padded planes (column pairs),
 // added to EY.  This and k_clip_x make EX, EY the derivatives of the
 // clipped ebuf = max(expand(e), emin) (comp1.f90:109,121; derivs2.f90:20-21).
-// Blocks whose points are all above emin return before the transforms (unclipped
-// 96x128x45 FP64: 20 -> 10 us here, 29 -> 13 in k_clip_x).
+// Blocks whose points are all above emin stop once they are loaded: clipped or not,
+// E is read once (k_clip_y and k_clip_x of 512x512x32 FP64, unclipped 102 and 26 us,
+// clipped 307 and 429; with a scan of E before the transform's own loads 120 and
+// 249, 355 and 877; always transforming 322 and 559).  Registers of the 768-point
+// blocks: 168 (FP64) and, in k_clip_x, 96 (FP32), a block per SM more than unbounded
+// (k_clip_y FP64 440 -> 307, k_clip_x FP32 274 -> 237).
 template <class T, int NSY>
-__global__ void __launch_bounds__(ColCfg<3 * NSY / 2, T>::THREADS)
+__global__ void __launch_bounds__(ColCfg<3 * NSY / 2, T>::THREADS, NSY == 512 && sizeof(T) == 8 ? 3 : 0)
 k_clip_y(const T* __restrict__ E, T* __restrict__ EY, int MX, T emin, T ky0, const cx<T>* __restrict__ tw) {
   constexpr int M = 3 * NSY / 2;
   using C = ColCfg<M, T>;
@@ -605,22 +609,17 @@ k_clip_y(const T* __restrict__ E, T* __restrict__ EY, int MX, T emin, T ky0, con
   const int c0 = blockIdx.x * C::TC, ncp = MX / 2;
   const cx<T>* Ez = reinterpret_cast<const cx<T>*>(E + zoff);
   bool below = false;
-  for (int i = threadIdx.x; i < C::TC * M; i += C::THREADS) {
-    const int t = i % C::TC, n = i / C::TC;
-    if (c0 + t >= ncp) continue;
-    const cx<T> v = Ez[(size_t)n * ncp + c0 + t];
-    below = below || emin - v.x > (T)0 || emin - v.y > (T)0;
-  }
-  if (!__syncthreads_or(below)) return;  // delta is zero: so are its derivatives
-  fft_core<M, -1, true, false, true>(C::TC, sm, tw, [&](int t, int n) {
+  const bool any = fft_core<M, -1, true, false, true>(C::TC, sm, tw, [&](int t, int n) {
     int c = c0 + t;
     cx<T> v = zero_cx<T>();
     if (c < ncp) {
       cx<T> ev = Ez[(size_t)n * ncp + c];
       v = mk(tmax(emin - ev.x, (T)0), tmax(emin - ev.y, (T)0));
     }
+    below |= (v.x > (T)0) | (v.y > (T)0);
     return v;
-  }, NoStore{});
+  }, NoStore{}, [&] { return __syncthreads_or(below) != 0; });
+  if (!any) return;  // delta is zero: so are its derivatives
   cx<T>* EYz = reinterpret_cast<cx<T>*>(EY + zoff);
   fft_core<M, +1, true, true, false>(C::TC, sm, tw, Derivative<T, M>(ky0), [&](int t, int n, cx<T> d) {
     int c = c0 + t;
@@ -632,7 +631,7 @@ k_clip_y(const T* __restrict__ E, T* __restrict__ EY, int MX, T emin, T ky0, con
 
 // xderiv of delta (row pairs), added to EX; E <- max(E, emin).
 template <class T, int NSX>
-__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS)
+__global__ void __launch_bounds__(RowCfg<3 * NSX / 2>::THREADS, NSX == 512 ? (sizeof(T) == 8 ? 3 : 5) : 0)
 k_clip_x(T* __restrict__ E, T* __restrict__ EX, int MY, T emin, T kx0, const cx<T>* __restrict__ tw) {
   constexpr int MX = 3 * NSX / 2;
   using C = RowCfg<MX>;
@@ -643,18 +642,17 @@ k_clip_x(T* __restrict__ E, T* __restrict__ EX, int MY, T emin, T kx0, const cx<
   T* Ez = E + zoff;
   T* EXz = EX + zoff;
   bool below = false;
-  for (int i = threadIdx.x; i < 2 * C::NT * MX; i += C::THREADS)
-    if (2 * p0 * MX + i < 2 * np * MX) below = below || !(Ez[(size_t)2 * p0 * MX + i] >= emin);
-  if (!__syncthreads_or(below)) return;  // nothing to raise, delta is zero
-  fft_core<MX, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
+  const bool any = fft_core<MX, -1, false, false, true>(C::NT, sm, tw, [&](int t, int n) {
     int p = p0 + t;
     cx<T> v = zero_cx<T>();
     if (p < np) {
       T a = Ez[(size_t)(2 * p) * MX + n], b = Ez[(size_t)(2 * p + 1) * MX + n];
       v = mk(tmax(emin - a, (T)0), tmax(emin - b, (T)0));
+      below |= !(a >= emin) | !(b >= emin);
     }
     return v;
-  }, NoStore{});
+  }, NoStore{}, [&] { return __syncthreads_or(below) != 0; });
+  if (!any) return;  // nothing to raise, delta is zero
   fft_core<MX, +1, false, true, false>(C::NT, sm, tw, Derivative<T, MX>(kx0), [&](int t, int n, cx<T> d) {
     int p = p0 + t;
     if (p >= np) return;
