@@ -373,7 +373,8 @@ __device__ __forceinline__ void smem_fft(int ntrans, cx<T>* sm, const cx<T>* __r
 // General four-step transform of `ntrans` sequences with one shared-memory
 // transpose.  Input comes from global memory through load(t, n) (pass A
 // issues N1 independent loads per thread before any arithmetic) or, with
-// IN_SMEM, from `sm` in natural layout (through load(n, v), unless NoLoad);
+// IN_SMEM, from `sm` in natural layout (unless NoLoad through load(n2, m, v), n =
+// n2 + m, m a compile-time constant);
 // output goes to store(t, k, v) or, with OUT_SMEM, back to `sm` in natural
 // layout.
 //   natural layout: rows  sm[t*N + n];  cols (COLS) sm[n*ntrans + t]
@@ -416,7 +417,7 @@ __device__ __forceinline__ bool fft_core_tab(int ntrans, cx<T>* sm, const cx<T>*
         const int n = n2 + N2 * n1;
         if constexpr (IN_SMEM) {
           v[n1] = COLS ? sm[n * ntrans + t] : sm[t * N + n];
-          if constexpr (std::is_invocable_v<LoadF, int, cx<T>>) v[n1] = load(n, v[n1]);
+          if constexpr (!std::is_same_v<LoadF, NoLoad>) v[n1] = load(n2, N2 * n1, v[n1]);
         } else {
           v[n1] = load(t, n);
         }

@@ -105,13 +105,18 @@ template <int N> __device__ __forceinline__ PairMode pair_mode(int n, int K) {
 }
 // d/dx of a transformed row or column, with the 1/N of the inverse transform
 // (the Nyquist mode dropped), at the inverse transform's loads: a pass over shared
-// memory, a barrier and a division per mode less (384x384x64 FP64: k_op_xderiv 139
-// -> 125 us, k_op_yderiv 205 -> 130).
+// memory, a barrier and a division per mode less.  Mode k = n2 + m with m known at
+// compile time: one conversion a thread, and only m = 0 and N/2 can be mode 0 or
+// Nyquist.  The kernels' registers are bounded (168 FP64, 128 FP32): unbounded, 512
+// points in FP64 lose a third of their blocks.  FP64 k_op_xderiv 576x576x27 66 us with
+// the factor in a pass of its own, 57 with a conversion per mode, 45 so; k_op_yderiv 92,
+// 62, 61; FP32 192x144x24 k_op_yderiv 5.2, 5.4, 3.6.
 template <class T, int N> struct Derivative {
   T k1;
   __device__ __forceinline__ explicit Derivative(T k0) : k1(k0 / (T)N) {}
-  __device__ __forceinline__ cx<T> operator()(int k, cx<T> v) const {
-    return (k == 0 || 2 * k == N) ? zero_cx<T>() : mul_i(v) * (k1 * (T)signed_k(k, N));
+  __device__ __forceinline__ cx<T> operator()(int n2, int m, cx<T> v) const {
+    const cx<T> d = mul_i(v) * (k1 * ((T)n2 + (T)(2 * m >= N ? m - N : m)));
+    return ((m == 0 || 2 * m == N) && n2 == 0) ? zero_cx<T>() : d;
   }
 };
 // ---------------------------------------------------------------------------
@@ -1742,7 +1747,7 @@ __global__ void k_set_mean(cx<T>* __restrict__ sp, const double* __restrict__ me
 // Batched 1D spectral derivative (xderiv/yderiv of filter_fftw.f90:138-248)
 // along rows or columns of real planes, pairing rows/columns.
 template <class T, int N>
-__global__ void __launch_bounds__(RowCfg<N>::THREADS)
+__global__ void __launch_bounds__(RowCfg<N>::THREADS, sizeof(T) == 8 ? 3 : 4)
 k_op_xderiv(const T* __restrict__ in, T* __restrict__ out, int nrows, T k0, const cx<T>* __restrict__ tw) {
   using C = RowCfg<N>;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1763,7 +1768,7 @@ k_op_xderiv(const T* __restrict__ in, T* __restrict__ out, int nrows, T k0, cons
   });
 }
 template <class T, int N>
-__global__ void __launch_bounds__(ColCfg<N, T>::THREADS)
+__global__ void __launch_bounds__(ColCfg<N, T>::THREADS, (sizeof(T) == 8 ? 384 : 512) / ColCfg<N, T>::THREADS)
 k_op_yderiv(const T* __restrict__ in, T* __restrict__ out, int n1, T k0, const cx<T>* __restrict__ tw) {
   using C = ColCfg<N, T>;
   extern __shared__ __align__(16) unsigned char smraw[];
