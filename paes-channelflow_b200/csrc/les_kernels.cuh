@@ -153,8 +153,11 @@ k_row_r2c(const T* __restrict__ in, cx<T>* __restrict__ out, int nrows, int KOUT
 
 // First KIN complex modes of each row (higher modes zero, imaginary parts of
 // mode 0 ignored as in a c2r transform) -> real rows of length N.
+// FP32 rows with a radix-16 first pass: six blocks per SM, or the twiddles asked for
+// with the data take 106 registers (384x192x40 10.2 us, 8.1 bounded; 9.4 with the
+// twiddles asked for after the data).
 template <class T, int N>
-__global__ void __launch_bounds__(RowCfg<N>::THREADS)
+__global__ void __launch_bounds__(RowCfg<N>::THREADS, sizeof(T) == 4 && Split<N>::N1 == 16 ? 6 : 0)
 k_row_c2r(const cx<T>* __restrict__ in, T* __restrict__ out, int nrows, int KIN, const cx<T>* __restrict__ tw) {
   using C = RowCfg<N>;
   extern __shared__ __align__(16) unsigned char smraw[];
