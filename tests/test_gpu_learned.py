@@ -282,3 +282,69 @@ def test_features_at_every_row_and_column_length(gpu_lib, product, nx, ny, nz):
         assert np.abs(got[:, :12] - ref).max() < tol * np.maximum(1.0, np.abs(ref).max()), precision
         assert not got[:, 12:].any()
         h.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 16), (32, 96), (64, 192), (96, 16), (128, 384), (192, 32), (256, 64),
+                                   (384, 128), (512, 256)])
+def test_every_feature_column_to_its_own_tolerance(gpu_lib, product, nx, ny):
+    """The gradient transforms of every grid length, each column held to its own
+    bound.  Smooth fields without a mean shear; a direction times |G| is within
+    twice the gradient vector's error of the gradient, whatever |G| is.  FP64:
+    the f32 rounding of the output (2^-21).  FP32: white noise of 4 units in the
+    last place of a field's rms (its own rounding and some 2 log2 n roundings of
+    each transform), times the largest wavenumbers over sqrt(3) and the vertical
+    difference, as a vector of nine, three times its rms.  The wall distances go
+    through no transform."""
+    nz = 4
+    cfg = product.channel_config(nx, ny, nz, dt=1e-3, re_tau=180.0, imodel=5)
+    rng = np.random.default_rng(nx * ny)
+    dz = cfg.zl / nz
+    x, y = np.arange(nx) * cfg.xl / nx, np.arange(ny) * cfg.yl / ny
+
+    def smooth():
+        a = np.zeros((nz, ny, nx))
+        for kx in (1, 2, 3):
+            for ky in (2, 4, 6):
+                c = 0.1 * rng.standard_normal((2, nz))
+                a += (c[0][:, None, None] * np.cos(kx * x)[None, None, :] * np.cos(ky * y)[None, :, None]
+                      + c[1][:, None, None] * np.sin(kx * x)[None, None, :] * np.sin(ky * y)[None, :, None])
+        return a
+
+    u, v, w = smooth(), smooth(), smooth()
+    w[-1] = 0.0
+
+    def d(a, axis, n, length):
+        kk = np.fft.fftfreq(n, 1.0 / n) * 2 * np.pi / length
+        kk[n // 2] = 0.0
+        sh = [1, 1, 1]
+        sh[axis] = n
+        return np.fft.ifft(np.fft.fft(a, axis=axis) * (1j * kk).reshape(sh), axis=axis).real
+
+    def dzc(a):
+        o = np.empty_like(a)
+        o[1:-1] = (a[2:] - a[:-2]) / (2 * dz)
+        o[0], o[-1] = (a[1] - a[0]) / dz, (a[-1] - a[-2]) / dz
+        return o
+
+    wl = np.concatenate([np.zeros((1, ny, nx)), w[:-1], np.zeros((1, ny, nx))])
+    wc = 0.5 * (wl[1:] + wl[:-1])
+    dx, dy = lambda a: d(a, 2, nx, cfg.xl), lambda a: d(a, 1, ny, cfg.yl)
+    g = np.stack([dx(u), dx(v), dx(wc), dy(u), dy(v), dy(wc), dzc(u), dzc(v), (wl[1:] - wl[:-1]) / dz], -1).reshape(-1, 9)
+    G = np.sqrt((g * g).sum(1))
+    z = (np.arange(nz) + 0.5) * dz
+    zw = np.minimum(z, cfg.zl - z)
+    delta = (cfg.xl / nx * cfg.yl / ny * dz) ** (1.0 / 3.0)
+    kxm, kym = np.pi * nx / cfg.xl, np.pi * ny / cfg.yl
+    rms2 = sum((a * a).mean() for a in (u, v, w))
+    noise = 4 * 2.0**-24 * np.sqrt(rms2 * ((kxm**2 + kym**2) / 3 + 2 / dz**2))
+    for precision, err in ((8, 0.0), (4, 3 * noise)):
+        cfg.precision = precision
+        h = product.LesGpu(cfg)
+        h.upload(u, v, w, np.full_like(u, 1e-4), None)
+        got = h.learned_features().cpu().numpy().astype(np.float64)
+        h.close()
+        for c in range(9):
+            assert (np.abs(got[:, c] * G - g[:, c]) <= 2 * err + 2.0**-21 * G).all(), (precision, c)
+        for c, ref in ((9, np.repeat(np.minimum(zw / delta, 16.0), nx * ny)), (10, np.repeat(zw * 2 / cfg.zl, nx * ny))):
+            assert (np.abs(got[:, c] - ref) <= 2.0**-21 * ref).all(), (precision, c)
+        assert (np.abs(got[:, 11] - delta * G) <= delta * (err + 2.0**-21 * G)).all(), precision
