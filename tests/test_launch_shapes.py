@@ -67,3 +67,17 @@ def test_row_elements_have_one_thread(shapes):
         assert len(owner) == 3 * plan[1] // 2, plan
         for t, (_, read) in enumerate(threads):
             assert all(owner[e] == t for e in read), (plan, t)
+
+
+def test_prefetch_tiles_of_the_column_plans(shapes):
+    """The tiles that k_y_inverse and k_y_forward prefetch are ColPlan's: boxes
+    of at most 256 rows and 256 reals that cover a column exactly, every tile at
+    a 16-byte boundary.  Row prefetches: multiples of 16 bytes."""
+    seen = set()
+    for real, ns, nrows, tc, nb, br in (map(int, r) for r in shapes["tile"]):
+        seen.add((real, ns, nrows))
+        assert nb * br == nrows and br <= 256, (real, ns, nrows)
+        assert (tc * 2 * real) % 16 == 0 and 2 * tc <= 256, (real, ns, nrows)
+    assert seen == {(r, n, m) for r in (4, 8) for n in SIZES for m in (n, 3 * n // 2)}
+    assert len(shapes["rows"]) == 2 * 2 * len(SIZES)
+    assert all(int(b) % 16 == 0 for _, _, b in shapes["rows"])
