@@ -177,9 +177,6 @@ template <> struct Split<768> { static constexpr int N1 = 24, N2 = 32; };
 
 // Outer twiddles exp(-2 pi i j / N) for every supported N, concatenated.
 // tw_off(N) is the offset of the table for N.
-struct TwTable {
-  const void* base;  // cx<T>*
-};
 constexpr int kSizes[] = {16, 24, 32, 48, 64, 96, 128, 144, 192, 256, 288, 384, 512, 576, 768};
 constexpr int kNumSizes = sizeof(kSizes) / sizeof(int);
 __host__ __device__ constexpr int tw_off(int n) {
@@ -201,198 +198,34 @@ __host__ __device__ constexpr int tw_off(int n) {
 }
 constexpr int kTwTotal = tw_off(768) + 768;
 
-template <int N> struct BlockFft {
-  static constexpr int N1 = Split<N>::N1;
-  static constexpr int N2 = Split<N>::N2;
-  // shared-memory elements needed for `ntrans` transforms
-  static constexpr int smem_elems(int ntrans) { return ntrans * N1 * (N2 + 1); }
-};
-
-// One batch of `ntrans` complex transforms of length N in a CTA.
-//   load(t, n)      -> input element n of transform t
-//   store(t, k, v)  <- output element k of transform t
-// TFAST = true maps consecutive threads to consecutive transforms (column
-// transforms); false maps them to consecutive elements (row transforms).
-// tw: the concatenated outer-twiddle table (global memory).
-// The caller must __syncthreads() before reusing `sm`.
-template <int N, int S, bool TFAST, class T, class LoadF, class StoreF>
-__device__ __forceinline__ void block_fft(int ntrans, cx<T>* sm, const cx<T>* __restrict__ tw, LoadF load,
-                                          StoreF store) {
-  constexpr int N1 = Split<N>::N1;
-  constexpr int N2 = Split<N>::N2;
-  constexpr int LD = N2 + 1;
-  const cx<T>* twn = tw + tw_off(N);
-  const int nA = ntrans * N2;
-  for (int it = threadIdx.x; it < nA; it += blockDim.x) {
-    int t, n2;
-    if (TFAST) { t = it % ntrans; n2 = it / ntrans; }
-    else { t = it / N2; n2 = it - t * N2; }
-    cx<T> v[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; n1++) v[n1] = load(t, n2 + N2 * n1);
-    Dft<N1, S, T>::run(v);
-#pragma unroll
-    for (int k1 = 0; k1 < N1; k1++) {
-      cx<T> w = twn[n2 * k1];
-      if (S > 0) w.y = -w.y;
-      cx<T> r = (k1 == 0) ? v[k1] : cmul(v[k1], w);
-      if (TFAST) sm[(k1 * N2 + n2) * ntrans + t] = r;
-      else sm[(t * N1 + k1) * LD + n2] = r;
-    }
-  }
-  __syncthreads();
-  const int nB = ntrans * N1;
-  for (int it = threadIdx.x; it < nB; it += blockDim.x) {
-    int t, k1;
-    if (TFAST) { t = it % ntrans; k1 = it / ntrans; }
-    else { t = it / N1; k1 = it - t * N1; }
-    cx<T> v[N2];
-#pragma unroll
-    for (int n2 = 0; n2 < N2; n2++) v[n2] = TFAST ? sm[(k1 * N2 + n2) * ntrans + t] : sm[(t * N1 + k1) * LD + n2];
-    Dft<N2, S, T>::run(v);
-#pragma unroll
-    for (int k2 = 0; k2 < N2; k2++) store(t, k1 + N1 * k2, v[k2]);
-  }
-}
-
-// Row variant with the result left in shared memory in natural order:
-// sm[t*N + k] = X_t[k].  Requires blockDim.x >= ntrans*N2 (>= ntrans*N1) and
-// BlockFft<N>::smem_elems(ntrans) elements of `sm` (>= ntrans*N).  Ends with
-// a __syncthreads().
-template <int N, int S, class T, class LoadF>
-__device__ __forceinline__ void row_fft_to_smem(int ntrans, cx<T>* sm, const cx<T>* __restrict__ tw,
-                                                LoadF load) {
-  constexpr int N1 = Split<N>::N1;
-  constexpr int N2 = Split<N>::N2;
-  constexpr int LD = N2 + 1;
-  const cx<T>* twn = tw + tw_off(N);
-  const int it = threadIdx.x;
-  if (it < ntrans * N2) {
-    int t = it / N2, n2 = it - t * N2;
-    cx<T> v[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; n1++) v[n1] = load(t, n2 + N2 * n1);
-    Dft<N1, S, T>::run(v);
-#pragma unroll
-    for (int k1 = 0; k1 < N1; k1++) {
-      cx<T> w = twn[n2 * k1];
-      if (S > 0) w.y = -w.y;
-      sm[(t * N1 + k1) * LD + n2] = (k1 == 0) ? v[k1] : cmul(v[k1], w);
-    }
-  }
-  __syncthreads();
-  cx<T> v[N2];
-  const bool active = it < ntrans * N1;
-  int t = 0, k1 = 0;
-  if (active) {
-    t = it / N1; k1 = it - t * N1;
-#pragma unroll
-    for (int n2 = 0; n2 < N2; n2++) v[n2] = sm[(t * N1 + k1) * LD + n2];
-  }
-  __syncthreads();
-  if (active) {
-    Dft<N2, S, T>::run(v);
-#pragma unroll
-    for (int k2 = 0; k2 < N2; k2++) sm[t * N + k1 + N1 * k2] = v[k2];
-  }
-  __syncthreads();
-}
-
-// In-place transform of `ntrans` sequences held in shared memory in natural
-// order, result in natural order.
-//   ROWS layout: element n of transform t at sm[t*N + n]
-//   COLS layout: element n of transform t at sm[n*ntrans + t]
-// Requires blockDim.x >= ntrans*N2 and smem_fft_elems<N, COLS>(ntrans)
-// elements.  Starts and ends with a __syncthreads().
+// Shared-memory elements of `ntrans` transforms of length N (COLS: columns).
 template <int N, bool COLS>
 __host__ __device__ constexpr int smem_fft_elems(int ntrans) {
   return COLS ? ntrans * N : ((ntrans * Split<N>::N1 * (Split<N>::N2 + 1) > ntrans * N)
                                   ? ntrans * Split<N>::N1 * (Split<N>::N2 + 1)
                                   : ntrans * N);
 }
-template <int N, int S, bool COLS, class T>
-__device__ __forceinline__ void smem_fft(int ntrans, cx<T>* sm, const cx<T>* __restrict__ tw) {
-  constexpr int N1 = Split<N>::N1;
-  constexpr int N2 = Split<N>::N2;
-  constexpr int LD = N2 + 1;
-  const cx<T>* twn = tw + tw_off(N);
-  const int it = threadIdx.x;
-  __syncthreads();
-  // pass A
-  {
-    const bool active = it < ntrans * N2;
-    int t = 0, n2 = 0;
-    cx<T> v[N1];
-    if (active) {
-      if (COLS) { t = it % ntrans; n2 = it / ntrans; }
-      else { t = it / N2; n2 = it - t * N2; }
-#pragma unroll
-      for (int n1 = 0; n1 < N1; n1++)
-        v[n1] = COLS ? sm[(n2 + N2 * n1) * ntrans + t] : sm[t * N + n2 + N2 * n1];
-    }
-    __syncthreads();
-    if (active) {
-      Dft<N1, S, T>::run(v);
-#pragma unroll
-      for (int k1 = 0; k1 < N1; k1++) {
-        cx<T> w = twn[n2 * k1];
-        if (S > 0) w.y = -w.y;
-        cx<T> r = (k1 == 0) ? v[k1] : cmul(v[k1], w);
-        if (COLS) sm[(k1 * N2 + n2) * ntrans + t] = r;
-        else sm[(t * N1 + k1) * LD + n2] = r;
-      }
-    }
-    __syncthreads();
-  }
-  // pass B
-  {
-    const bool active = it < ntrans * N1;
-    int t = 0, k1 = 0;
-    cx<T> v[N2];
-    if (active) {
-      if (COLS) { t = it % ntrans; k1 = it / ntrans; }
-      else { t = it / N1; k1 = it - t * N1; }
-#pragma unroll
-      for (int n2 = 0; n2 < N2; n2++)
-        v[n2] = COLS ? sm[(k1 * N2 + n2) * ntrans + t] : sm[(t * N1 + k1) * LD + n2];
-    }
-    __syncthreads();
-    if (active) {
-      Dft<N2, S, T>::run(v);
-#pragma unroll
-      for (int k2 = 0; k2 < N2; k2++) {
-        int k = k1 + N1 * k2;
-        if (COLS) sm[k * ntrans + t] = v[k2];
-        else sm[t * N + k] = v[k2];
-      }
-    }
-    __syncthreads();
-  }
-}
-
 // General four-step transform of `ntrans` sequences with one shared-memory
 // transpose.  Input comes from global memory through load(t, n) (pass A
 // issues N1 independent loads per thread before any arithmetic) or, with
 // IN_SMEM, from `sm` in natural layout (unless NoLoad through load(n2, m, v), n =
-// n2 + m, m a compile-time constant);
-// output goes to store(t, k, v) or, with OUT_SMEM, back to `sm` in natural
-// layout.
+// n2 + m, m a compile-time constant); output goes to store(t, k, v) or, with
+// OUT_SMEM, back to `sm` in natural layout.
 //   natural layout: rows  sm[t*N + n];  cols (COLS) sm[n*ntrans + t]
 // Requires blockDim.x >= ntrans*N2 and smem_fft_elems<N, COLS>(ntrans)
 // elements; every thread of the block must call it.  Ends with a
 // __syncthreads() when OUT_SMEM.  With a gate, the transform goes on only if
 // gate(), called by every thread once its inputs are loaded, says so for the
-// whole block; returns whether it did.  fft_core_tab takes the length-N twiddle
-// table itself (e.g. staged in shared memory by stage_twiddles); fft_core
-// reads it from the global table.
+// whole block; returns whether it did.  tw: the concatenated twiddle tables.
 struct NoLoad {};
 struct NoStore {
   template <class V> __device__ void operator()(int, int, V) const {}
 };
 struct NoGate {};
-template <int N, int S, bool COLS, bool IN_SMEM, bool OUT_SMEM, class T, class LoadF, class StoreF, class GateF>
-__device__ __forceinline__ bool fft_core_tab(int ntrans, cx<T>* sm, const cx<T>* twn, LoadF load, StoreF store,
-                                             GateF gate) {
+template <int N, int S, bool COLS, bool IN_SMEM, bool OUT_SMEM, class T, class LoadF, class StoreF, class GateF = NoGate>
+__device__ __forceinline__ bool fft_core(int ntrans, cx<T>* sm, const cx<T>* __restrict__ tw, LoadF load, StoreF store,
+                                         GateF gate = GateF{}) {
+  const cx<T>* const twn = tw + tw_off(N);
   constexpr int N1 = Split<N>::N1;
   constexpr int N2 = Split<N>::N2;
   constexpr int LD = N2 + 1;
@@ -468,21 +301,6 @@ __device__ __forceinline__ bool fft_core_tab(int ntrans, cx<T>* sm, const cx<T>*
   }
   return true;
 }
-template <int N, int S, bool COLS, bool IN_SMEM, bool OUT_SMEM, class T, class LoadF, class StoreF, class GateF = NoGate>
-__device__ __forceinline__ bool fft_core(int ntrans, cx<T>* sm, const cx<T>* __restrict__ tw, LoadF load,
-                                         StoreF store, GateF gate = GateF{}) {
-  return fft_core_tab<N, S, COLS, IN_SMEM, OUT_SMEM, T>(ntrans, sm, tw + tw_off(N), load, store, gate);
-}
-// Copy of the length-N twiddle table into shared memory `dst` (N entries),
-// by the whole block; ends with a barrier.
-template <int N, class T>
-__device__ __forceinline__ const cx<T>* stage_twiddles(cx<T>* dst, const cx<T>* __restrict__ tw) {
-  const cx<T>* g = tw + tw_off(N);
-  for (int i = threadIdx.x; i < N; i += blockDim.x) dst[i] = g[i];
-  __syncthreads();
-  return dst;
-}
-
 // Signed wavenumber index of FFT bin k for length n (k > n/2 -> k - n).
 __host__ __device__ __forceinline__ int signed_k(int k, int n) { return (k > n / 2) ? k - n : k; }
 

@@ -101,7 +101,6 @@ template <class F> bool with_any(int n, F&& f) {
   }
 }
 inline bool supported_small(int n) { return with_small(n, [](auto) {}); }
-inline bool supported_any(int n) { return with_any(n, [](auto) {}); }
 
 template <class T> struct DevBuf {
   T* p = nullptr;

@@ -231,7 +231,7 @@ k_row_fused(const __grid_constant__ FusedArgs f, const __grid_constant__ StageAr
   // -i kx a^ + b^ to array o1, a^ to o2, b^ to o3 (8: none)
   auto pick = [&](unsigned table) { return (int)((table >> (4 * team)) & 15u); };
   const int qa = pick(0x641040), qb = pick(learned ? 0x753362 : 0x753262);
-  const bool ma = (learned ? 0x34 : 0x34) >> team & 1, mb = !learned && team == 2;
+  const bool ma = 0x34 >> team & 1, mb = !learned && team == 2;
   const int o1 = pick(0x864820), o2 = pick(0x788318), o3 = pick(0x888588);
 
   // the window at this thread's points: level z - 1 and level z
