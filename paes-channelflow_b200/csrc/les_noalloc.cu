@@ -98,8 +98,8 @@ void expand_static(const T* in, T* out, int nx, int ny, int howmany, cudaStream_
   with_small(nx, [&](auto cn) {
     constexpr int N = decltype(cn)::value;
     using C = RowCfg<N>;
-    launch(k_op_row_r2c<T, N>, dim3(cdiv((howmany * ny + 1) / 2, C::NT)), dim3(C::THREADS), C::template smem<T>(), s, in, t1,
-           howmany * ny, KX, l1, tw);
+    launch(k_op_row_r2c<T, N, N / 2>, dim3(cdiv(howmany * ny / 2, C::NT)), dim3(C::THREADS), C::template smem<T>(), s, in, t1,
+           howmany * ny / 2, l1, tw);
   });
   with_small(ny, [&](auto cn) {
     constexpr int N = decltype(cn)::value;

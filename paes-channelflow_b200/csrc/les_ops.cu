@@ -35,11 +35,11 @@ void op_yderiv(const T* in, T* out, int n1, int n2, int howmany, double len, cud
 // The three kernels of expand, compress and deal: rows of length NR forward
 // (the first KX modes, layout la of x-spectral rows at `a`), columns, rows
 // back from layout lb at `b`.
-template <class T, int N>
-static void rows_forward(const T* in, cx<T>* a, int nrows, int KX, RowLayout la, const cx<T>* tw, cudaStream_t s) {
+template <class T, int N, int KX>
+static void rows_forward(const T* in, cx<T>* a, int nrows, RowLayout la, const cx<T>* tw, cudaStream_t s) {
   using C = RowCfg<N>;
-  launch(k_op_row_r2c<T, N>, dim3(cdiv((nrows + 1) / 2, C::NT)), dim3(C::THREADS), C::template smem<T>(), s, in, a, nrows,
-         KX, la, tw);
+  launch(k_op_row_r2c<T, N, KX>, dim3(cdiv(nrows / 2, C::NT)), dim3(C::THREADS), C::template smem<T>(), s, in, a, nrows / 2,
+         la, tw);
 }
 template <class T, int N>
 static void rows_back(const cx<T>* b, T* out, int nrows, int KX, RowLayout lb, const cx<T>* tw, cudaStream_t s) {
@@ -75,7 +75,10 @@ void op_expand(const T* in, T* out, int nx, int ny, int howmany, cudaStream_t s,
     t1 = t2 = reinterpret_cast<cx<T>*>(out);
     l1.ps = l2.ps;
   }
-  with_small(nx, [&](auto cn) { rows_forward<T, decltype(cn)::value>(in, t1, howmany * ny, KX, l1, tw, s); });
+  with_small(nx, [&](auto cn) {
+    constexpr int N = decltype(cn)::value;
+    rows_forward<T, N, N / 2>(in, t1, howmany * ny, l1, tw, s);
+  });
   columns<T, false, true>(t1, t2, ny, KX, howmany, l1, l2, 1.0 / ((double)nx * ny), tw, s);
   with_small(nx, [&](auto cn) { rows_back<T, 3 * decltype(cn)::value / 2>(t2, out, howmany * MY, KX, l2, tw, s); });
 }
@@ -90,7 +93,10 @@ void op_compress(const T* in, T* out, int nx, int ny, int howmany, cudaStream_t 
   if (!supported_small(nx) || !supported_small(ny)) throw CudaError("compress: unsupported size", LES_EINVAL);
   if (!t1) t1 = reinterpret_cast<cx<T>*>(out);
   const RowLayout l1 = layout(ny, KX), l2 = layout(MY, KX);
-  with_small(nx, [&](auto cn) { rows_forward<T, 3 * decltype(cn)::value / 2>(in, t2, howmany * MY, KX, l2, tw, s); });
+  with_small(nx, [&](auto cn) {
+    constexpr int N = decltype(cn)::value;
+    rows_forward<T, 3 * N / 2, N / 2>(in, t2, howmany * MY, l2, tw, s);
+  });
   columns<T, true, false>(t2, t1, ny, KX, howmany, l2, l1, 1.0 / ((double)MX * MY), tw, s);
   with_small(nx, [&](auto cn) { rows_back<T, decltype(cn)::value>(t1, out, howmany * ny, KX, l1, tw, s); });
 }
@@ -104,7 +110,10 @@ void op_deal(T* x, int nx, int ny, int howmany, cudaStream_t s, cx<T>* t1) {
   if (!supported_small(nx) || !supported_small(ny)) throw CudaError("deal: unsupported size", LES_EINVAL);
   if (!t1) t1 = reinterpret_cast<cx<T>*>(x);
   const RowLayout l = layout(ny, KX);
-  with_small(nx, [&](auto cn) { rows_forward<T, decltype(cn)::value>(x, t1, howmany * ny, KX, l, tw, s); });
+  with_small(nx, [&](auto cn) {
+    constexpr int N = decltype(cn)::value;
+    rows_forward<T, N, N / 2>(x, t1, howmany * ny, l, tw, s);
+  });
   columns<T, false, false>(t1, t1, ny, KX, howmany, l, l, 1.0 / ((double)nx * ny), tw, s);
   with_small(nx, [&](auto cn) { rows_back<T, decltype(cn)::value>(t1, x, howmany * ny, KX, l, tw, s); });
 }
