@@ -329,10 +329,11 @@ struct Ptr12 { void* p[12]; };
 // pointer arrays are __grid_constant__: indexed by blockIdx.z, a plain struct
 // parameter was copied to local memory by every thread (a quarter of the
 // kernels' time).  Per stage at 512x512x256, against one two-pass transform
-// per CTA: k_y_inverse FP32 1.09 -> 0.92 ms, FP64 2.03 -> 1.89; k_y_forward
-// 1.87 -> 1.21, 3.43 -> 2.32 ms (HBM floors 0.66 and 1.31); at 64x64x64 FP64
-// 18 -> 11 and 28 -> 12 us.  Bound by load latency and the load/store path
-// (64-byte rows) at about half of DRAM's peak.
+// per CTA: k_y_inverse FP32 1.09 -> 0.92 ms, FP64 2.03 -> 1.89 (0.96 and 1.95
+// now that e's forward transform, a kernel of its own then, is in it too);
+// k_y_forward 1.87 -> 1.21, 3.43 -> 2.34 ms (HBM floors 0.66 and 1.31); at
+// 64x64x64 FP64 18 -> 11 and 28 -> 12 us.  Bound by load latency and the
+// load/store path (64-byte rows) at 0.54-0.68 of the copy rate.
 template <class T, int M> struct ColPlan {
   using P = InPlace<M>;
   static constexpr int M1 = P::M1, R2 = P::R2, R3 = P::R3, NS = 8 * M1;
@@ -784,7 +785,7 @@ __device__ __forceinline__ void wall_rows_block(const cx<T>* __restrict__ Um, co
 // and the global dudt, dvdt (lowerbc.f90:70-72) from the FP64 mean shadows.
 // One block of 18 warps: a warp per sum (16 plane sums, then mru, mrv), each
 // in a fixed order, then one lane per wall.  (One thread for everything: 55
-// us per stage at any size; this 7 us.)
+// us per stage at any size; this 8-10 us.)
 constexpr int kWallFinalThreads = 18 * 32;
 static __global__ void __launch_bounds__(kWallFinalThreads)
 k_wall_final(const double* __restrict__ part, int nblk, const double* __restrict__ mru,
